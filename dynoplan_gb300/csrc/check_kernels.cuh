@@ -939,6 +939,16 @@ __device__ void load_obstacles(const EnvView &ev, void *sm) {
   __syncthreads();
 }
 
+// The abort flag lies in host memory: a read of it crosses the host link, and
+// the link serves about 150 M such reads a second whatever the SMs do, so a
+// read per item bounded the whole check (car1, 100,000 nodes x 5,000 motions,
+// 260,000 items: 1.73 ms for fetching the items alone, 0.18 ms without the
+// reads).  The warps that draw every kAbortPoll-th item of a launch read it
+// (the first item always, then one read in a few hundred nanoseconds of a full
+// GPU), and on an abort move the launch's item counter past its end.
+constexpr unsigned long long kAbortPoll = 64;
+constexpr unsigned long long kNoMoreItems = 1ull << 62;
+
 // Persistent warps over (primitive, 32 nodes) work items.
 // SLOTS: the slot-parallel narrow phase (FP32 tests with the band, NW > 0);
 // its per-warp scratch follows the obstacles at A.slot_offset.
@@ -972,17 +982,16 @@ __global__ void __launch_bounds__(kCheckThreads, SLOTS ? Robot<KIND>::SLOT_BLOCK
   };
   while (true) {
     unsigned long long item = 0;
-    int stop = 0;
     if (lane == 0) {
-      stop = *A.abort_flag;
-      item = stop ? n_items : i_lo + atomicAdd(&A.ctr->next_sub[A.sub], 1ull);
+      const unsigned long long drawn = atomicAdd(&A.ctr->next_sub[A.sub], 1ull);
+      item = i_lo + drawn;
+      if (item < n_items && drawn % kAbortPoll == 0 && *A.abort_flag) {
+        A.ctr->status = DPG_ERR_ABORTED;  // every warp's next item lies past the end
+        atomicMax(&A.ctr->next_sub[A.sub], kNoMoreItems);
+        item = n_items;
+      }
     }
     item = __shfl_sync(kFull, item, 0);
-    stop = __shfl_sync(kFull, stop, 0);
-    if (stop) {
-      if (lane == 0) A.ctr->status = DPG_ERR_ABORTED;
-      break;
-    }
     if (item >= n_items) break;
     if (A.n_ranges > 1) {
       const int nr = A.n_ranges, tot = A.sub_cum[nr];
