@@ -52,6 +52,8 @@ struct CheckArgs {
   // double->float conversions at 1/64 of the FP32 rate)
   float dt32, half_len32, half_wid32, radius32, band32;
   float lo32[3], hi32[3];
+  float lo_out[3], lo_in[3], hi_in[3], hi_out[3];  // the bounds less and plus the band
+  float lo_box[3], hi_box[3];  // a box within these (band and slack inside) needs no bounds test
   // this launch takes work items [n_items cum[sub] / cum[nsub],
   // n_items cum[sub + 1] / cum[nsub]) (integer weights; nsub <= 1: all items)
   int sub, nsub;
@@ -66,9 +68,24 @@ struct CheckArgs {
   // when set, the pair's node id is written back through it (processing
   // order -> caller's numbering) once the pair is checked
   const uint32_t *perm;
-  // slot variant: byte offset of the per-warp scratch in dynamic shared memory
-  int slot_offset;
+  // slot variant: byte offset of the warps' scratch in dynamic shared memory,
+  // and its bytes per warp
+  int slot_offset, slot_stride;
 };
+
+// The FP32 bounds and the limits derived from them.
+inline void set_bounds(CheckArgs &a, const double *lo, const double *hi) {
+  for (int i = 0; i < 3; i++) {
+    a.lo32[i] = (float)lo[i];
+    a.hi32[i] = (float)hi[i];
+    a.lo_out[i] = a.lo32[i] - a.band32;
+    a.lo_in[i] = a.lo32[i] + a.band32;
+    a.hi_in[i] = a.hi32[i] - a.band32;
+    a.hi_out[i] = a.hi32[i] + a.band32;
+    a.lo_box[i] = a.lo_in[i] + 1e-3f;
+    a.hi_box[i] = a.hi_in[i] - 1e-3f;
+  }
+}
 
 // Obstacle culling margin: every obstacle within the FP64 band, plus a slack
 // for the FP32 box arithmetic, and within the min_gap cap when min_gap is an
@@ -90,6 +107,11 @@ template <> __device__ __forceinline__ double node_off<double>(const NodeView &n
 
 // ------------------------------------------------------------ narrow phase --
 
+// a b + c d with the rounding written out in FP32: every kernel that makes a
+// test rounds it alike, so they send the same tests to FP64 (DPG_FLAG_CONTACT_RECHECK)
+__device__ __forceinline__ float dot2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
+__device__ __forceinline__ double dot2(double a, double b, double c, double d) { return a * b + c * d; }
+
 // Oriented box (pose c,s; half extents a,b; axis-aligned half extents ex,ey)
 // against an obstacle box.  Returns 0 clear, 1 contact, 2 ambiguous (|gap| <=
 // band, FP32 path).  mg takes the axis-aligned clearance.
@@ -101,7 +123,7 @@ __device__ __forceinline__ int planar_test(Real px, Real py, Real c, Real s, Rea
   mg = fmin(mg, g);
   if (g > band) return 0;
   const Real ac = fabs(c), as = fabs(s);
-  const Real du = dx * c + dy * s, dv = dy * c - dx * s;
+  const Real du = dot2(dx, c, dy, s), dv = dot2(dy, c, -dx, s);
   const Real gu = fabs(du) - (a + ob.hx * ac + ob.hy * as);
   const Real gv = fabs(dv) - (b + ob.hx * as + ob.hy * ac);
   const Real gs = fmax(g, fmax(gu, gv));
@@ -386,7 +408,7 @@ __device__ void check_one(const CheckArgs &A, const void *obs_sm, int p, int64_t
 #pragma unroll
         for (int q = 0; q < R::PARTS; q++) {
           const Real ac = fabs(ps[q].c), as = fabs(ps[q].s);
-          const Real ex = hl * ac + hw * as, ey = hl * as + hw * ac;
+          const Real ex = dot2(hl, ac, hw, as), ey = dot2(hl, as, hw, ac);
           int r = planar_test<Real, BAND>(ps[q].cx + sx, ps[q].cy + sy, ps[q].c, ps[q].s, ex, ey, ob, hl, hw,
                                           band, mg);
           if (BAND && r == 2) { r = gap64<KIND>(A, s0, k, q, x64, o) <= 0.0 ? 1 : 0; rechecked = true; }
@@ -458,7 +480,7 @@ __device__ void check_one(const CheckArgs &A, const void *obs_sm, int p, int64_t
     const int64_t row = s0 + er;
 #pragma unroll
     for (int c = 0; c < R::NX; c++) {
-      Real v = sizeof(Real) == 4 ? Real(pv.st32[row * R::NX + c]) : Real(pv.st64[row * R::NX + c]);
+      Real v = sizeof(Real) == 4 ? Real(pv.st32[row * R::NXP + c]) : Real(pv.st64[row * R::NX + c]);
       if (c < D) {
         v += off[c];
         if (V) v += t * off[D + c];
@@ -474,35 +496,64 @@ __device__ void check_one(const CheckArgs &A, const void *obs_sm, int p, int64_t
 // ------------------------------------------------- slot-parallel variant --
 //
 // The lockstep walk above makes every state cost the largest candidate count
-// of any lane: lanes with fewer candidates (most have none) wait.  This
-// variant keeps the walk over chunks of R::CHUNK states but runs the narrow
-// phase as a list of (lane, chunk, candidate obstacle) slots spread over the
-// warp's 32 lanes; a slot tests its obstacle against every state of its chunk
-// (all parts) and stops at its first contact.  One narrow round takes
-// consecutive chunks until the warp has about a round of slots (car1 chunks
-// average about 10 slots a warp), at most 32 states; chunks after a lane's
-// first contact are tested speculatively and discarded by the fold.  Per lane
-// and state, the contacts, the FP64 decisions and the minimum axis-aligned gap
-// are merged in shared memory; each lane then folds the states up to its first
-// contact, which gives exactly the per-state results of the sequential walk
-// (every candidate is tested at every state up to the first contact).  FP32
-// tests with FP64 decisions in the band; the bounds tests stay per lane.
+// of any lane: lanes with fewer candidates (most have none) wait.  Here the
+// warp goes through the primitive in windows of R::WINDOW chunks of R::CHUNK
+// states and gives every test to a lane of its own:
+//   - slots (lane, obstacle): the union of the lanes' window boxes selects the
+//     obstacles near any lane (a lane per obstacle, one ballot per 32), each of
+//     these is tested against the 32 lanes' boxes, and the lanes it is near to
+//     append their slots;
+//   - a lane per slot tests its obstacle against the boxes of the window's
+//     chunks at its owner's offset (a bit per chunk);
+//   - chunk by chunk, the near slots are listed and tested with a lane per
+//     (entry, state), 32 / CHUNK entries a step; the lane keeps its state's
+//     poses for the whole chunk.
+// Contacts and FP64 decisions come back as ballots and are merged per owner
+// (shared words, one atomic per entry with a contact); each lane then folds
+// the states up to its first contact, which gives exactly the per-state
+// results of the sequential walk (every candidate is tested at every state up
+// to the first contact, no state from the first one out of bounds on).  FP32
+// tests with FP64 decisions in the band.
+//
+// Bound by instruction issue (ncu, car1, 50,000 nodes: 75 % of the issue slots,
+// 27.6 active lanes an instruction, 5,200 warp instructions an item).  Against
+// the earlier form, which dealt (lane, chunk, obstacle) slots out and walked a
+// slot's states in one lane (17.7 active lanes, 6,800 instructions, spills):
+// check kernel of car1 (100,000 x 5,000) 1.91 -> 1.34 ms, quadrotor (50,000 x
+// 5,000) 10.6 -> 6.6 ms, unicycle1 FP64 0.127 -> 0.106 ms, a search round of
+// quad2d (32 x 10,000) 0.168 -> 0.121 ms.  Measured beside it: each lane walking
+// its own states for the bounds tests when many lanes need them, quadrotor
+// 6.6 -> 8.7 ms; 3 blocks an SM at 80 registers car1 1.40 ms, 5 at 48 (spills)
+// 2.01 ms; chunks of 8 or 32 states for the quadrotor 6.65 and 8.9 ms.
+// The end states go out through shared memory: rows of 52 bytes written by a
+// lane each cost the quadrotor 2.2 ms.
 
-constexpr int kSlotFill = 16;  // a narrow round stops taking chunks at this many slots
+constexpr int kSlotCap = 512;  // slots of a window held at a time; also the most obstacles of this variant
 
-template <int CH, int PARTS, int NW> struct SlotScratch {
-  static constexpr int GMAX = 32 / CH;  // chunks a round can take (32 hit bits)
-  static constexpr int MGS = 16;        // states a round takes when min_gap is an output
-  Pose<float> pose[32 * PARTS];         // the round's pose rows, [s * PARTS + q]
-  float2 ext[32 * PARTS];               // planar robots: axis-aligned half extents of each part
-  unsigned cm[GMAX][NW][32];            // per chunk, word and lane: the chunk's candidates
-  unsigned l1[NW][32];                  // per word and lane: level-1 candidates
-  unsigned mg[MGS][32];                 // per state and lane: min axis-aligned gap (order-preserving bits)
-  unsigned hit[32];                     // per lane: bit s = contact at state k0 + s
-  unsigned rc[32];                      // per lane: bit s = a test at k0 + s was decided in FP64
-  // (the bounds slots of a chunk use hit / rc before the narrow phase does:
-  // bit j = state j of the chunk out of bounds / decided in FP64)
+template <int KIND, bool ES64> struct SlotScratch {
+  static constexpr int C = Robot<KIND>::POSD + Robot<KIND>::VELOFF;
+  using Es = std::conditional_t<ES64, double, float>;
+  union {
+    struct {
+      uint16_t slot[kSlotCap];   // obstacle << 5 | lane
+      uint16_t list[kSlotCap];   // a chunk's entries
+      uint8_t near_[kSlotCap];   // the window's chunks the slot's obstacle is near to
+    };
+    Es end[32 * Robot<KIND>::NX];  // the item's end states on their way out
+  };
+  float off[C][32];  // the lanes' node offsets
+  uint32_t node[32];
+  unsigned hit[32];  // per lane: bit j = contact at state j of the chunk
+  unsigned rc[32];   // per lane: bit j = a test at state j was decided in FP64
 };
+// (with the min_gap output the warp's scratch is followed by (CHUNK + 1) x 32
+// words: per state of the chunk and lane, the min axis-aligned gap as ordered
+// bits, then each lane's minimum so far)
+
+template <int KIND, bool ES64>
+constexpr size_t slot_scratch_bytes(bool min_gap) {
+  return (sizeof(SlotScratch<KIND, ES64>) + (min_gap ? sizeof(unsigned) * 32 * (Robot<KIND>::CHUNK + 1) : 0) + 15) / 16 * 16;
+}
 
 __device__ __forceinline__ unsigned ord_gap(float f) {
   const unsigned u = __float_as_uint(f);
@@ -512,416 +563,458 @@ __device__ __forceinline__ float unord_gap(unsigned u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-template <int KIND, int NW>
-constexpr size_t slot_scratch_bytes() {
-  return sizeof(SlotScratch<Robot<KIND>::CHUNK, Robot<KIND>::PARTS, NW>);
+// FP64 decision of an ambiguous obstacle test (rare: kept out of line)
+template <int KIND>
+__device__ __noinline__ bool contact64(const CheckArgs &A, int p, int k, int q, uint32_t node, int o) {
+  return gap64<KIND>(A, A.pv.soff[p], k, q, A.nv.x64 + (int64_t)node * Robot<KIND>::NX, o) <= 0.0;
+}
+// FP64 decision of an ambiguous bounds test of position component i
+template <int KIND>
+__device__ __noinline__ bool outside64(const CheckArgs &A, int p, int k, uint32_t node, int i) {
+  const double v = pos64<KIND>(A, A.pv.soff[p] + k, k, A.nv.x64 + (int64_t)node * Robot<KIND>::NX, i);
+  return !(v >= A.ev.lo[i] && v <= A.ev.hi[i]);
 }
 
-template <int KIND, int NW, bool ES64>
-__device__ void check_one_slots(const CheckArgs &A, const void *obs_sm,
-                                SlotScratch<Robot<KIND>::CHUNK, Robot<KIND>::PARTS, NW> &S, int p, int64_t pair,
-                                uint32_t node, bool active) {
+// Bounds test of state k (pose ps) for the lane whose offsets are in column
+// `own` of S; `amb` set when a component was decided in FP64.
+template <int KIND, class Scratch>
+__device__ __forceinline__ bool out_of_bounds(const CheckArgs &A, const Scratch &S, const Pose<float> &ps, int p, int k,
+                                              int own, bool &amb) {
   using R = Robot<KIND>;
-  using Scratch = SlotScratch<Robot<KIND>::CHUNK, Robot<KIND>::PARTS, NW>;
-  constexpr int D = R::POSD, V = R::VELOFF, CH = R::CHUNK, PARTS = R::PARTS;
-  static_assert(NW > 0, "the slot variant needs the candidate bitmasks");
-  static_assert(CH <= 16 && Scratch::MGS % CH == 0, "5-bit state counts; whole chunks under the min_gap limit");
-  const int lane = threadIdx.x & 31;
-  const PrimView &pv = A.pv;
-  const RobotParams &rp = A.rp;
-  const int L = pv.len[p];
-  const int64_t s0 = pv.soff[p];
-  const Pose<float> *pose = pv.pose32;
-  const float band = A.band32, dt = A.dt32;
-  const double *x64 = A.nv.x64 + (int64_t)(active ? node : 0) * R::NX;
-  const int n_obs = A.ev.n_obs;
-  const bool want_mg = A.out.min_gap != nullptr;  // per-state gap merges only for that output
-  const int GL = want_mg ? Scratch::MGS / CH : Scratch::GMAX;
+  constexpr int D = R::POSD, V = R::VELOFF;
+  const float tk = float(k) * A.dt32;
+  float osh[D + V];
+#pragma unroll
+  for (int i = 0; i < D + V; i++) osh[i] = S.off[i][own];
+  const float pv3[3] = {ps.cx + osh[0] + (V ? tk * osh[D] : 0.f), ps.cy + osh[1] + (V ? tk * osh[D + 1] : 0.f),
+                        D == 3 ? ps.c + osh[2] + (V ? tk * osh[D + 2] : 0.f) : 0.f};
+  int bt = 0;
+#pragma unroll
+  for (int i = 0; i < D; i++) {
+    const float v = pv3[i];
+    int r = (v < A.lo_out[i] || v > A.hi_out[i]) ? 1 : ((v <= A.lo_in[i] || v >= A.hi_in[i]) ? 2 : 0);
+    if (r == 2) {  // decide in FP64
+      r = outside64<KIND>(A, p, k, S.node[own], i) ? 1 : 0;
+      amb = true;
+    }
+    bt |= r;
+  }
+  return bt != 0;
+}
 
-  float off[D + V];
+// centre and half extents of the culling box at `box` (D centres, D halves)
+template <int D>
+__device__ __forceinline__ void load_box(const float *box, float *c, float *h) {
+  if constexpr (D == 2) {
+    const float4 v = *reinterpret_cast<const float4 *>(box);
+    c[0] = v.x; c[1] = v.y; h[0] = v.z; h[1] = v.w;
+  } else {
+    const float2 *v = reinterpret_cast<const float2 *>(box);
+    const float2 v0 = v[0], v1 = v[1], v2 = v[2];
+    c[0] = v0.x; c[1] = v0.y; c[2] = v1.x; h[0] = v1.y; h[1] = v2.x; h[2] = v2.y;
+  }
+}
+
+template <int KIND, bool ES64>
+__device__ __forceinline__ void check_item(const CheckArgs &A, const void *obs_sm, SlotScratch<KIND, ES64> &S, int p,
+                                           uint32_t pair0, int count, uint32_t node) {
+  using R = Robot<KIND>;
+  using Ob = std::conditional_t<R::SPHERE, Obs3<float>, Obs2<float>>;
+  constexpr int D = R::POSD, V = R::VELOFF, CH = R::CHUNK, PARTS = R::PARTS, WIN = R::WINDOW;
+  constexpr int NE = 32 / CH;  // entries a step tests at once
+  constexpr unsigned kChunkBits = CH == 32 ? 0xffffffffu : (1u << CH) - 1u;
+  static_assert(32 % CH == 0 && WIN <= 8, "a lane per (entry, state); a byte of chunk bits");
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const bool active = lane < count;
+  const PrimView &pv = A.pv;
+  const int L = pv.len[p], n_chunks = (L + CH - 1) / CH;
+  const float dt = A.dt32, M = A.cull_margin;
+  const int n_obs = A.ev.n_obs;
+  const PairView &o = A.out;
+  const bool want_mg = o.min_gap != nullptr;
+  unsigned *mgs = reinterpret_cast<unsigned *>(&S + 1);  // [CH + 1][32] with min_gap
+
 #pragma unroll
-  for (int i = 0; i < D; i++) off[i] = active ? node_off<float>(A.nv, node, i, R::NX, i) : 0.f;
+  for (int i = 0; i < D; i++) S.off[i][lane] = active ? node_off<float>(A.nv, node, i, R::NX, i) : 0.f;
 #pragma unroll
-  for (int i = 0; i < V; i++) off[D + i] = active ? node_off<float>(A.nv, node, D + i, R::NX, R::vel_comp(i)) : 0.f;
+  for (int i = 0; i < V; i++)
+    S.off[D + i][lane] = active ? node_off<float>(A.nv, node, D + i, R::NX, R::vel_comp(i)) : 0.f;
+  S.node[lane] = node;
+  S.hit[lane] = 0u;
+  S.rc[lane] = 0u;
+  if (want_mg)
+    for (int i = 0; i <= CH; i++) mgs[32 * i + lane] = 0xffffffffu;
+  if (active && (A.perm || o.node_host)) {  // the pair's node in the caller's numbering
+    const uint32_t n = A.perm ? A.perm[node] : node;
+    if (A.perm) o.node[pair0 + lane] = n;
+    if (o.node_host) {
+      o.node_host[pair0 + lane] = n;
+      o.prim_host[pair0 + lane] = (uint32_t)p;
+    }
+  }
 
   // bounds pre-check on the swept box of the positions (as check_one)
-  bool need_bounds = true;
-  if (active) {
+  bool need_bounds;
+  {
     const float *bx32 = pv.pbox32 + (int64_t)p * 2 * D;
     const float tmax = float(L - 1) * dt;
     bool inside = true;
 #pragma unroll
     for (int i = 0; i < D; i++) {
-      float lo = bx32[i] + off[i], hi = bx32[D + i] + off[i];
-      if (V) {
-        const float sv = tmax * off[D + i];
+      const float off = S.off[i][lane];
+      float lo = bx32[i] + off, hi = bx32[D + i] + off;
+      if constexpr (V > 0) {
+        const float sv = tmax * S.off[D + i][lane];
         lo += fminf(sv, 0.f);
         hi += fmaxf(sv, 0.f);
       }
-      inside = inside && lo > A.lo32[i] + band + 1e-3f && hi < A.hi32[i] - band - 1e-3f;
+      inside = inside && lo > A.lo_box[i] && hi < A.hi_box[i];
     }
-    need_bounds = !inside;
+    need_bounds = active && !inside;
   }
 
-  // level-1 culling against the whole transformed primitive
-  const float M = A.cull_margin;
-  {
-    const float *tb = pv.tbox32 + (int64_t)p * 2 * D;
-    const float tmax = float(L - 1) * dt;
+  bool live = active, collided = false, rechecked = false;
+  bool oob = false;
+  int fi = L;  // first state out of bounds, else first contact, else L
+  const int j = lane % CH, sub = lane / CH;  // this lane's state of a chunk and its entry of a step
+  const Pose<float> *pose = pv.pose32 + pv.soff[p];
+  const float *cbox = pv.cbox32 + pv.coff[p] * 2 * D;
+  __syncwarp();
+
+  for (int c0 = 0; c0 < n_chunks; c0 += WIN) {
+    unsigned rest = __ballot_sync(kFull, live);  // lanes whose window is still to check
+    if (!rest) break;
+    const int nc = min(WIN, n_chunks - c0);
+    // the lane's box over the window: the union of its chunks' boxes, moved by
+    // the offset (and the velocity over the window's time); the chunks in
+    // which the lane's box is not inside the bounds
     float cen[D], hf[D];
+    unsigned nbw = 0u;
+    const bool any_nb = __any_sync(kFull, live && need_bounds);
+    {
+      float lo[D], hi[D];
 #pragma unroll
-    for (int i = 0; i < D; i++) {
-      cen[i] = tb[i] + off[i];
-      hf[i] = tb[D + i];
-      if (V) {
-        const float sv = tmax * off[D + i];
-        cen[i] += 0.5f * sv;
-        hf[i] += 0.5f * fabsf(sv);
-      }
-    }
-#pragma unroll
-    for (int w = 0; w < NW; w++) {
-      uint32_t bits = 0u;
-      if (active) {
-        const int o0 = 32 * w, o1 = min(n_obs, o0 + 32);
-        for (int o = o0; o < o1; o++)
-          if (near_box<D, float>(cen, hf, obs_sm, o, M)) bits |= 1u << (o - o0);
-      }
-      S.l1[w][lane] = bits;
-    }
-  }
-
-  bool done = !active, collided = false, rechecked = false;
-  int first_oob = L, first_col = L;
-  float mg = INFINITY;
-  const float hl = A.half_len32, hw = A.half_wid32, rad = A.radius32;
-
-  for (int k0 = 0; k0 < L;) {
-    if (!__any_sync(kFull, !done)) break;
-    // the round's chunks: level-2 culling, bounds tests, per-chunk state and candidate counts
-    uint32_t nsts = 0u, ncs = 0u;  // chunk g: states to test (5 bits at 5g), candidates (8 bits at 8g)
-    int n_lane = 0;                // this lane's slots in the round
-    int G = 0, kk = k0;
-    while (true) {
-      const int kend = min(L, kk + CH);
-      int nc = 0;
-      bool nb = false;
-      if (!done) {
-        const float *cb = pv.cbox32 + (pv.coff[p] + kk / CH) * 2 * D;
-        const float t0 = float(kk) * dt, t1 = float(kend - 1) * dt;
-        float cen[D], hf[D];
+      for (int i = 0; i < D; i++) { lo[i] = INFINITY; hi[i] = -INFINITY; }
+      for (int c = 0; c < nc; c++) {
+        float cc[D], ch[D];
+        load_box<D>(cbox + (c0 + c) * 2 * D, cc, ch);
 #pragma unroll
         for (int i = 0; i < D; i++) {
-          cen[i] = cb[i] + off[i];
-          hf[i] = cb[D + i];
-          if (V) {
-            const float v = off[D + i];
-            cen[i] += 0.5f * (t0 + t1) * v;
-            hf[i] += 0.5f * (t1 - t0) * fabsf(v);
-          }
+          lo[i] = fminf(lo[i], cc[i] - ch[i]);
+          hi[i] = fmaxf(hi[i], cc[i] + ch[i]);
         }
-        if (!collided) {
-#pragma unroll
-          for (int w = 0; w < NW; w++) {
-            uint32_t m = S.l1[w][lane], c = 0;
-            while (m) {
-              const int b = __ffs(m) - 1;
-              m &= m - 1;
-              if (near_box<D, float>(cen, hf, obs_sm, 32 * w + b, M)) c |= 1u << b;
-            }
-            S.cm[G][w][lane] = c;
-            nc += __popc(c);
-          }
-        }
-        if (need_bounds) {
+        if (any_nb) {
+          const int k0 = (c0 + c) * CH;
+          const float t0 = float(k0) * dt, t1 = float(min(L, k0 + CH) - 1) * dt;
           bool in = true;
 #pragma unroll
-          for (int i = 0; i < D; i++)
-            in = in && cen[i] - hf[i] > A.lo32[i] + band + 1e-3f && cen[i] + hf[i] < A.hi32[i] - band - 1e-3f;
-          nb = !in;
-        }
-      }
-      // bounds tests of the chunk's states, up to each lane's first state out.
-      // Few lanes with tests: (lane, state) slots over the warp, each lane's
-      // first state out (and the FP64 decisions up to it) from bitmasks, as
-      // the sequential walk finds them; else each lane walks its states.
-      int j_oob = CH;
-      bool walk = nb;
-      if constexpr (R::BOUNDS_SLOTS) {
-        const unsigned nbm = __ballot_sync(kFull, nb);
-        const int nbs = __popc(nbm) * (kend - kk);
-        if (nbm && nbs <= 64) {
-          walk = false;
-          const int ns = kend - kk;
-          S.hit[lane] = 0u;
-          S.rc[lane] = 0u;
-          __syncwarp();
-          for (int base = 0; base < nbs; base += 32) {
-            const int t = base + lane;
-            const int li = t / ns, j = t - li * ns;
-            const int owner = t < nbs ? (int)__fns(nbm, 0u, li + 1) : 0;
-            float osh[D + V];
-  #pragma unroll
-            for (int i = 0; i < D + V; i++) osh[i] = __shfl_sync(kFull, off[i], owner);
-            const uint32_t onode = __shfl_sync(kFull, node, owner);
-            if (t < nbs) {
-              const int k = kk + j;
-              const Pose<float> ps = pose[s0 + k];  // part 0 = the state position
-              const float tk = float(k) * dt;
-              const float pv3[3] = {ps.cx + osh[0] + (V ? tk * osh[D] : 0.f), ps.cy + osh[1] + (V ? tk * osh[D + 1] : 0.f),
-                                    D == 3 ? ps.c + osh[2] + (V ? tk * osh[D + 2] : 0.f) : 0.f};
-              int bt = 0;
-              bool amb = false;
-  #pragma unroll
-              for (int i = 0; i < D; i++) {
-                const float v = pv3[i], lo = A.lo32[i], hi = A.hi32[i];
-                int r = (v < lo - band || v > hi + band) ? 1 : ((v <= lo + band || v >= hi - band) ? 2 : 0);
-                if (r == 2) {  // decide in FP64
-                  const double v64 = pos64<KIND>(A, s0 + k, k, A.nv.x64 + (int64_t)onode * R::NX, i);
-                  r = (v64 >= A.ev.lo[i] && v64 <= A.ev.hi[i]) ? 0 : 1;
-                  amb = true;
-                }
-                bt |= r;
-              }
-              if (bt) atomicOr(&S.hit[owner], 1u << j);
-              if (amb) atomicOr(&S.rc[owner], 1u << j);
-            }
-          }
-          __syncwarp();
-          if (nb) {
-            const unsigned bo = S.hit[lane];
-            const int first = bo ? __ffs(bo) - 1 : CH;
-            if (bo) j_oob = first;
-            if (S.rc[lane] & (bo ? ((2u << first) - 1u) : 0xffffffffu)) rechecked = true;
-          }
-          __syncwarp();  // the next chunk's slots and the narrow phase reuse the masks
-        }
-      }
-      if (walk) {
-        for (int k = kk; k < kend; k++) {
-          const Pose<float> ps = pose[s0 + k];  // part 0 = the state position
-          const float t = float(k) * dt;
-          const float pv3[3] = {ps.cx + off[0] + (V ? t * off[D] : 0.f), ps.cy + off[1] + (V ? t * off[D + 1] : 0.f),
-                                D == 3 ? ps.c + off[2] + (V ? t * off[D + 2] : 0.f) : 0.f};
-          int bt = 0;
-#pragma unroll
           for (int i = 0; i < D; i++) {
-            const float v = pv3[i], lo = A.lo32[i], hi = A.hi32[i];
-            int r = (v < lo - band || v > hi + band) ? 1 : ((v <= lo + band || v >= hi - band) ? 2 : 0);
-            if (r == 2) {  // decide in FP64
-              const double v64 = pos64<KIND>(A, s0 + k, k, x64, i);
-              r = (v64 >= A.ev.lo[i] && v64 <= A.ev.hi[i]) ? 0 : 1;
-              rechecked = true;
+            float x = cc[i] + S.off[i][lane], h = ch[i];
+            if constexpr (V > 0) {
+              const float v = S.off[D + i][lane];
+              x += 0.5f * (t0 + t1) * v;
+              h += 0.5f * (t1 - t0) * fabsf(v);
             }
-            bt |= r;
+            in = in && x - h > A.lo_box[i] && x + h < A.hi_box[i];
           }
-          if (bt) {
-            j_oob = k - kk;
-            break;
-          }
+          if (!in) nbw |= 1u << c;
         }
       }
-      const int nst = (!done && !collided) ? min(kend - kk, j_oob) : 0;
-      if (nst == 0) nc = 0;
-      nsts |= (uint32_t)nst << (5 * G);
-      ncs |= (uint32_t)nc << (8 * G);
-      n_lane += nc;
-      if (!done && j_oob < CH) {  // later states of this lane are never tested
-        first_oob = kk + j_oob;
-        done = true;
-      }
-      G++;
-      kk = kend;
-      if (G >= GL || kk >= L) break;
-      if (__reduce_add_sync(kFull, (unsigned)n_lane) >= (unsigned)kSlotFill) break;
-    }
-    const int nS = kk - k0;  // states of the round, <= 32 (<= MGS with min_gap)
-    // the narrow phase as (lane, chunk, candidate) slots
-    int pre = n_lane;
+      if (!need_bounds) nbw = 0u;
+      const float tm0 = float(c0 * CH) * dt, tm1 = float(min(L, (c0 + nc) * CH) - 1) * dt;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int v = __shfl_up_sync(kFull, pre, d);
-      if (lane >= d) pre += v;
-    }
-    const int T = __shfl_sync(kFull, pre, 31);
-    pre -= n_lane;  // exclusive prefix
-    if (T > 0) {
-      for (int e = lane; e < nS * PARTS; e += 32) {
-        const int j = e / PARTS, q = e % PARTS;
-        const Pose<float> ps = pose[(int64_t)q * pv.S + s0 + k0 + j];
-        S.pose[e] = ps;
-        const float ac = fabsf(ps.c), as = fabsf(ps.s);
-        S.ext[e] = make_float2(hl * ac + hw * as, hl * as + hw * ac);
+      for (int i = 0; i < D; i++) {
+        cen[i] = 0.5f * (lo[i] + hi[i]) + S.off[i][lane];
+        hf[i] = 0.5f * (hi[i] - lo[i]);
+        if constexpr (V > 0) {
+          const float v = S.off[D + i][lane];
+          cen[i] += 0.5f * (tm0 + tm1) * v;
+          hf[i] += 0.5f * (tm1 - tm0) * fabsf(v);
+        }
       }
-      if (want_mg)
-        for (int j = 0; j < nS; j++) S.mg[j][lane] = ord_gap(INFINITY);
-      S.hit[lane] = 0u;
-      S.rc[lane] = 0u;
+    }
+    // (usually one pass: all lanes; more slots than the list holds: as many
+    // lanes as fit, then the others)
+    while (rest) {
+      unsigned take = rest;
+      int n_slot;
+      while (true) {
+        n_slot = 0;
+        const bool inc = ((take >> lane) & 1u) && !collided;
+        // union of the lanes' boxes, a little wider than their own tests (a
+        // lane with a NaN offset is near no obstacle and stays out of it)
+        float ulo[D], uhi[D];
+#pragma unroll
+        for (int i = 0; i < D; i++) {
+          const float lo = cen[i] - hf[i], hi = cen[i] + hf[i];
+          const bool ok = inc && lo <= hi;
+          ulo[i] = unord_gap(__reduce_min_sync(kFull, ok ? ord_gap(lo) : ord_gap(INFINITY)));
+          uhi[i] = unord_gap(__reduce_max_sync(kFull, ok ? ord_gap(hi) : ord_gap(-INFINITY)));
+          const float m = M + 1e-3f + 1e-6f * (fabsf(ulo[i]) + fabsf(uhi[i]));
+          ulo[i] -= m;
+          uhi[i] += m;
+        }
+        for (int w0 = 0; w0 < n_obs; w0 += 32) {
+          bool u = w0 + lane < n_obs;
+          if (u) {
+            const Ob ob = ((const Ob *)obs_sm)[w0 + lane];
+            u = ob.cx + ob.hx >= ulo[0] && ob.cx - ob.hx <= uhi[0] && ob.cy + ob.hy >= ulo[1] && ob.cy - ob.hy <= uhi[1];
+            if constexpr (D == 3) u = u && ob.cz + ob.hz >= ulo[2] && ob.cz - ob.hz <= uhi[2];
+          }
+          for (unsigned m = __ballot_sync(kFull, u); m; m &= m - 1) {
+            const int o = w0 + __ffs(m) - 1;
+            const bool h = inc && near_box<D, float>(cen, hf, obs_sm, o, M);
+            const unsigned hm = __ballot_sync(kFull, h);
+            const int pos = n_slot + __popc(hm & lt);
+            if (h && pos < kSlotCap) S.slot[pos] = (uint16_t)(o << 5 | lane);
+            n_slot += __popc(hm);
+          }
+        }
+        if (n_slot <= kSlotCap) break;
+        // one lane always fits (at most kSlotCap obstacles): halve the set
+        for (int k = __popc(take) / 2; k > 0; k--) take &= ~(0x80000000u >> __clz(take));
+      }
+      rest &= ~take;
       __syncwarp();
-      for (int base = 0; base < T; base += 32) {
-        const int t = base + lane;
-        int owner = 0;  // the last lane whose exclusive prefix is <= t
-#pragma unroll
-        for (int step = 16; step >= 1; step >>= 1) {
-          const int cand = owner + step;
-          const int pv_ = __shfl_sync(kFull, pre, cand & 31);
-          if (cand < 32 && pv_ <= t) owner = cand;
+      // the window's chunks each slot is near to
+      unsigned near_any = 0u;
+      for (int b = lane; b < n_slot; b += 32) {
+        const unsigned e = S.slot[b];
+        const int own = (int)(e & 31u);
+        const Ob ob = ((const Ob *)obs_sm)[e >> 5];
+        float r[D], v[D], h[D];  // owner's offset from the obstacle's centre
+        r[0] = S.off[0][own] - ob.cx;
+        h[0] = ob.hx + M;
+        r[1] = S.off[1][own] - ob.cy;
+        h[1] = ob.hy + M;
+        if constexpr (D == 3) {
+          r[2] = S.off[2][own] - ob.cz;
+          h[2] = ob.hz + M;
         }
-        const int opre = __shfl_sync(kFull, pre, owner);
-        const uint32_t onsts = __shfl_sync(kFull, nsts, owner);
-        const uint32_t oncs = __shfl_sync(kFull, ncs, owner);
-        const uint32_t onode = __shfl_sync(kFull, node, owner);
-        float osh[D + V];
 #pragma unroll
-        for (int i = 0; i < D + V; i++) osh[i] = __shfl_sync(kFull, off[i], owner);
-        if (t < T) {
-          // the slot's chunk g and candidate index within it
-          int cidx = t - opre, g = 0;
-          for (; g < Scratch::GMAX - 1; g++) {
-            const int c = (oncs >> (8 * g)) & 255u;
-            if (cidx < c) break;
-            cidx -= c;
+        for (int i = 0; i < D; i++) v[i] = V > 0 ? S.off[(V > 0 ? D : 0) + i][own] : 0.f;
+        unsigned near = 0u;
+#pragma unroll 4
+        for (int c = 0; c < nc; c++) {
+          float cc[D], ch[D];
+          load_box<D>(cbox + (c0 + c) * 2 * D, cc, ch);
+          bool in = true;
+          if constexpr (V > 0) {
+            const int k0 = (c0 + c) * CH, k1 = min(L, k0 + CH) - 1;
+            const float tm = 0.5f * dt * float(k0 + k1), th = 0.5f * dt * float(k1 - k0);
+#pragma unroll
+            for (int i = 0; i < D; i++) in = in && fabsf(cc[i] + tm * v[i] + r[i]) <= ch[i] + th * fabsf(v[i]) + h[i];
+          } else {
+#pragma unroll
+            for (int i = 0; i < D; i++) in = in && fabsf(cc[i] + r[i]) <= ch[i] + h[i];
           }
-          const int onst = (onsts >> (5 * g)) & 31u;
-          int o = -1;
-#pragma unroll
-          for (int w = 0; w < NW; w++) {
-            if (o < 0) {
-              const uint32_t ow = S.cm[g][w][owner];
-              const int c = __popc(ow);
-              if (cidx < c) o = 32 * w + (int)__fns(ow, 0u, cidx + 1);
-              else cidx -= c;
+          if (in) near |= 1u << c;
+        }
+        S.near_[b] = (uint8_t)near;
+        near_any |= near;
+      }
+      near_any = __reduce_or_sync(kFull, near_any);
+      __syncwarp();
+
+      const bool mine = (take >> lane) & 1u;  // a lane of this pass
+      for (unsigned todo = near_any | __reduce_or_sync(kFull, mine ? nbw : 0u); todo; todo &= todo - 1) {
+        const int c = __ffs(todo) - 1, k0 = (c0 + c) * CH, kend = min(L, k0 + CH);
+        const unsigned nbm = __ballot_sync(kFull, mine && live && ((nbw >> c) & 1u));
+        const unsigned chk_m = ((near_any >> c) & 1u) ? __ballot_sync(kFull, mine && live && !collided) : 0u;
+        if (!(nbm | chk_m)) continue;
+        const int k = k0 + j;
+
+        // bounds tests of the chunk's states: a lane per (lane, state)
+        int j_oob = CH;
+        if (nbm) {
+          const bool nb = (nbm >> lane) & 1u;
+          unsigned out_bits = 0u, rc_bits = 0u;
+          const Pose<float> ps = pose[min(k, L - 1)];
+          const int rank = __popc(nbm & lt), n = __popc(nbm);
+          if (nb) S.list[rank] = (uint16_t)lane;
+          __syncwarp();
+          for (int it = 0; it * NE < n; it++) {
+            const int i = it * NE + sub;
+            bool out = false, amb = false;
+            if (i < n && k < kend) out = out_of_bounds<KIND>(A, S, ps, p, k, S.list[i], amb);
+            const unsigned ow = __ballot_sync(kFull, out), aw = __ballot_sync(kFull, amb);
+            if (nb && rank / NE == it) {
+              out_bits = (ow >> (rank % NE * CH)) & kChunkBits;
+              rc_bits = (aw >> (rank % NE * CH)) & kChunkBits;
             }
           }
-          if (o >= 0 && o < n_obs) {
-            const double *ox64 = A.nv.x64 + (int64_t)onode * R::NX;
-            using Ob = std::conditional_t<R::SPHERE, Obs3<float>, Obs2<float>>;
-            const Ob ob = ((const Ob *)obs_sm)[o];
-            const int sb = g * CH;  // the chunk's first state in the round
-            for (int j = 0; j < onst; j++) {
-              const int sj = sb + j, k = k0 + sj;
-              float sx = osh[0], sy = osh[1], sz = 0.f;
-              if (V) {
-                const float tk = float(k) * dt;
-                sx += tk * osh[D + 0];
-                sy += tk * osh[D + 1];
-                if (D == 3) sz = osh[2] + tk * osh[D + 2];
-              } else if (D == 3) {
-                sz = osh[2];
-              }
-              float gmin = INFINITY;
-              bool hit = false;
+          __syncwarp();
+          if (out_bits) j_oob = __ffs(out_bits) - 1;
+          if (rc_bits & (out_bits ? (2u << j_oob) - 1u : 0xffffffffu)) rechecked = true;
+        }
+
+        // obstacle tests: a lane per (near slot, state)
+        if (chk_m) {
+          const int nst = min(kend - k0, j_oob);  // states of the chunk to test
+          int n_ent = 0;
+          for (int b = 0; b < n_slot; b += 32) {
+            bool in = b + lane < n_slot && ((S.near_[b + lane] >> c) & 1u);
+            const unsigned e = in ? S.slot[b + lane] : 0u;
+            in = in && ((chk_m >> (e & 31u)) & 1u);
+            const unsigned m = __ballot_sync(kFull, in);
+            if (in) S.list[n_ent + __popc(m & lt)] = (uint16_t)e;
+            n_ent += __popc(m);
+          }
+          __syncwarp();
+          if (n_ent) {
+            Pose<float> ps[PARTS];  // this lane's state of the chunk
 #pragma unroll
-              for (int q = 0; q < PARTS; q++) {
-                int r;
-                const Pose<float> ps = S.pose[sj * PARTS + q];
-                if constexpr (R::SPHERE) {
-                  r = sphere_test<float, true>(ps.cx + sx, ps.cy + sy, ps.c + sz, ob, rad, band, gmin);
-                } else {
-                  // axis-aligned reject first; the oriented axes only within the band
-                  const float2 ex = S.ext[sj * PARTS + q];
-                  const float dx = ps.cx + sx - ob.cx, dy = ps.cy + sy - ob.cy;
-                  const float ga = fmaxf(fabsf(dx) - (ex.x + ob.hx), fabsf(dy) - (ex.y + ob.hy));
-                  gmin = fminf(gmin, ga);
-                  if (ga > band) {
-                    r = 0;
+            for (int q = 0; q < PARTS; q++) ps[q] = pose[q * pv.S + min(k, L - 1)];
+            const float tk = float(k) * dt;
+            unsigned seen = 0u;  // contacts or FP64 decisions of the chunk
+            for (int i0 = 0; i0 < n_ent; i0 += NE) {
+              const bool in = i0 + sub < n_ent;
+              const unsigned e = in ? S.list[i0 + sub] : 0u;
+              const int own = (int)(e & 31u), o = (int)(e >> 5);
+              const int own_nst = __shfl_sync(kFull, nst, own);
+              bool hit = false, amb = false;
+              if (in && j < own_nst) {
+                const Ob ob = ((const Ob *)obs_sm)[o];
+                float sx = S.off[0][own], sy = S.off[1][own], sz = D == 3 ? S.off[D - 1][own] : 0.f;
+                if constexpr (V > 0) {
+                  sx += tk * S.off[D][own];
+                  sy += tk * S.off[D + 1][own];
+                  if constexpr (D == 3) sz += tk * S.off[D + 2][own];
+                }
+                float gmin = INFINITY;
+#pragma unroll
+                for (int q = 0; q < PARTS; q++) {
+                  int r;
+                  if constexpr (R::SPHERE) {
+                    r = sphere_test<float, true>(ps[q].cx + sx, ps[q].cy + sy, ps[q].c + sz, ob, A.radius32, A.band32,
+                                                 gmin);
                   } else {
-                    float unused = INFINITY;
-                    r = planar_test<float, true>(ps.cx + sx, ps.cy + sy, ps.c, ps.s, ex.x, ex.y, ob, hl, hw, band,
-                                                 unused);
+                    const float ac = fabsf(ps[q].c), as = fabsf(ps[q].s), hl = A.half_len32, hw = A.half_wid32;
+                    r = planar_test<float, true>(ps[q].cx + sx, ps[q].cy + sy, ps[q].c, ps[q].s, dot2(hl, ac, hw, as),
+                                                 dot2(hl, as, hw, ac), ob, hl, hw, A.band32, gmin);
                   }
+                  if (r == 2) {  // decide in FP64
+                    r = contact64<KIND>(A, p, k, q, S.node[own], o) ? 1 : 0;
+                    amb = true;
+                  }
+                  hit |= r == 1;
                 }
-                if (r == 2) {  // decide in FP64
-                  r = gap64<KIND>(A, s0, k, q, ox64, o) <= 0.0 ? 1 : 0;
-                  atomicOr(&S.rc[owner], 1u << sj);
-                }
-                hit |= r == 1;
+                // gaps above the cap are reported as +inf: only smaller ones are merged
+                if (want_mg && gmin <= kGapCap) atomicMin(&mgs[32 * j + own], ord_gap(gmin));
               }
-              // gaps above the cap are reported as +inf: only smaller ones are merged
-              if (want_mg && gmin <= kGapCap) atomicMin(&S.mg[sj][owner], ord_gap(gmin));
-              if (hit) {
-                atomicOr(&S.hit[owner], 1u << sj);
-                break;  // later states of this candidate lie past the lane's first contact
+              const unsigned hb = __ballot_sync(kFull, hit), ab = __ballot_sync(kFull, amb);
+              if (hb | ab) {
+                seen |= hb | ab;
+                if (j == 0) {  // the entry's first lane merges its states' bits
+                  const unsigned h = (hb >> (sub * CH)) & kChunkBits, a = (ab >> (sub * CH)) & kChunkBits;
+                  if (h) atomicOr(&S.hit[own], h);
+                  if (a) atomicOr(&S.rc[own], a);
+                }
               }
             }
+            if (seen || want_mg) {
+              __syncwarp();
+              const unsigned h = S.hit[lane], a = S.rc[lane];
+              const int last = h ? __ffs(h) - 1 : CH - 1;
+              if (a & ((2u << last) - 1u)) rechecked = true;
+              if (want_mg) {
+                unsigned mg = mgs[32 * CH + lane];
+                for (int i = 0; i < CH; i++) {
+                  if (i <= last) mg = min(mg, mgs[32 * i + lane]);
+                  mgs[32 * i + lane] = 0xffffffffu;
+                }
+                mgs[32 * CH + lane] = mg;
+              }
+              if (h) {
+                collided = true;
+                fi = k0 + last;
+                if (!need_bounds) live = false;
+              }
+              S.hit[lane] = 0u;
+              S.rc[lane] = 0u;
+            }
           }
+          __syncwarp();  // the next chunk rewrites the list
+        }
+        if (live && j_oob < CH) {  // later states of this lane are never tested
+          oob = true;
+          fi = k0 + j_oob;
+          live = false;
         }
       }
-      __syncwarp();
-      if (n_lane > 0) {
-        const unsigned h = S.hit[lane];
-        const int last = h ? __ffs(h) - 1 : nS - 1;
-        if (want_mg)
-          for (int j = 0; j <= last; j++) mg = fminf(mg, unord_gap(S.mg[j][lane]));
-        if (S.rc[lane] & (last >= 31 ? 0xffffffffu : ((2u << last) - 1u))) rechecked = true;
-        if (h) {
-          collided = true;
-          first_col = k0 + last;
-        }
-      }
-      __syncwarp();  // the next round reuses the scratch
+      __syncwarp();  // the next pass rewrites the slots
     }
-    if (!done && collided && !need_bounds) done = true;
-    k0 = kk;
   }
 
   const unsigned rmask = __ballot_sync(kFull, active && rechecked);
   if (lane == 0 && rmask) atomicAdd(&A.ctr->n_recheck, (unsigned long long)__popc(rmask));
-  if (!active) return;
-  const PairView &o = A.out;
-  if (A.perm) o.node[pair] = A.perm[node];
-  uint8_t verdict;
-  int fi;
-  if (first_oob < L) { verdict = DPG_OUT_OF_BOUNDS; fi = first_oob; }
-  else if (collided) { verdict = DPG_COLLISION; fi = first_col; }
-  else { verdict = DPG_VALID; fi = L; }
-  const int er = first_oob < L ? first_oob : L - 1;  // end-state row
-  const int64_t row_out = o.out_index ? (int64_t)o.out_index[pair] : pair;
-  if (o.node_host) {
-    o.node_host[row_out] = A.perm ? A.perm[node] : node;
-    o.prim_host[row_out] = (uint32_t)p;
+  const uint32_t row_out = active && o.out_index ? o.out_index[pair0 + lane] : pair0 + lane;
+  if (active) {
+    const uint8_t verdict = oob ? DPG_OUT_OF_BOUNDS : (collided ? DPG_COLLISION : DPG_VALID);
+    if (o.verdict) o.verdict[row_out] = verdict;
+    if (o.first_invalid) o.first_invalid[row_out] = (int16_t)fi;
+    if (want_mg) {  // (no gap up to the cap: NaN bits, reported as +inf)
+      const float mg = unord_gap(mgs[32 * CH + lane]);
+      o.min_gap[row_out] = oob ? __int_as_float(0x7fc00000) : (mg <= kGapCap ? mg : __int_as_float(0x7f800000));
+    }
+    if (o.flags) o.flags[row_out] = rechecked ? DPG_FLAG_CONTACT_RECHECK : 0;
   }
-  if (o.verdict) o.verdict[row_out] = verdict;
-  if (o.first_invalid) o.first_invalid[row_out] = (int16_t)fi;
-  if (o.min_gap)
-    o.min_gap[row_out] = verdict == DPG_OUT_OF_BOUNDS ? __int_as_float(0x7fc00000)
-                                                   : (mg <= kGapCap ? mg : __int_as_float(0x7f800000));
-  if (o.flags) o.flags[row_out] = rechecked ? DPG_FLAG_CONTACT_RECHECK : 0;
-  if (o.end_state) {
-    if constexpr (ES64) {
-      double *es = (double *)o.end_state + row_out * R::NX;
-      const double t = double(er) * rp.dt;
-      const double *xs = pv.st64 + (s0 + er) * R::NX;
+  if (!o.end_state) return;
+  // end states: each lane its row, then through shared memory so that the
+  // stores of the item's rows are coalesced
+  using Es = std::conditional_t<ES64, double, float>;
+  Es *es = (Es *)o.end_state;
+  Es v[R::NX];
+  const int er = oob ? fi : L - 1;  // end-state row
+  const int64_t s0 = pv.soff[p];
+  if constexpr (ES64) {
+    const double *st = pv.st64 + (s0 + er) * R::NX;
 #pragma unroll
-      for (int c = 0; c < R::NX; c++) {
-        double v = xs[c];
-        if (c < D) {
-          v += x64[c];
-          if (V) v += t * x64[R::vel_comp(c)];
-        }
+    for (int c = 0; c < R::NX; c++) v[c] = st[c];
+    const double *x64 = A.nv.x64 + (int64_t)node * R::NX;
+    const double t = double(er) * A.rp.dt;
 #pragma unroll
-        for (int i = 0; i < V; i++)
-          if (c == R::vel_comp(i)) v += x64[R::vel_comp(i)];
-        es[c] = v;
-      }
-    } else {
-      float *es = (float *)o.end_state + row_out * R::NX;
-      const float t = float(er) * dt;
-      const int64_t row = s0 + er;
+    for (int i = 0; i < D; i++) {
+      v[i] += x64[i];
+      if (V) v[i] += t * x64[R::vel_comp(i)];
+    }
 #pragma unroll
-      for (int c = 0; c < R::NX; c++) {
-        float v = pv.st32[row * R::NX + c];
-        if (c < D) {
-          v += off[c];
-          if (V) v += t * off[D + c];
-        }
+    for (int i = 0; i < V; i++) v[R::vel_comp(i)] += x64[R::vel_comp(i)];
+  } else {
+    const float4 *st = reinterpret_cast<const float4 *>(pv.st32 + (s0 + er) * R::NXP);
 #pragma unroll
-        for (int i = 0; i < V; i++)
-          if (c == R::vel_comp(i)) v += off[D + i];
-        es[c] = v;
-      }
+    for (int c = 0; c < R::NXP / 4; c++) {
+      const float4 x = st[c];
+      const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (4 * c + i < R::NX) v[4 * c + i] = xs[i];
+    }
+    const float t = float(er) * dt;
+#pragma unroll
+    for (int i = 0; i < D; i++) {
+      v[i] += S.off[i][lane];
+      if constexpr (V > 0) v[i] += t * S.off[D + i][lane];
+    }
+    if constexpr (V > 0) {
+#pragma unroll
+      for (int i = 0; i < V; i++) v[R::vel_comp(i)] += S.off[D + i][lane];
     }
   }
+  if (o.out_index) {  // rows of their own
+    if (active)
+#pragma unroll
+      for (int c = 0; c < R::NX; c++) es[(int64_t)row_out * R::NX + c] = v[c];
+    return;
+  }
+#pragma unroll
+  for (int c = 0; c < R::NX; c++) S.end[lane * R::NX + c] = v[c];
+  __syncwarp();
+  Es *dst = es + (int64_t)pair0 * R::NX;
+#pragma unroll
+  for (int e = 0; e < 32 * R::NX; e += 32)
+    if (e + lane < count * R::NX) dst[e + lane] = S.end[e + lane];
 }
 
 template <class Real, int KIND>
@@ -949,54 +1042,57 @@ __device__ void load_obstacles(const EnvView &ev, void *sm) {
 constexpr unsigned long long kAbortPoll = 64;
 constexpr unsigned long long kNoMoreItems = 1ull << 62;
 
-// Persistent warps over (primitive, 32 nodes) work items.
-// SLOTS: the slot-parallel narrow phase (FP32 tests with the band, NW > 0);
-// its per-warp scratch follows the obstacles at A.slot_offset.
-template <int KIND, class Real, bool BAND, int NW, bool ES64 = false, bool SLOTS = false>
-__global__ void __launch_bounds__(kCheckThreads, SLOTS ? Robot<KIND>::SLOT_BLOCKS : Robot<KIND>::CHECK_BLOCKS)
-    check_pairs(CheckArgs A) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  load_obstacles<Real, KIND>(A.ev, smem);
+// Persistent warps over (primitive, 32 nodes) work items: item(p, pair, count,
+// node) for each, `pair` its first pair, `count` (<= 32) its pairs, `node` the
+// lane's node.
+template <class Item>
+__device__ __forceinline__ void for_items(const CheckArgs &A, Item item_fn) {
   const int lane = threadIdx.x & 31;
-  const int P = A.pv.P;
+  // (items and pairs stay below 2^32: the capacity does)
   const unsigned long long n_all = A.ctr->n_items;
   const int nsub = A.nsub > 0 ? A.nsub : 1;
-  const unsigned long long i_lo = nsub > 1 ? n_all * A.sub_cum[A.sub] / A.sub_cum[nsub] : 0ull;
-  const unsigned long long n_items = nsub > 1 ? n_all * A.sub_cum[A.sub + 1] / A.sub_cum[nsub] : n_all;
-  int cur_range = -1;        // progress-driven copies: the range of this warp's items,
-  unsigned long long cur_cnt = 0;  // and how many of them it finished
+  const uint32_t i_lo = nsub > 1 ? (uint32_t)(n_all * A.sub_cum[A.sub] / A.sub_cum[nsub]) : 0u;
+  const uint32_t n_items = (uint32_t)(nsub > 1 ? n_all * A.sub_cum[A.sub + 1] / A.sub_cum[nsub] : n_all);
+  int cur_range = -1;    // progress-driven copies: the range of this warp's items,
+  uint32_t cur_cnt = 0;  // and how many of them it finished
+  auto range_end = [&](int j) {  // first item past range j
+    return (uint32_t)(A.ctr->n_items * A.sub_cum[j + 1] / A.sub_cum[A.n_ranges]);
+  };
   auto flush_range = [&]() {  // warp-uniform
     if (cur_cnt == 0) return;
     __threadfence();  // this lane's result writes, before the count
     __syncwarp();
     if (lane == 0) {
-      const int nr = A.n_ranges, tot = A.sub_cum[nr], j = cur_range;
-      const unsigned long long lo = n_all * A.sub_cum[j] / tot;
-      const unsigned long long hi = j + 1 == nr ? n_all : n_all * A.sub_cum[j + 1] / tot;
-      if (atomicAdd(&A.ctr->range_done[j], cur_cnt) + cur_cnt == hi - lo) {
+      const int j = cur_range;
+      const uint32_t lo = j > 0 ? range_end(j - 1) : 0u, hi = range_end(j);
+      if (atomicAdd(&A.ctr->range_done[j], (unsigned long long)cur_cnt) + cur_cnt == hi - lo) {
         __threadfence_system();
         reinterpret_cast<volatile int *>(A.range_flag)[j] = 1;
       }
     }
     cur_cnt = 0;
   };
-  while (true) {
-    unsigned long long item = 0;
+  // the next item is drawn while the current one is checked
+  uint32_t next = 0;
+  auto draw = [&]() {
     if (lane == 0) {
       const unsigned long long drawn = atomicAdd(&A.ctr->next_sub[A.sub], 1ull);
-      item = i_lo + drawn;
-      if (item < n_items && drawn % kAbortPoll == 0 && *A.abort_flag) {
+      next = drawn < n_items - i_lo ? i_lo + (uint32_t)drawn : n_items;
+      if (next < n_items && drawn % kAbortPoll == 0 && *A.abort_flag) {
         A.ctr->status = DPG_ERR_ABORTED;  // every warp's next item lies past the end
         atomicMax(&A.ctr->next_sub[A.sub], kNoMoreItems);
-        item = n_items;
+        next = n_items;
       }
     }
-    item = __shfl_sync(kFull, item, 0);
+  };
+  draw();
+  while (true) {
+    const uint32_t item = __shfl_sync(kFull, next, 0);
     if (item >= n_items) break;
+    draw();
     if (A.n_ranges > 1) {
-      const int nr = A.n_ranges, tot = A.sub_cum[nr];
       int j = 0;
-      while (j + 1 < nr && item >= n_all * A.sub_cum[j + 1] / tot) j++;
+      while (j + 1 < A.n_ranges && item >= range_end(j)) j++;
       if (j != cur_range) {
         flush_range();
         cur_range = j;
@@ -1008,28 +1104,43 @@ __global__ void __launch_bounds__(kCheckThreads, SLOTS ? Robot<KIND>::SLOT_BLOCK
     if (A.item_pos) {
       lo = (int)A.item_pos[item];
     } else {
-      int hi = P;
+      int hi = A.pv.P;
       while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
         if (A.ord_ibase[mid] <= item) lo = mid; else hi = mid;
       }
     }
     const int p = A.pv.order[lo];
-    const unsigned long long j = item - A.ord_ibase[lo];
-    const unsigned long long first = A.ord_pbase[lo] + 32ull * j;
-    const unsigned long long end = A.ord_pbase[lo + 1];
-    const unsigned long long pair = first + lane;
-    const bool active = pair < end;
-    const uint32_t node = active ? A.out.node[pair] : 0u;
-    if constexpr (SLOTS) {
-      using Scratch = SlotScratch<Robot<KIND>::CHUNK, Robot<KIND>::PARTS, NW>;
-      Scratch *scr = reinterpret_cast<Scratch *>(smem + A.slot_offset) + (threadIdx.x >> 5);
-      check_one_slots<KIND, NW, ES64>(A, smem, *scr, p, (int64_t)pair, node, active);
-    } else {
-      check_one<KIND, Real, BAND, NW, true, ES64>(A, smem, p, (int64_t)pair, node, active);
-    }
+    const uint32_t first = (uint32_t)(A.ord_pbase[lo] + 32ull * (item - A.ord_ibase[lo]));
+    const int count = (int)min(32u, (uint32_t)A.ord_pbase[lo + 1] - first);
+    const uint32_t node = lane < count ? A.out.node[first + lane] : 0u;
+    item_fn(p, first, count, node);
   }
   if (A.n_ranges > 1) flush_range();
+}
+
+// lockstep walk
+template <int KIND, class Real, bool BAND, int NW, bool ES64 = false>
+__global__ void __launch_bounds__(kCheckThreads, Robot<KIND>::CHECK_BLOCKS) check_pairs(CheckArgs A) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  load_obstacles<Real, KIND>(A.ev, smem);
+  const int lane = threadIdx.x & 31;
+  for_items(A, [&](int p, uint32_t pair, int count, uint32_t node) {
+    check_one<KIND, Real, BAND, NW, true, ES64>(A, smem, p, (int64_t)pair + lane, node, lane < count);
+  });
+}
+
+// slot-parallel tests (FP32 with the band); the warps' scratch follows the
+// obstacles at A.slot_offset, A.slot_stride bytes apart
+template <int KIND, bool ES64>
+__global__ void __launch_bounds__(kCheckThreads, Robot<KIND>::SLOT_BLOCKS) check_pairs_slots(CheckArgs A) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  load_obstacles<float, KIND>(A.ev, smem);
+  auto &scr = *reinterpret_cast<SlotScratch<KIND, ES64> *>(smem + A.slot_offset + (threadIdx.x >> 5) * A.slot_stride);
+  for_items(A, [&](int p, uint32_t pair, int count, uint32_t node) {
+    check_item<KIND, ES64>(A, smem, scr, p, pair, count, node);
+    __syncwarp();  // the next item rewrites the scratch
+  });
 }
 
 }  // namespace dpg

@@ -97,6 +97,16 @@ int off_dim(int kind) {
     default: return 2;
   }
 }
+int padded_dim(int kind) {  // floats of a row of st32
+  int n = 0;
+  switch (kind) {
+    case DPG_ROBOT_UNICYCLE1: n = Robot<DPG_ROBOT_UNICYCLE1>::NXP; break;
+    case DPG_ROBOT_CAR1: n = Robot<DPG_ROBOT_CAR1>::NXP; break;
+    case DPG_ROBOT_QUAD2D: n = Robot<DPG_ROBOT_QUAD2D>::NXP; break;
+    case DPG_ROBOT_QUAD3D: n = Robot<DPG_ROBOT_QUAD3D>::NXP; break;
+  }
+  return n;
+}
 bool is_rollout(int kind) { return kind == DPG_ROBOT_QUAD2D || kind == DPG_ROBOT_QUAD3D; }
 
 // dispatch a functor templated on the robot kind
@@ -127,10 +137,7 @@ static void launch_check(dpg_ctx *c, const CheckArgs &ca, int prec, cudaStream_t
   const size_t ob = fp64 ? (R::SPHERE ? sizeof(Obs3<double>) : sizeof(Obs2<double>))
                          : (R::SPHERE ? sizeof(Obs3<float>) : sizeof(Obs2<float>));
   const size_t sm_obs = (ob * std::max(c->n_obs, 1) + 15) / 16 * 16;
-  // the slot-parallel narrow phase for FP32 tests with culling
-  const bool slots = !fp64 && nw > 0 && c->tune.check_variant == DPG_CHECK_SLOTS;
   CheckArgs a = ca;
-  a.slot_offset = (int)sm_obs;
   auto go = [&](auto kern, size_t scratch = 0) {
     const size_t sm = sm_obs + scratch * (kCheckThreads / 32);
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -139,15 +146,24 @@ static void launch_check(dpg_ctx *c, const CheckArgs &ca, int prec, cudaStream_t
     if (c->tune.check_blocks_per_sm > 0) per_sm = std::min(per_sm, c->tune.check_blocks_per_sm);
     kern<<<c->sm_count * std::max(per_sm, 1), kCheckThreads, sm, st>>>(a);
   };
+  // the slot-parallel tests: FP32 with the band, an item's slots listed
+  if (!fp64 && c->n_obs <= kSlotCap && c->tune.check_variant == DPG_CHECK_SLOTS) {
+    const bool gap = ca.out.min_gap != nullptr, es64 = prec == DPG_FP64;
+    const size_t scratch = es64 ? slot_scratch_bytes<KIND, true>(gap) : slot_scratch_bytes<KIND, false>(gap);
+    a.slot_offset = (int)sm_obs;
+    a.slot_stride = (int)scratch;
+    if (es64) go(check_pairs_slots<KIND, true>, scratch);
+    else go(check_pairs_slots<KIND, false>, scratch);
+    return;
+  }
   auto by_words = [&](auto real, auto band, auto es64) {
     using Real = decltype(real);
     constexpr bool BAND = decltype(band)::value, ES64 = decltype(es64)::value;
-    constexpr bool F32 = sizeof(Real) == 4;
     switch (nw) {
-      case 1: slots ? go(check_pairs<KIND, Real, BAND, 1, ES64, F32>, slot_scratch_bytes<KIND, 1>()) : go(check_pairs<KIND, Real, BAND, 1, ES64>); break;
-      case 2: slots ? go(check_pairs<KIND, Real, BAND, 2, ES64, F32>, slot_scratch_bytes<KIND, 2>()) : go(check_pairs<KIND, Real, BAND, 2, ES64>); break;
-      case 3: slots ? go(check_pairs<KIND, Real, BAND, 3, ES64, F32>, slot_scratch_bytes<KIND, 3>()) : go(check_pairs<KIND, Real, BAND, 3, ES64>); break;
-      case 4: slots ? go(check_pairs<KIND, Real, BAND, 4, ES64, F32>, slot_scratch_bytes<KIND, 4>()) : go(check_pairs<KIND, Real, BAND, 4, ES64>); break;
+      case 1: go(check_pairs<KIND, Real, BAND, 1, ES64>); break;
+      case 2: go(check_pairs<KIND, Real, BAND, 2, ES64>); break;
+      case 3: go(check_pairs<KIND, Real, BAND, 3, ES64>); break;
+      case 4: go(check_pairs<KIND, Real, BAND, 4, ES64>); break;
       default: go(check_pairs<KIND, Real, BAND, 0, ES64>); break;
     }
   };
@@ -470,7 +486,7 @@ static int load_tables(dpg_ctx *c, int32_t P, const int32_t *len, const double *
       (rc = ensure(c, c->key32, sizeof(float) * kd * P)) ||
       (rc = ensure(c, c->kconst32, sizeof(float) * P)) ||
       (rc = ensure(c, c->st64, sizeof(double) * nx * S)) ||
-      (rc = ensure(c, c->st32, sizeof(float) * nx * S)) ||
+      (rc = ensure(c, c->st32, sizeof(float) * padded_dim(kind) * S)) ||
       (rc = ensure(c, c->act64, sizeof(double) * nu * std::max<int64_t>(A, 1))) ||
       (rc = ensure(c, c->pose32, sizeof(Pose<float>) * parts * S)) ||
       (rc = ensure(c, c->pose64, sizeof(Pose<double>) * parts * S)) ||
@@ -869,7 +885,7 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
   ca.half_wid32 = (float)rp.half_wid;
   ca.radius32 = (float)rp.radius;
   ca.band32 = (float)ca.band;
-  for (int i = 0; i < 3; i++) { ca.lo32[i] = (float)c->lo[i]; ca.hi32[i] = (float)c->hi[i]; }
+  set_bounds(ca, c->lo, c->hi);
 
   cudaError_t launch_err = cudaSuccess;
   with_kind(kind, [&](auto K) {
@@ -1220,7 +1236,7 @@ int dpg_expand_noalloc(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const
   ca.half_wid32 = (float)rp.half_wid;
   ca.radius32 = (float)rp.radius;
   ca.band32 = (float)ca.band;
-  for (int i = 0; i < 3; i++) { ca.lo32[i] = (float)c->lo[i]; ca.hi32[i] = (float)c->hi[i]; }
+  set_bounds(ca, c->lo, c->hi);
 
   cudaError_t launch_err = cudaSuccess;
   with_kind(kind, [&](auto K) {
@@ -1344,7 +1360,7 @@ CheckArgs ctx_check_args(dpg_ctx *c, int prec, double contact_band, const NodeVi
   ca.half_wid32 = (float)rp.half_wid;
   ca.radius32 = (float)rp.radius;
   ca.band32 = (float)ca.band;
-  for (int i = 0; i < 3; i++) { ca.lo32[i] = (float)c->lo[i]; ca.hi32[i] = (float)c->hi[i]; }
+  set_bounds(ca, c->lo, c->hi);
   return ca;
 }
 

@@ -69,7 +69,7 @@ struct PrimView {
   const float *key32;        // [KEYD][P] kept key components, angles wrapped
   const float *kconst32;     // [P] constant part of the metric
   const double *st64;        // [S][NX] canonical states (row-major)
-  const float *st32;         // [S][NX]
+  const float *st32;         // [S][NXP]: rows padded to whole 16-byte vectors
   const Pose<float> *pose32; // [PARTS][S] (3-D: cx,cy,c = position, s unused)
   const Pose<double> *pose64;
   const double *pbox;        // [P][2*POSD]: lo..., hi... of the state positions
@@ -618,7 +618,7 @@ __global__ void build_poses(RobotParams rp, int64_t S, const double *st64, Pose<
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= S) return;
   const double *x = st64 + s * R::NX;
-  for (int c = 0; c < R::NX; c++) st32[s * R::NX + c] = (float)x[c];
+  for (int c = 0; c < R::NXP; c++) st32[s * R::NXP + c] = c < R::NX ? (float)x[c] : 0.f;
   Pose<double> ps[2];
   if constexpr (R::SPHERE) {
     ps[0] = Pose<double>{x[0], x[1], x[2], 0.0};

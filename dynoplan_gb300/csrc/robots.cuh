@@ -37,49 +37,49 @@ struct RobotParams {
 template <int KIND> struct Robot;
 
 template <> struct Robot<DPG_ROBOT_UNICYCLE1> {
-  static constexpr int NX = 3, NU = 2, PARTS = 1, POSD = 2, VELOFF = 0;
+  static constexpr int NX = 3, NXP = 4, NU = 2, PARTS = 1, POSD = 2, VELOFF = 0;
   static constexpr bool ROLLOUT = false, SPHERE = false;
   static constexpr int KEYD = 1;  // kept key components: theta
   static constexpr int CHUNK = 8;  // states per culling chunk
   static constexpr int CHECK_BLOCKS = 4;  // check_pairs blocks per SM (register bound)
   static constexpr int SLOT_BLOCKS = 4;  // slot-parallel check: 64 registers a thread
-  static constexpr bool BOUNDS_SLOTS = false;  // bounds tests walked per lane (the slot form: car1 2.07 -> 2.28 ms)
+  static constexpr int WINDOW = 8;  // chunks whose slots are listed together
   __host__ __device__ static int key_comp(int i) { return 2; }
   __host__ __device__ static int vel_comp(int i) { return -1; }
 };
 
 template <> struct Robot<DPG_ROBOT_CAR1> {
-  static constexpr int NX = 4, NU = 2, PARTS = 2, POSD = 2, VELOFF = 0;
+  static constexpr int NX = 4, NXP = 4, NU = 2, PARTS = 2, POSD = 2, VELOFF = 0;
   static constexpr bool ROLLOUT = false, SPHERE = false;
   static constexpr int KEYD = 2;  // theta0, theta1
   static constexpr int CHUNK = 8;
   static constexpr int CHECK_BLOCKS = 4;  // measured: 4 beats 3, 5 and 6 here
   static constexpr int SLOT_BLOCKS = 4;  // slot-parallel check: 64 registers a thread
-  static constexpr bool BOUNDS_SLOTS = false;  // bounds tests walked per lane (the slot form: car1 2.07 -> 2.28 ms)
+  static constexpr int WINDOW = 8;  // chunks whose slots are listed together
   __host__ __device__ static int key_comp(int i) { return 2 + i; }
   __host__ __device__ static int vel_comp(int i) { return -1; }
 };
 
 template <> struct Robot<DPG_ROBOT_QUAD2D> {
-  static constexpr int NX = 6, NU = 2, PARTS = 1, POSD = 2, VELOFF = 2;
+  static constexpr int NX = 6, NXP = 8, NU = 2, PARTS = 1, POSD = 2, VELOFF = 2;
   static constexpr bool ROLLOUT = true, SPHERE = false;
   static constexpr int KEYD = 2;  // theta, w
   static constexpr int CHUNK = 16;  // dt 0.01: ten times the states of the others per second
   static constexpr int CHECK_BLOCKS = 4;
   static constexpr int SLOT_BLOCKS = 4;  // slot-parallel check: 64 registers a thread
-  static constexpr bool BOUNDS_SLOTS = false;  // bounds tests walked per lane
+  static constexpr int WINDOW = 8;  // chunks whose slots are listed together
   __host__ __device__ static int key_comp(int i) { return i == 0 ? 2 : 5; }
   __host__ __device__ static int vel_comp(int i) { return 3 + i; }
 };
 
 template <> struct Robot<DPG_ROBOT_QUAD3D> {
-  static constexpr int NX = 13, NU = 4, PARTS = 1, POSD = 3, VELOFF = 3;
+  static constexpr int NX = 13, NXP = 16, NU = 4, PARTS = 1, POSD = 3, VELOFF = 3;
   static constexpr bool ROLLOUT = true, SPHERE = true;
   static constexpr int KEYD = 7;  // quaternion (4), w (3)
   static constexpr int CHUNK = 16;
   static constexpr int CHECK_BLOCKS = 5;  // measured: 5 beats 4 and 6 here
   static constexpr int SLOT_BLOCKS = 4;  // slot-parallel check: 64 registers a thread
-  static constexpr bool BOUNDS_SLOTS = true;   // bounds tests as (lane, state) slots when few lanes need them (11.45 -> 10.65 ms)
+  static constexpr int WINDOW = 4;  // chunks whose slots are listed together
   __host__ __device__ static int key_comp(int i) { return i < 4 ? 3 + i : 6 + i; }
   __host__ __device__ static int vel_comp(int i) { return 7 + i; }
 };
