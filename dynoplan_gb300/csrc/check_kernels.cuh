@@ -503,48 +503,60 @@ __device__ void check_one(const CheckArgs &A, const void *obs_sm, int p, int64_t
 //     obstacles near any lane (a lane per obstacle, one ballot per 32), each of
 //     these is tested against the 32 lanes' boxes, and the lanes it is near to
 //     append their slots;
-//   - a lane per slot tests its obstacle against the boxes of the window's
-//     chunks at its owner's offset (a bit per chunk);
-//   - chunk by chunk, the near slots are listed and tested with a lane per
-//     (entry, state), 32 / CHUNK entries a step; the lane keeps its state's
-//     poses for the whole chunk.
-// Contacts and FP64 decisions come back as ballots and are merged per owner
-// (shared words, one atomic per entry with a contact); each lane then folds
-// the states up to its first contact, which gives exactly the per-state
+//   - a lane per slot tests its obstacle against the boxes of each part over
+//     the window's chunks at its owner's offset (a bit per chunk and part);
+//   - the bounds are tested with a lane per (lane, state of a chunk);
+//   - the near (slot, part, chunk) entries are listed in the chunks' order and
+//     tested with a lane per (entry, state), 32 / CHUNK entries a step, up to
+//     the owner's first state out of bounds.
+// Per lane the first state out of bounds, the first contact and the first FP64
+// decisions are kept in shared memory (one atomic per entry with a contact):
+// decisions after the first contact do not count, which gives exactly the
 // results of the sequential walk (every candidate is tested at every state up
-// to the first contact, no state from the first one out of bounds on).  FP32
-// tests with FP64 decisions in the band.
+// to the first contact).  FP32 tests with FP64 decisions in the band.
 //
-// Bound by instruction issue (ncu, car1, 50,000 nodes: 75 % of the issue slots,
-// 27.6 active lanes an instruction, 5,200 warp instructions an item).  Against
-// the earlier form, which dealt (lane, chunk, obstacle) slots out and walked a
-// slot's states in one lane (17.7 active lanes, 6,800 instructions, spills):
-// check kernel of car1 (100,000 x 5,000) 1.91 -> 1.34 ms, quadrotor (50,000 x
-// 5,000) 10.6 -> 6.6 ms, unicycle1 FP64 0.127 -> 0.106 ms, a search round of
-// quad2d (32 x 10,000) 0.168 -> 0.121 ms.  Measured beside it: each lane walking
-// its own states for the bounds tests when many lanes need them, quadrotor
-// 6.6 -> 8.7 ms; 3 blocks an SM at 80 registers car1 1.40 ms, 5 at 48 (spills)
-// 2.01 ms; chunks of 8 or 32 states for the quadrotor 6.65 and 8.9 ms.
-// The end states go out through shared memory: rows of 52 bytes written by a
-// lane each cost the quadrotor 2.2 ms.
+// Bound by instruction issue (75 % of the issue slots on car1, 27.6 active
+// lanes an instruction; its table reads hit L1 / L2).  Check kernel, ms, against
+// the form that dealt (lane, chunk, obstacle) slots out and walked a slot's
+// states in one lane (17.7 active lanes), and against the first form of this
+// one (a box for all parts of a chunk, bounds and tests chunk by chunk, every
+// axis of an ambiguous test in FP64):
+//   car1 100,000 x 5,000          1.91   1.34   1.03
+//   quadrotor 50,000 x 5,000     10.6    6.6    5.2
+//   unicycle1 FP64 10,000 x 1,000 0.127  0.106  0.098
+//   quad2d 32 x 10,000            0.168  0.121  0.102
+// Measured beside it: a lane walking its own states in the bounds tests when
+// many lanes need them, quadrotor 6.6 -> 8.7; entries of several chunks listed
+// before they are tested (fuller steps, but lanes past their contact), car1
+// 1.06 at 4 entries, 1.08 at 12, 1.36 at 32; windows of 8 chunks instead of 4
+// car1 1.06, of 4 instead of 2 the quadrotor 5.26; chunks of 8 or 32 states for
+// the quadrotor 6.65 and 8.9 (first form); 3 blocks an SM car1 1.18, 5 (spills)
+// 1.75.  End-state rows of 52 bytes written by a lane each cost the quadrotor
+// 2.2 ms: they go out through shared memory.
 
 constexpr int kSlotCap = 512;  // slots of a window held at a time; also the most obstacles of this variant
+constexpr int kListCap = 160;  // entries held at a time
+constexpr int kListMin = 4;    // entries from which a listed chunk is tested at once
+constexpr int kNever = 0x7fffffff;
 
 template <int KIND, bool ES64> struct SlotScratch {
   static constexpr int C = Robot<KIND>::POSD + Robot<KIND>::VELOFF;
   using Es = std::conditional_t<ES64, double, float>;
   union {
     struct {
-      uint16_t slot[kSlotCap];   // obstacle << 5 | lane
-      uint16_t list[kSlotCap];   // a chunk's entries
-      uint8_t near_[kSlotCap];   // the window's chunks the slot's obstacle is near to
+      // chunk of the window << 16 | part << 14 | obstacle << 5 | lane; bounds: chunk << 16 | lane
+      uint32_t list[kListCap];
+      uint16_t slot[kSlotCap];  // obstacle << 5 | lane
+      std::conditional_t<Robot<KIND>::PARTS == 1, uint8_t, uint16_t>
+          near_[kSlotCap];  // the window's chunks (8 bits a part) the slot's obstacle is near to
     };
     Es end[32 * Robot<KIND>::NX];  // the item's end states on their way out
   };
   float off[C][32];  // the lanes' node offsets
   uint32_t node[32];
-  unsigned hit[32];  // per lane: bit j = contact at state j of the chunk
-  unsigned rc[32];   // per lane: bit j = a test at state j was decided in FP64
+  // per lane, the first state: out of bounds (L: none), with a contact, with a
+  // bounds / an obstacle test decided in FP64 (kNever: none)
+  int oob[32], contact[32], oob_amb[32], contact_amb[32];
 };
 // (with the min_gap output the warp's scratch is followed by (CHUNK + 1) x 32
 // words: per state of the chunk and lane, the min axis-aligned gap as ordered
@@ -563,10 +575,42 @@ __device__ __forceinline__ float unord_gap(unsigned u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-// FP64 decision of an ambiguous obstacle test (rare: kept out of line)
+// FP64 decision of an ambiguous obstacle test of part q at state k (rare: kept
+// out of line).  Planar robots: an axis whose FP32 gap (px, py, c, s: the FP32
+// pose) is below the band by more than the FP32 error is below zero in FP64
+// too, so only the others, usually one, are evaluated (all four: 27 FP64
+// instructions at 16 SM cycles each, an eighth of car1's check).
 template <int KIND>
-__device__ __noinline__ bool contact64(const CheckArgs &A, int p, int k, int q, uint32_t node, int o) {
-  return gap64<KIND>(A, A.pv.soff[p], k, q, A.nv.x64 + (int64_t)node * Robot<KIND>::NX, o) <= 0.0;
+__device__ __noinline__ bool contact64(const CheckArgs &A, int p, int k, int q, uint32_t node, int o, float px,
+                                       float py, float c, float s) {
+  using R = Robot<KIND>;
+  const double *x64 = A.nv.x64 + (int64_t)node * R::NX;
+  const int64_t s0 = A.pv.soff[p];
+  if constexpr (R::SPHERE) {
+    return gap64<KIND>(A, s0, k, q, x64, o) <= 0.0;
+  } else {
+    const Obs2<float> of = ((const Obs2<float> *)A.ev.obs32)[o];
+    const Obs2<double> ob = ((const Obs2<double> *)A.ev.obs64)[o];
+    const Pose<double> ps = A.pv.pose64[q * A.pv.S + s0 + k];
+    const float a32 = A.half_len32, b32 = A.half_wid32, fc = fabsf(c), fs = fabsf(s), dxf = px - of.cx, dyf = py - of.cy;
+    const float cut = -(A.band32 + 1e-4f + 1e-6f * (fabsf(px) + fabsf(py)));
+    double sx = x64[0], sy = x64[1];
+    if (R::VELOFF) {
+      const double t = double(k) * A.rp.dt;
+      sx += t * x64[R::vel_comp(0)];
+      sy += t * x64[R::vel_comp(1)];
+    }
+    const double a = A.rp.half_len, b = A.rp.half_wid, ac = fabs(ps.c), as = fabs(ps.s);
+    const double dx = ps.cx + sx - ob.cx, dy = ps.cy + sy - ob.cy;
+    bool in = true;
+    if (fabsf(dxf) - (a32 * fc + b32 * fs + of.hx) > cut) in = fabs(dx) - (a * ac + b * as + ob.hx) <= 0.0;
+    if (in && fabsf(dyf) - (a32 * fs + b32 * fc + of.hy) > cut) in = fabs(dy) - (a * as + b * ac + ob.hy) <= 0.0;
+    if (in && fabsf(dxf * c + dyf * s) - (a32 + of.hx * fc + of.hy * fs) > cut)
+      in = fabs(dx * ps.c + dy * ps.s) - (a + ob.hx * ac + ob.hy * as) <= 0.0;
+    if (in && fabsf(dyf * c - dxf * s) - (b32 + of.hx * fs + of.hy * fc) > cut)
+      in = fabs(-dx * ps.s + dy * ps.c) - (b + ob.hx * as + ob.hy * ac) <= 0.0;
+    return in;
+  }
 }
 // FP64 decision of an ambiguous bounds test of position component i
 template <int KIND>
@@ -615,6 +659,12 @@ __device__ __forceinline__ void load_box(const float *box, float *c, float *h) {
   }
 }
 
+// This lane is the first of its group of CH lanes in the ballot m (it is one of m).
+template <int CH>
+__device__ __forceinline__ bool first_of_group(unsigned m, int lane) {
+  return ((m >> (lane & ~(CH - 1))) & ((1u << (lane & (CH - 1))) - 1u)) == 0u;
+}
+
 template <int KIND, bool ES64>
 __device__ __forceinline__ void check_item(const CheckArgs &A, const void *obs_sm, SlotScratch<KIND, ES64> &S, int p,
                                            uint32_t pair0, int count, uint32_t node) {
@@ -622,7 +672,6 @@ __device__ __forceinline__ void check_item(const CheckArgs &A, const void *obs_s
   using Ob = std::conditional_t<R::SPHERE, Obs3<float>, Obs2<float>>;
   constexpr int D = R::POSD, V = R::VELOFF, CH = R::CHUNK, PARTS = R::PARTS, WIN = R::WINDOW;
   constexpr int NE = 32 / CH;  // entries a step tests at once
-  constexpr unsigned kChunkBits = CH == 32 ? 0xffffffffu : (1u << CH) - 1u;
   static_assert(32 % CH == 0 && WIN <= 8, "a lane per (entry, state); a byte of chunk bits");
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
@@ -641,8 +690,8 @@ __device__ __forceinline__ void check_item(const CheckArgs &A, const void *obs_s
   for (int i = 0; i < V; i++)
     S.off[D + i][lane] = active ? node_off<float>(A.nv, node, D + i, R::NX, R::vel_comp(i)) : 0.f;
   S.node[lane] = node;
-  S.hit[lane] = 0u;
-  S.rc[lane] = 0u;
+  S.oob[lane] = L;
+  S.contact[lane] = S.oob_amb[lane] = S.contact_amb[lane] = kNever;
   if (want_mg)
     for (int i = 0; i <= CH; i++) mgs[32 * i + lane] = 0xffffffffu;
   if (active && (A.perm || o.node_host)) {  // the pair's node in the caller's numbering
@@ -674,12 +723,10 @@ __device__ __forceinline__ void check_item(const CheckArgs &A, const void *obs_s
     need_bounds = active && !inside;
   }
 
-  bool live = active, collided = false, rechecked = false;
-  bool oob = false;
-  int fi = L;  // first state out of bounds, else first contact, else L
+  bool live = active, collided = false;
   const int j = lane % CH, sub = lane / CH;  // this lane's state of a chunk and its entry of a step
   const Pose<float> *pose = pv.pose32 + pv.soff[p];
-  const float *cbox = pv.cbox32 + pv.coff[p] * 2 * D;
+  const float *cbox = pv.cbox32 + pv.coff[p] * 2 * D, *qbox = pv.qbox32 + pv.coff[p] * (PARTS * 2 * D);
   __syncwarp();
 
   for (int c0 = 0; c0 < n_chunks; c0 += WIN) {
@@ -721,7 +768,7 @@ __device__ __forceinline__ void check_item(const CheckArgs &A, const void *obs_s
           if (!in) nbw |= 1u << c;
         }
       }
-      if (!need_bounds) nbw = 0u;
+      if (!(live && need_bounds)) nbw = 0u;
       const float tm0 = float(c0 * CH) * dt, tm1 = float(min(L, (c0 + nc) * CH) - 1) * dt;
 #pragma unroll
       for (int i = 0; i < D; i++) {
@@ -734,14 +781,44 @@ __device__ __forceinline__ void check_item(const CheckArgs &A, const void *obs_s
         }
       }
     }
+
+    // bounds: the (lane, chunk) entries of each chunk, tested with a lane per
+    // (entry, state), so that a lane out of bounds has none in later chunks
+    if (any_nb) {
+      for (unsigned todo = __reduce_or_sync(kFull, nbw); todo; todo &= todo - 1) {
+        const int c = __ffs(todo) - 1, k = (c0 + c) * CH + j;
+        const bool nb = ((nbw >> c) & 1u) && S.oob[lane] == L;
+        const unsigned nbm = __ballot_sync(kFull, nb);
+        if (!nbm) continue;
+        const Pose<float> ps = pose[min(k, L - 1)];
+        const int n = __popc(nbm);
+        if (nb) S.list[__popc(nbm & lt)] = (uint32_t)lane;
+        __syncwarp();
+        for (int i0 = 0; i0 < n; i0 += NE) {
+          const int i = i0 + sub;
+          bool out = false, amb = false;
+          int own = 0;
+          if (i < n && k < L) {
+            own = (int)S.list[i];
+            out = out_of_bounds<KIND>(A, S, ps, p, k, own, amb);
+          }
+          const unsigned ow = __ballot_sync(kFull, out), aw = __ballot_sync(kFull, amb);
+          if (out && first_of_group<CH>(ow, lane)) S.oob[own] = k;
+          if (aw && amb && first_of_group<CH>(aw, lane)) atomicMin(&S.oob_amb[own], k);
+        }
+        __syncwarp();
+      }
+    }
+
     // (usually one pass: all lanes; more slots than the list holds: as many
     // lanes as fit, then the others)
+    rest = __ballot_sync(kFull, live && !collided);
     while (rest) {
       unsigned take = rest;
       int n_slot;
       while (true) {
         n_slot = 0;
-        const bool inc = ((take >> lane) & 1u) && !collided;
+        const bool inc = (take >> lane) & 1u;
         // union of the lanes' boxes, a little wider than their own tests (a
         // lane with a NaN offset is near no obstacle and stays out of it)
         float ulo[D], uhi[D];
@@ -763,11 +840,11 @@ __device__ __forceinline__ void check_item(const CheckArgs &A, const void *obs_s
             if constexpr (D == 3) u = u && ob.cz + ob.hz >= ulo[2] && ob.cz - ob.hz <= uhi[2];
           }
           for (unsigned m = __ballot_sync(kFull, u); m; m &= m - 1) {
-            const int o = w0 + __ffs(m) - 1;
-            const bool h = inc && near_box<D, float>(cen, hf, obs_sm, o, M);
+            const int ob = w0 + __ffs(m) - 1;
+            const bool h = inc && near_box<D, float>(cen, hf, obs_sm, ob, M);
             const unsigned hm = __ballot_sync(kFull, h);
             const int pos = n_slot + __popc(hm & lt);
-            if (h && pos < kSlotCap) S.slot[pos] = (uint16_t)(o << 5 | lane);
+            if (h && pos < kSlotCap) S.slot[pos] = (uint16_t)(ob << 5 | lane);
             n_slot += __popc(hm);
           }
         }
@@ -797,156 +874,124 @@ __device__ __forceinline__ void check_item(const CheckArgs &A, const void *obs_s
         unsigned near = 0u;
 #pragma unroll 4
         for (int c = 0; c < nc; c++) {
-          float cc[D], ch[D];
-          load_box<D>(cbox + (c0 + c) * 2 * D, cc, ch);
-          bool in = true;
-          if constexpr (V > 0) {
-            const int k0 = (c0 + c) * CH, k1 = min(L, k0 + CH) - 1;
-            const float tm = 0.5f * dt * float(k0 + k1), th = 0.5f * dt * float(k1 - k0);
 #pragma unroll
-            for (int i = 0; i < D; i++) in = in && fabsf(cc[i] + tm * v[i] + r[i]) <= ch[i] + th * fabsf(v[i]) + h[i];
-          } else {
+          for (int q = 0; q < PARTS; q++) {
+            float cc[D], ch[D];
+            load_box<D>(qbox + ((c0 + c) * PARTS + q) * 2 * D, cc, ch);
+            bool in = true;
+            if constexpr (V > 0) {
+              const int k0 = (c0 + c) * CH, k1 = min(L, k0 + CH) - 1;
+              const float tm = 0.5f * dt * float(k0 + k1), th = 0.5f * dt * float(k1 - k0);
 #pragma unroll
-            for (int i = 0; i < D; i++) in = in && fabsf(cc[i] + r[i]) <= ch[i] + h[i];
+              for (int i = 0; i < D; i++) in = in && fabsf(cc[i] + tm * v[i] + r[i]) <= ch[i] + th * fabsf(v[i]) + h[i];
+            } else {
+#pragma unroll
+              for (int i = 0; i < D; i++) in = in && fabsf(cc[i] + r[i]) <= ch[i] + h[i];
+            }
+            if (in) near |= 1u << (8 * q + c);
           }
-          if (in) near |= 1u << c;
         }
-        S.near_[b] = (uint8_t)near;
+        S.near_[b] = near;
         near_any |= near;
       }
       near_any = __reduce_or_sync(kFull, near_any);
+      if (PARTS > 1) near_any = (near_any | near_any >> 8) & 0xffu;
       __syncwarp();
 
-      const bool mine = (take >> lane) & 1u;  // a lane of this pass
-      for (unsigned todo = near_any | __reduce_or_sync(kFull, mine ? nbw : 0u); todo; todo &= todo - 1) {
-        const int c = __ffs(todo) - 1, k0 = (c0 + c) * CH, kend = min(L, k0 + CH);
-        const unsigned nbm = __ballot_sync(kFull, mine && live && ((nbw >> c) & 1u));
-        const unsigned chk_m = ((near_any >> c) & 1u) ? __ballot_sync(kFull, mine && live && !collided) : 0u;
-        if (!(nbm | chk_m)) continue;
-        const int k = k0 + j;
-
-        // bounds tests of the chunk's states: a lane per (lane, state)
-        int j_oob = CH;
-        if (nbm) {
-          const bool nb = (nbm >> lane) & 1u;
-          unsigned out_bits = 0u, rc_bits = 0u;
-          const Pose<float> ps = pose[min(k, L - 1)];
-          const int rank = __popc(nbm & lt), n = __popc(nbm);
-          if (nb) S.list[rank] = (uint16_t)lane;
-          __syncwarp();
-          for (int it = 0; it * NE < n; it++) {
-            const int i = it * NE + sub;
-            bool out = false, amb = false;
-            if (i < n && k < kend) out = out_of_bounds<KIND>(A, S, ps, p, k, S.list[i], amb);
-            const unsigned ow = __ballot_sync(kFull, out), aw = __ballot_sync(kFull, amb);
-            if (nb && rank / NE == it) {
-              out_bits = (ow >> (rank % NE * CH)) & kChunkBits;
-              rc_bits = (aw >> (rank % NE * CH)) & kChunkBits;
-            }
-          }
-          __syncwarp();
-          if (out_bits) j_oob = __ffs(out_bits) - 1;
-          if (rc_bits & (out_bits ? (2u << j_oob) - 1u : 0xffffffffu)) rechecked = true;
-        }
-
-        // obstacle tests: a lane per (near slot, state)
-        if (chk_m) {
-          const int nst = min(kend - k0, j_oob);  // states of the chunk to test
-          int n_ent = 0;
-          for (int b = 0; b < n_slot; b += 32) {
-            bool in = b + lane < n_slot && ((S.near_[b + lane] >> c) & 1u);
-            const unsigned e = in ? S.slot[b + lane] : 0u;
-            in = in && ((chk_m >> (e & 31u)) & 1u);
+      // obstacle tests: the near (slot, part) entries of the chunks in order,
+      // listed until there are enough of them (a chunk at a time with min_gap,
+      // whose gaps are kept per state of a chunk), then tested with a lane per
+      // (entry, state)
+      unsigned free_m = take;  // lanes of this pass without a contact yet
+      int n_ent = 0, b = 0;
+      while (near_any) {
+        const int c = __ffs(near_any) - 1;
+        for (; b < n_slot && n_ent <= kListCap - 32 * PARTS; b += 32) {
+          unsigned near = b + lane < n_slot ? S.near_[b + lane] >> c : 0u;
+          const unsigned e = near ? S.slot[b + lane] : 0u;
+          if (!((free_m >> (e & 31u)) & 1u)) near = 0u;
+#pragma unroll
+          for (int q = 0; q < PARTS; q++) {
+            const bool in = (near >> (8 * q)) & 1u;
             const unsigned m = __ballot_sync(kFull, in);
-            if (in) S.list[n_ent + __popc(m & lt)] = (uint16_t)e;
+            if (in) S.list[n_ent + __popc(m & lt)] = (uint32_t)c << 16 | (uint32_t)q << 14 | e;
             n_ent += __popc(m);
           }
-          __syncwarp();
-          if (n_ent) {
-            Pose<float> ps[PARTS];  // this lane's state of the chunk
-#pragma unroll
-            for (int q = 0; q < PARTS; q++) ps[q] = pose[q * pv.S + min(k, L - 1)];
-            const float tk = float(k) * dt;
-            unsigned seen = 0u;  // contacts or FP64 decisions of the chunk
-            for (int i0 = 0; i0 < n_ent; i0 += NE) {
-              const bool in = i0 + sub < n_ent;
-              const unsigned e = in ? S.list[i0 + sub] : 0u;
-              const int own = (int)(e & 31u), o = (int)(e >> 5);
-              const int own_nst = __shfl_sync(kFull, nst, own);
-              bool hit = false, amb = false;
-              if (in && j < own_nst) {
-                const Ob ob = ((const Ob *)obs_sm)[o];
-                float sx = S.off[0][own], sy = S.off[1][own], sz = D == 3 ? S.off[D - 1][own] : 0.f;
-                if constexpr (V > 0) {
-                  sx += tk * S.off[D][own];
-                  sy += tk * S.off[D + 1][own];
-                  if constexpr (D == 3) sz += tk * S.off[D + 2][own];
-                }
-                float gmin = INFINITY;
-#pragma unroll
-                for (int q = 0; q < PARTS; q++) {
-                  int r;
-                  if constexpr (R::SPHERE) {
-                    r = sphere_test<float, true>(ps[q].cx + sx, ps[q].cy + sy, ps[q].c + sz, ob, A.radius32, A.band32,
-                                                 gmin);
-                  } else {
-                    const float ac = fabsf(ps[q].c), as = fabsf(ps[q].s), hl = A.half_len32, hw = A.half_wid32;
-                    r = planar_test<float, true>(ps[q].cx + sx, ps[q].cy + sy, ps[q].c, ps[q].s, dot2(hl, ac, hw, as),
-                                                 dot2(hl, as, hw, ac), ob, hl, hw, A.band32, gmin);
-                  }
-                  if (r == 2) {  // decide in FP64
-                    r = contact64<KIND>(A, p, k, q, S.node[own], o) ? 1 : 0;
-                    amb = true;
-                  }
-                  hit |= r == 1;
-                }
-                // gaps above the cap are reported as +inf: only smaller ones are merged
-                if (want_mg && gmin <= kGapCap) atomicMin(&mgs[32 * j + own], ord_gap(gmin));
-              }
-              const unsigned hb = __ballot_sync(kFull, hit), ab = __ballot_sync(kFull, amb);
-              if (hb | ab) {
-                seen |= hb | ab;
-                if (j == 0) {  // the entry's first lane merges its states' bits
-                  const unsigned h = (hb >> (sub * CH)) & kChunkBits, a = (ab >> (sub * CH)) & kChunkBits;
-                  if (h) atomicOr(&S.hit[own], h);
-                  if (a) atomicOr(&S.rc[own], a);
-                }
-              }
+        }
+        const bool whole = b >= n_slot;  // all of the chunk is listed
+        if (whole) {
+          b = 0;
+          near_any &= near_any - 1;
+          if (near_any && !want_mg && n_ent < kListMin) continue;
+        }
+        __syncwarp();
+        for (int i0 = 0; i0 < n_ent; i0 += NE) {
+          const bool in = i0 + sub < n_ent;
+          const unsigned e = in ? S.list[i0 + sub] : 0u;
+          const int own = (int)(e & 31u), ob_i = (int)(e >> 5 & (kSlotCap - 1u));
+          const int k = (c0 + (int)(e >> 16)) * CH + j;
+          bool hit = false, amb = false;
+          if (in && k < S.oob[own] && k <= S.contact[own]) {
+            const int q = PARTS > 1 ? (int)(e >> 14 & 1u) : 0;
+            const Pose<float> ps = pose[(PARTS > 1 ? q * pv.S : 0) + k];
+            const Ob ob = ((const Ob *)obs_sm)[ob_i];
+            float sx = S.off[0][own], sy = S.off[1][own], sz = D == 3 ? S.off[D - 1][own] : 0.f;
+            if constexpr (V > 0) {
+              const float tk = float(k) * dt;
+              sx += tk * S.off[D][own];
+              sy += tk * S.off[D + 1][own];
+              if constexpr (D == 3) sz += tk * S.off[D + 2][own];
             }
-            if (seen || want_mg) {
-              __syncwarp();
-              const unsigned h = S.hit[lane], a = S.rc[lane];
-              const int last = h ? __ffs(h) - 1 : CH - 1;
-              if (a & ((2u << last) - 1u)) rechecked = true;
-              if (want_mg) {
-                unsigned mg = mgs[32 * CH + lane];
-                for (int i = 0; i < CH; i++) {
-                  if (i <= last) mg = min(mg, mgs[32 * i + lane]);
-                  mgs[32 * i + lane] = 0xffffffffu;
-                }
-                mgs[32 * CH + lane] = mg;
-              }
-              if (h) {
-                collided = true;
-                fi = k0 + last;
-                if (!need_bounds) live = false;
-              }
-              S.hit[lane] = 0u;
-              S.rc[lane] = 0u;
+            float gmin = INFINITY;
+            int r;
+            if constexpr (R::SPHERE) {
+              r = sphere_test<float, true>(ps.cx + sx, ps.cy + sy, ps.c + sz, ob, A.radius32, A.band32, gmin);
+            } else {
+              const float ac = fabsf(ps.c), as = fabsf(ps.s), hl = A.half_len32, hw = A.half_wid32;
+              r = planar_test<float, true>(ps.cx + sx, ps.cy + sy, ps.c, ps.s, dot2(hl, ac, hw, as),
+                                           dot2(hl, as, hw, ac), ob, hl, hw, A.band32, gmin);
             }
+            if (r == 2) {  // decide in FP64
+              r = contact64<KIND>(A, p, k, q, S.node[own], ob_i, ps.cx + sx, ps.cy + sy, ps.c, ps.s) ? 1 : 0;
+              amb = true;
+            }
+            hit = r == 1;
+            // gaps above the cap are reported as +inf: only smaller ones are merged
+            if (want_mg && gmin <= kGapCap) atomicMin(&mgs[32 * j + own], ord_gap(gmin));
           }
-          __syncwarp();  // the next chunk rewrites the list
+          const unsigned hb = __ballot_sync(kFull, hit);
+          if (hit && first_of_group<CH>(hb, lane)) atomicMin(&S.contact[own], k);
+          if (amb) atomicMin(&S.contact_amb[own], k);
         }
-        if (live && j_oob < CH) {  // later states of this lane are never tested
-          oob = true;
-          fi = k0 + j_oob;
-          live = false;
+        n_ent = 0;
+        __syncwarp();
+        // (a contact found amid a chunk may not be the chunk's first)
+        if (!whole) continue;
+        if (S.contact[lane] != kNever) collided = true;
+        if (want_mg) {
+          const int k0 = (c0 + c) * CH, last = S.contact[lane];
+          unsigned mg = mgs[32 * CH + lane];
+          for (int i = 0; i < CH; i++) {
+            if (k0 + i <= last) mg = min(mg, mgs[32 * i + lane]);
+            mgs[32 * i + lane] = 0xffffffffu;
+          }
+          mgs[32 * CH + lane] = mg;
+          __syncwarp();
         }
+        free_m &= __ballot_sync(kFull, !collided);
+        if (!free_m) break;
       }
       __syncwarp();  // the next pass rewrites the slots
     }
+    if ((collided && !need_bounds) || S.oob[lane] != L) live = false;
   }
 
+  // what was tested after a lane's first contact or first state out of bounds does not count
+  const int first_oob = S.oob[lane], first_contact = S.contact[lane];
+  const bool oob = first_oob < L;
+  const int fi = oob ? first_oob : (collided ? first_contact : L);
+  const bool rechecked = (S.oob_amb[lane] != kNever && S.oob_amb[lane] <= first_oob) ||
+                         (S.contact_amb[lane] != kNever && S.contact_amb[lane] <= first_contact);
   const unsigned rmask = __ballot_sync(kFull, active && rechecked);
   if (lane == 0 && rmask) atomicAdd(&A.ctr->n_recheck, (unsigned long long)__popc(rmask));
   const uint32_t row_out = active && o.out_index ? o.out_index[pair0 + lane] : pair0 + lane;

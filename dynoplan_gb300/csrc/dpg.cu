@@ -351,7 +351,7 @@ void dpg_destroy(dpg_ctx *c) {
                     &c->st32, &c->act64, &c->pose32, &c->pose64, &c->pbox, &c->pbox32, &c->obs32, &c->obs64,
                     &c->x64, &c->nkey32, &c->noff32, &c->mask, &c->cnt, &c->tot, &c->pbase,
                     &c->ord_pbase, &c->ord_ibase, &c->item_pos, &c->p_node, &c->p_prim, &c->p_verdict, &c->p_fi,
-                    &c->p_end, &c->p_gap, &c->p_flags, &c->coff, &c->cbox32, &c->tbox32,
+                    &c->p_end, &c->p_gap, &c->p_flags, &c->coff, &c->cbox32, &c->qbox32, &c->tbox32,
                     &c->q_node, &c->q_prim, &c->q_sorted, &c->q_idx, &c->q_fill,
                     &c->ord_cell, &c->ord_perm, &c->ord_cnt, &c->ord_start, &c->ord_rank, &c->ord_tiles, &c->x64s,
                     &c->kg_start, &c->kg_tab, &c->lz_off, &c->lz_cnt, &c->lz_cur, &c->lz_next, &c->lz_valid,
@@ -494,6 +494,7 @@ static int load_tables(dpg_ctx *c, int32_t P, const int32_t *len, const double *
       (rc = ensure(c, c->pbox32, sizeof(float) * 2 * pd * P)) ||
       (rc = ensure(c, c->coff, sizeof(int64_t) * P)) ||
       (rc = ensure(c, c->cbox32, sizeof(float) * 2 * pd * NC)) ||
+      (rc = ensure(c, c->qbox32, parts > 1 ? sizeof(float) * 2 * pd * parts * NC : 0)) ||
       (rc = ensure(c, c->tbox32, sizeof(float) * 2 * pd * P)) ||
       (rc = ensure(c, c->rkey32, sizeof(float) * kd * P)) || (rc = ensure(c, c->rkconst32, sizeof(float) * P)) ||
       (rc = ensure(c, c->rkrow, sizeof(int64_t) * P)))
@@ -528,7 +529,9 @@ static int load_tables(dpg_ctx *c, int32_t P, const int32_t *len, const double *
                                                        P_<float>(c->rkconst32), nullptr, nullptr, true);
     build_chunks<KIND><<<(P + 127) / 128, 128, 0, st>>>(rp, P, P_<int32_t>(c->len), P_<int64_t>(c->soff),
                                                          P_<int64_t>(c->coff), P_<Pose<double>>(c->pose64), S,
-                                                         P_<float>(c->cbox32), P_<float>(c->tbox32));
+                                                         P_<float>(c->cbox32),
+                                                         parts > 1 ? P_<float>(c->qbox32) : P_<float>(c->cbox32),
+                                                         P_<float>(c->tbox32));
   });
   CUDA_TRY(c, cudaGetLastError());
   CUDA_TRY(c, cudaStreamSynchronize(st));
@@ -849,6 +852,7 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
   pv.pbox32 = P_<float>(c->pbox32);
   pv.coff = P_<int64_t>(c->coff);
   pv.cbox32 = P_<float>(c->cbox32);
+  pv.qbox32 = c->robot.n_parts > 1 ? P_<float>(c->qbox32) : pv.cbox32;
   pv.tbox32 = P_<float>(c->tbox32);
   if (reverse) {  // the ball keys on each primitive's last state (the key grid holds start keys)
     pv.key32 = P_<float>(c->rkey32);
@@ -1199,6 +1203,7 @@ int dpg_expand_noalloc(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const
   pv.pbox32 = P_<float>(c->pbox32);
   pv.coff = P_<int64_t>(c->coff);
   pv.cbox32 = P_<float>(c->cbox32);
+  pv.qbox32 = c->robot.n_parts > 1 ? P_<float>(c->qbox32) : pv.cbox32;
   pv.tbox32 = P_<float>(c->tbox32);
   NodeView nv{N, x_dev, nkey32, noff32};
   EnvView ev{};
@@ -1326,6 +1331,7 @@ PrimView ctx_prim_view(dpg_ctx *c) {
   pv.pbox32 = P_<float>(c->pbox32);
   pv.coff = P_<int64_t>(c->coff);
   pv.cbox32 = P_<float>(c->cbox32);
+  pv.qbox32 = c->robot.n_parts > 1 ? P_<float>(c->qbox32) : pv.cbox32;
   pv.tbox32 = P_<float>(c->tbox32);
   return pv;
 }

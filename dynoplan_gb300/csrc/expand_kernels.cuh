@@ -77,6 +77,7 @@ struct PrimView {
   const int64_t *coff;       // [P] first chunk row of primitive p
   const float *cbox32;       // [sum chunks][2*POSD]: centre..., half... of the parts'
                              //   bounding box over Robot::CHUNK states (outward rounded)
+  const float *qbox32;       // [sum chunks][PARTS][2*POSD]: the same, a box per part
   const float *tbox32;       // [P][2*POSD]: the same over the whole primitive
 };
 
@@ -680,14 +681,25 @@ __global__ void build_keys(RobotParams rp, int P, const int32_t *len, const int6
   }
 }
 
+// box of D centres and D half extents: the centre to nearest, the half extent
+// up by the centre's rounding error and to the next float
+template <int D>
+__device__ void store_box(const double *lo, const double *hi, float *box) {
+  for (int i = 0; i < D; i++) {
+    const double cen = 0.5 * (lo[i] + hi[i]), half = 0.5 * (hi[i] - lo[i]);
+    const float c32 = (float)cen;
+    box[i] = c32;
+    box[D + i] = __double2float_ru(half + fabs(cen - (double)c32));
+  }
+}
+
 // Culling boxes: per chunk of Robot::CHUNK states, the bounding box of every
-// collision part over those canonical states; per primitive, the union.
-// FP64, then rounded outward to FP32 (centre to nearest, half extent up by
-// the centre's rounding error).
+// collision part over those canonical states, part by part and together; per
+// primitive, the union.  FP64, then rounded outward to FP32.
 template <int KIND>
 __global__ void build_chunks(RobotParams rp, int P, const int32_t *len, const int64_t *soff,
                              const int64_t *coff, const Pose<double> *pose64, int64_t S,
-                             float *cbox32, float *tbox32) {
+                             float *cbox32, float *qbox32, float *tbox32) {
   using R = Robot<KIND>;
   constexpr int D = R::POSD;
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -696,40 +708,36 @@ __global__ void build_chunks(RobotParams rp, int P, const int32_t *len, const in
   const int L = len[p];
   for (int c = 0; c * R::CHUNK < L; c++) {
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-    for (int k = c * R::CHUNK; k < min(L, (c + 1) * R::CHUNK); k++) {
-      for (int q = 0; q < R::PARTS; q++) {
+    for (int q = 0; q < R::PARTS; q++) {
+      double qlo[3] = {1e300, 1e300, 1e300}, qhi[3] = {-1e300, -1e300, -1e300};
+      for (int k = c * R::CHUNK; k < min(L, (c + 1) * R::CHUNK); k++) {
         const Pose<double> ps = pose64[q * S + soff[p] + k];
         if constexpr (R::SPHERE) {
           const double v[3] = {ps.cx, ps.cy, ps.c};
           for (int i = 0; i < 3; i++) {
-            lo[i] = fmin(lo[i], v[i] - rp.radius);
-            hi[i] = fmax(hi[i], v[i] + rp.radius);
+            qlo[i] = fmin(qlo[i], v[i] - rp.radius);
+            qhi[i] = fmax(qhi[i], v[i] + rp.radius);
           }
         } else {
           const double ac = fabs(ps.c), as = fabs(ps.s);
           const double ex = rp.half_len * ac + rp.half_wid * as, ey = rp.half_len * as + rp.half_wid * ac;
-          lo[0] = fmin(lo[0], ps.cx - ex); hi[0] = fmax(hi[0], ps.cx + ex);
-          lo[1] = fmin(lo[1], ps.cy - ey); hi[1] = fmax(hi[1], ps.cy + ey);
+          qlo[0] = fmin(qlo[0], ps.cx - ex); qhi[0] = fmax(qhi[0], ps.cx + ex);
+          qlo[1] = fmin(qlo[1], ps.cy - ey); qhi[1] = fmax(qhi[1], ps.cy + ey);
         }
       }
+      store_box<D>(qlo, qhi, qbox32 + ((coff[p] + c) * R::PARTS + q) * 2 * D);
+      for (int i = 0; i < D; i++) {
+        lo[i] = fmin(lo[i], qlo[i]);
+        hi[i] = fmax(hi[i], qhi[i]);
+      }
     }
-    float *cb = cbox32 + (coff[p] + c) * 2 * D;
+    store_box<D>(lo, hi, cbox32 + (coff[p] + c) * 2 * D);
     for (int i = 0; i < D; i++) {
-      const double cen = 0.5 * (lo[i] + hi[i]), half = 0.5 * (hi[i] - lo[i]);
-      const float c32 = (float)cen;
-      cb[i] = c32;
-      cb[D + i] = __double2float_ru(half + fabs(cen - (double)c32));
       tlo[i] = fmin(tlo[i], lo[i]);
       thi[i] = fmax(thi[i], hi[i]);
     }
   }
-  float *tb = tbox32 + (int64_t)p * 2 * D;
-  for (int i = 0; i < D; i++) {
-    const double cen = 0.5 * (tlo[i] + thi[i]), half = 0.5 * (thi[i] - tlo[i]);
-    const float c32 = (float)cen;
-    tb[i] = c32;
-    tb[D + i] = __double2float_ru(half + fabs(cen - (double)c32));
-  }
+  store_box<D>(tlo, thi, tbox32 + (int64_t)p * 2 * D);
 }
 
 }  // namespace dpg
