@@ -1293,13 +1293,20 @@ extern "C" int dpg_mlp_node_features(dpg_ctx *c, const double *x_dev, int64_t N,
   ev.n_obs = c->n_obs;
   ev.obs32 = c->obs32.p;
   ev.obs64 = c->obs64.p;
+  FeatureScale fs{};
+  for (int i = 0; i < c->dim; i++) {
+    const double ext = c->hi[i] - c->lo[i];
+    fs.lo[i] = c->lo[i];
+    fs.ok[i] = ext > 0 ? 1 : 0;
+    fs.scale[i] = 2.0 / ext;
+  }
   GoalView gv{};
   gv.has = goal ? 1 : 0;
   for (int i = 0; i < 3 && goal; i++) gv.g[i] = i < c->dim ? goal[i] : 0.0;
   with_kind(c->robot.kind, [&](auto K) {
     constexpr int KIND = decltype(K)::value;
-    mlp_node_features<KIND><<<(unsigned)((N + 127) / 128), 128, 0, c->stream>>>(
-        nv, ev, gv, static_cast<__nv_bfloat16 *>(feat_dev));
+    mlp_node_features<KIND><<<(unsigned)((N + kFeatNodes - 1) / kFeatNodes), 8 * kFeatNodes, 0, c->stream>>>(
+        nv, ev, fs, gv, static_cast<__nv_bfloat16 *>(feat_dev));
   });
   CUDA_TRY(c, cudaGetLastError());
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));

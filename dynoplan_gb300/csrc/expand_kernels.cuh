@@ -112,8 +112,11 @@ struct PairView {
 };
 
 __device__ __forceinline__ float wrap_pi_f64(double a) {
-  double w = fmod(a + kPi, kTwoPi);
-  if (w < 0) w += kTwoPi;
+  double w = a + kPi;
+  if (!(w >= 0 && w < kTwoPi)) {  // (fmod(w, 2 pi) = w inside)
+    w = fmod(w, kTwoPi);
+    if (w < 0) w += kTwoPi;
+  }
   return (float)(w - kPi);
 }
 
