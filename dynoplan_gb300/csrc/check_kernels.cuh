@@ -1081,9 +1081,9 @@ __device__ void load_obstacles(const EnvView &ev, void *sm) {
 // the link serves about 150 M such reads a second whatever the SMs do, so a
 // read per item bounded the whole check (car1, 100,000 nodes x 5,000 motions,
 // 260,000 items: 1.73 ms for fetching the items alone, 0.18 ms without the
-// reads).  The warps that draw every kAbortPoll-th item of a launch read it
-// (the first item always, then one read in a few hundred nanoseconds of a full
-// GPU), and on an abort move the launch's item counter past its end.
+// reads).  The launch's first warp reads it, then the warps that draw every
+// kAbortPoll-th item (one read in a few hundred nanoseconds of a full GPU); on
+// an abort they move the launch's item counter past its end.
 constexpr unsigned long long kAbortPoll = 64;
 constexpr unsigned long long kNoMoreItems = 1ull << 62;
 
@@ -1117,20 +1117,26 @@ __device__ __forceinline__ void for_items(const CheckArgs &A, Item item_fn) {
     }
     cur_cnt = 0;
   };
-  // the next item is drawn while the current one is checked
-  uint32_t next = 0;
+  // A warp's first item is its number in the launch (consecutive items on
+  // different blocks), the others are drawn from the counter, the next one
+  // while the current one is checked.
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5), w_id = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  uint32_t next = w_id < n_items - i_lo ? i_lo + w_id : n_items;
+  auto poll_abort = [&]() {
+    if (*A.abort_flag) {
+      A.ctr->status = DPG_ERR_ABORTED;  // every warp's next item lies past the end
+      atomicMax(&A.ctr->next_sub[A.sub], kNoMoreItems);
+      next = n_items;
+    }
+  };
   auto draw = [&]() {
     if (lane == 0) {
       const unsigned long long drawn = atomicAdd(&A.ctr->next_sub[A.sub], 1ull);
-      next = drawn < n_items - i_lo ? i_lo + (uint32_t)drawn : n_items;
-      if (next < n_items && drawn % kAbortPoll == 0 && *A.abort_flag) {
-        A.ctr->status = DPG_ERR_ABORTED;  // every warp's next item lies past the end
-        atomicMax(&A.ctr->next_sub[A.sub], kNoMoreItems);
-        next = n_items;
-      }
+      next = drawn + warps < n_items - i_lo ? i_lo + warps + (uint32_t)drawn : n_items;
+      if (next < n_items && drawn % kAbortPoll == 0) poll_abort();
     }
   };
-  draw();
+  if (lane == 0 && w_id == 0 && next < n_items) poll_abort();
   while (true) {
     const uint32_t item = __shfl_sync(kFull, next, 0);
     if (item >= n_items) break;

@@ -74,6 +74,14 @@ struct dpg_ctx {
   // size from which the ball scan uses the key grid, pipelined check launches
   dpg_tuning tune{DPG_CHECK_SLOTS, 0, 2048, 8, DPG_HOST_OUT_PROGRESS};
   cudaEvent_t ev[6] = {};
+  // stage times of the last call; timings_due: dpg_expand's events hold them
+  // (read when asked for)
   double timings[4] = {0, 0, 0, 0};
+  bool timings_due = false;
+  // resident blocks per SM of the check kernels, as launched before
+  struct Occupancy { const void *kernel; size_t smem; int blocks; };
+  std::vector<Occupancy> occupancy;
+  // small batches: inputs and results through mapped page-locked memory
+  void *h_small = nullptr, *d_small = nullptr;
 };
 

@@ -121,6 +121,20 @@ template <class F> void with_kind(int kind, F &&f) {
 
 }  // namespace
 
+// Resident blocks per SM of a check kernel with `smem` bytes, asked for once
+// per context, kernel and size (the two runtime calls cost microseconds a
+// launch); the kernel may then use all the shared memory a block can have.
+static int check_occupancy(dpg_ctx *c, const void *kernel, size_t smem) {
+  for (const auto &o : c->occupancy)
+    if (o.kernel == kernel && o.smem == smem) return o.blocks;
+  int optin = 0, blocks = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, kCheckThreads, smem);
+  c->occupancy.push_back({kernel, smem, blocks});
+  return blocks;
+}
+
 // The exact check of the pair list on `st`: lockstep warps over (primitive,
 // 32 nodes) items, with obstacle culling when the candidate masks cover
 // every obstacle.
@@ -140,9 +154,7 @@ static void launch_check(dpg_ctx *c, const CheckArgs &ca, int prec, cudaStream_t
   CheckArgs a = ca;
   auto go = [&](auto kern, size_t scratch = 0) {
     const size_t sm = sm_obs + scratch * (kCheckThreads / 32);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCheckThreads, sm);
+    int per_sm = check_occupancy(c, reinterpret_cast<const void *>(kern), sm);
     if (c->tune.check_blocks_per_sm > 0) per_sm = std::min(per_sm, c->tune.check_blocks_per_sm);
     kern<<<c->sm_count * std::max(per_sm, 1), kCheckThreads, sm, st>>>(a);
   };
@@ -193,7 +205,17 @@ static int nn_tiles_per_y(int P, int64_t B, int sm_count) {
 // (an expand whose results go to host buffers runs tune.pipe_launches <=
 // kMaxSub check launches, one work-queue counter each)
 
-constexpr size_t kMinCopyBytes = 16u << 20;  // smallest group of copy ranges copied together
+// smallest group of copy ranges copied together: a quarter of the results, so
+// that a search round's 10 MB leave while they are checked, within these (a
+// copy call costs host time, and below 2 MB more than it hides)
+constexpr size_t kMinCopyBytes = 2u << 20, kMaxCopyBytes = 16u << 20;
+// results (of N x P pairs) from which a batch under kReorderMin nodes is copied
+// in ranges too: quad2d x 10,000 with every output, copies after the check /
+// in ranges: 32 nodes (13 MB) 238 / 259 us, 64 nodes 388 / 382, 100 nodes
+// 538 / 502, 128 nodes 661 / 587
+constexpr size_t kRangeBytes = 32u << 20;
+// mapped buffer of a context: a small batch's nodes, then its results
+constexpr size_t kSmallX = sizeof(double) * 13 * kSmallNodes, kSmallBytes = 1u << 20;
 
 // Cumulative item weights of the copy ranges of a host-buffer expand: each
 // range `decay` times the one before, so a range's result copy overlaps the
@@ -329,6 +351,8 @@ int dpg_create(dpg_ctx **out, int device, const dpg_robot_desc *robot) {
     if (cudaHostAlloc(&c->h_ctr, 2 * sizeof(DevCounters), cudaHostAllocDefault) != cudaSuccess) { rc = DPG_ERR_OOM; break; }
     if (cudaHostAlloc(&c->h_abort, sizeof(int), cudaHostAllocMapped) != cudaSuccess) { rc = DPG_ERR_OOM; break; }
     *c->h_abort = 0;
+    if (cudaHostAlloc(&c->h_small, kSmallX + kSmallBytes, cudaHostAllocMapped) != cudaSuccess) { rc = DPG_ERR_OOM; break; }
+    if (cudaHostGetDevicePointer(&c->d_small, c->h_small, 0) != cudaSuccess) { rc = DPG_ERR_CUDA; break; }
     if (cudaHostGetDevicePointer(&c->d_abort, c->h_abort, 0) != cudaSuccess) { rc = DPG_ERR_CUDA; break; }
     for (auto &e : c->ev)
       if (cudaEventCreate(&e) != cudaSuccess) { rc = DPG_ERR_CUDA; break; }
@@ -361,6 +385,7 @@ void dpg_destroy(dpg_ctx *c) {
   if (c->h_ctr) cudaFreeHost(c->h_ctr);
   if (c->h_bases) cudaFreeHost(c->h_bases);
   if (c->h_lz) cudaFreeHost(c->h_lz);
+  if (c->h_small) cudaFreeHost(c->h_small);
   if (c->h_rflag) cudaFreeHost(c->h_rflag);
   for (auto &e : c->ev_sub)
     if (e) cudaEventDestroy(e);
@@ -638,6 +663,24 @@ int dpg_upload_env(dpg_ctx *c, int32_t dim, const double *lo, const double *hi, 
   return DPG_OK;
 }
 
+}  // extern "C"
+
+// stage times of the last dpg_expand from its events (all complete)
+static void read_timings(dpg_ctx *c) {
+  float a = 0, b = 0, t_in = 0, t_out = 0;
+  cudaEventElapsedTime(&a, c->ev[1], c->ev[2]);
+  cudaEventElapsedTime(&b, c->ev[2], c->ev[3]);
+  cudaEventElapsedTime(&t_in, c->ev[0], c->ev[1]);
+  cudaEventElapsedTime(&t_out, c->ev[3], c->ev[5]);
+  c->timings[0] = a;
+  c->timings[1] = b;
+  c->timings[2] = 0;
+  c->timings[3] = t_in + t_out;
+  c->timings_due = false;
+}
+
+extern "C" {
+
 int dpg_sync(dpg_ctx *c) {
   if (!c) return DPG_ERR_ARG;
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
@@ -662,6 +705,7 @@ void dpg_host_free(void *p) {
 
 int dpg_last_timings(const dpg_ctx *c, double *t, int32_t n) {
   if (!c || !t || n < 0) return DPG_ERR_ARG;
+  if (c->timings_due) read_timings(const_cast<dpg_ctx *>(c));
   const int k = std::min(n, 4);
   for (int i = 0; i < k; i++) t[i] = c->timings[i];
   return k;
@@ -792,10 +836,44 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
     }
   }
 
-  // host-buffer outputs of a checked batch in spatial order: the check runs as
-  // tune.pipe_launches launches over item ranges and each range's results are copied out
-  // while the next range is checked
-  const bool pipelined = !dev_out && !direct && !(opts->mode & DPG_MODE_BALL_ONLY) && reorder && cap > 0;
+  // Small batches (kSmallNodes nodes): two ball kernels.  Their host inputs
+  // are read by the GPU from mapped page-locked memory, and host results of at
+  // most kSmallBytes are written there by the check and copied on the host: a
+  // call is three launches and one wait (car1, one node: 68 us, 144 us with an
+  // input copy, seven launches, two waits and seven result copies).
+  const bool small = N > 0 && N <= kSmallNodes && P <= kSmallMaxP;
+  struct { void *dst; size_t row, at; } sm_out[7] = {
+      {out->node, 4, 0}, {out->prim, 4, 0}, {out->verdict, 1, 0}, {out->first_invalid, 2, 0},
+      {out->end_state, es_bytes * nx, 0}, {out->min_gap, 4, 0}, {out->flags, 1, 0}};
+  bool small_out = false;
+  if (small && !dev_out && !direct && !(opts->mode & DPG_MODE_BALL_ONLY) && out->node && out->prim) {
+    const size_t rows = (size_t)std::min<int64_t>(cap, N * P);
+    size_t at = kSmallX;
+    for (auto &f : sm_out) {
+      f.at = at;
+      if (f.dst) at += (f.row * rows + 255) / 256 * 256;
+    }
+    small_out = rows > 0 && at <= kSmallX + kSmallBytes;
+    if (small_out) {
+      unsigned char *d = static_cast<unsigned char *>(c->d_small);
+      pv_out.node_host = reinterpret_cast<uint32_t *>(d + sm_out[0].at);
+      pv_out.prim_host = reinterpret_cast<uint32_t *>(d + sm_out[1].at);
+      if (out->verdict) pv_out.verdict = d + sm_out[2].at;
+      if (out->first_invalid) pv_out.first_invalid = reinterpret_cast<int16_t *>(d + sm_out[3].at);
+      if (out->end_state) pv_out.end_state = d + sm_out[4].at;
+      if (out->min_gap) pv_out.min_gap = reinterpret_cast<float *>(d + sm_out[5].at);
+      if (out->flags) pv_out.flags = d + sm_out[6].at;
+    }
+  }
+
+  // host-buffer outputs of a checked batch in spatial order, or of a smaller
+  // one that may have kRangeBytes of results: checked in tune.pipe_launches
+  // item ranges, each range's results copied out while the next is checked
+  size_t row_bytes = 0;
+  for (const auto &f : sm_out)
+    if (f.dst) row_bytes += f.row;
+  const bool pipelined = !dev_out && !direct && !small_out && !(opts->mode & DPG_MODE_BALL_ONLY) && cap > 0 &&
+                         (reorder || (size_t)std::min<int64_t>(cap, N * P) * row_bytes >= kRangeBytes);
   // one check launch whose warps flag finished copy ranges in mapped memory
   const bool progress = pipelined && c->tune.host_output == DPG_HOST_OUT_PROGRESS;
   const int n_ranges = pipelined ? c->tune.pipe_launches : 1;
@@ -826,13 +904,12 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
   }
 
   CUDA_TRY(c, cudaEventRecord(c->ev[0], st));
-  if (N > 0) {
-    if (opts->x_on_device)
-      CUDA_TRY(c, cudaMemcpyAsync(c->x64.p, x, sizeof(double) * nx * N, cudaMemcpyDeviceToDevice, st));
-    else
-      CUDA_TRY(c, cudaMemcpyAsync(c->x64.p, x, sizeof(double) * nx * N, cudaMemcpyHostToDevice, st));
-  }
-  CUDA_TRY(c, cudaMemsetAsync(c->d_ctr, 0, sizeof(DevCounters), st));
+  if (small && !opts->x_on_device)
+    std::memcpy(c->h_small, x, sizeof(double) * nx * N);
+  else if (N > 0 && !opts->x_on_device)
+    CUDA_TRY(c, cudaMemcpyAsync(c->x64.p, x, sizeof(double) * nx * N, cudaMemcpyHostToDevice, st));
+  const double *x_dev = opts->x_on_device ? x : P_<double>(c->x64);  // the nodes, in the caller's order
+  if (!small) CUDA_TRY(c, cudaMemsetAsync(c->d_ctr, 0, sizeof(DevCounters), st));
   CUDA_TRY(c, cudaEventRecord(c->ev[1], st));
 
   PrimView pv{};
@@ -859,7 +936,7 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
     pv.kconst32 = P_<float>(c->rkconst32);
     pv.krow = P_<int64_t>(c->rkrow);
   }
-  NodeView nv{N, P_<double>(c->x64), P_<float>(c->nkey32), P_<float>(c->noff32)};
+  NodeView nv{N, x_dev, P_<float>(c->nkey32), P_<float>(c->noff32)};
   EnvView ev{};
   ev.dim = c->dim;
   for (int i = 0; i < 3; i++) { ev.lo[i] = c->lo[i]; ev.hi[i] = c->hi[i]; }
@@ -898,7 +975,7 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
     if (reorder) {  // nodes by Z-order cell, then index; the pipeline runs on the sorted copy
       const unsigned nb = (unsigned)((N + 255) / 256);
       const int64_t tile = order_tile(N), ntile = (N + tile - 1) / tile;
-      node_tiles<KIND><<<(unsigned)ntile, 256, 0, st>>>(P_<double>(c->x64), N, ev, tile, P_<uint32_t>(c->ord_cell),
+      node_tiles<KIND><<<(unsigned)ntile, 256, 0, st>>>(x_dev, N, ev, tile, P_<uint32_t>(c->ord_cell),
                                                          P_<uint32_t>(c->ord_rank), P_<uint32_t>(c->ord_tiles));
       nn_prefix<<<kOrderCells / 32, 256, 0, st>>>(kOrderCells, (int)ntile, P_<uint32_t>(c->ord_tiles),
                                                   P_<uint32_t>(c->ord_cnt));
@@ -907,9 +984,23 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
                                        P_<uint32_t>(c->ord_tiles), P_<uint32_t>(c->ord_start),
                                        P_<uint32_t>(c->ord_perm));
       gather_nodes<R::NX><<<(unsigned)((N * R::NX + 255) / 256), 256, 0, st>>>(
-          P_<double>(c->x64), P_<uint32_t>(c->ord_perm), N, P_<double>(c->x64s));
+          x_dev, P_<uint32_t>(c->ord_perm), N, P_<double>(c->x64s));
       nv.x64 = P_<double>(c->x64s);
       ca.nv = nv;
+    }
+    if (small) {
+      const float4 w32 = make_float4((float)rp.w[0], (float)rp.w[1], (float)rp.w[2], (float)rp.w[3]);
+      const bool staged = !opts->x_on_device;
+      small_ball<KIND><<<(unsigned)((P + 127) / 128), 128, 0, st>>>(
+          rp, pv, nv, staged ? static_cast<const double *>(c->d_small) : x_dev,
+          staged ? P_<double>(c->x64) : nullptr, w32, (float)opts->radius, opts->radius, (float)ball_band,
+          P_<uint32_t>(c->mask), P_<uint32_t>(c->cnt));
+      small_emit<<<(unsigned)((P + 255) / 256), 256, 0, st>>>(
+          P, (int)W, P_<int32_t>(c->order), P_<uint32_t>(c->mask), P_<uint32_t>(c->cnt), cap, pv_out.node, pv_out.prim,
+          P_<unsigned long long>(c->ord_pbase), P_<unsigned long long>(c->ord_ibase), P_<uint32_t>(c->item_pos), ctr);
+      cudaEventRecord(c->ev[2], st);
+      launch_err = cudaGetLastError();
+      return;
     }
     if (N > 0) {
       prep_nodes<KIND><<<(unsigned)((N + 255) / 256), 256, 0, st>>>(nv);
@@ -972,7 +1063,6 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
                                                                     pv_out.node);
     }
     cudaEventRecord(c->ev[3], st);
-    cudaEventRecord(c->ev[4], st);
     launch_err = cudaGetLastError();
   });
   if (launch_err != cudaSuccess)
@@ -996,12 +1086,10 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
       const int np = n_ranges;
       int cum[kMaxSub + 1];
       pipe_weights(np, cum, decay);
-      size_t bpp = 0;  // bytes copied per pair
-      for (const auto &f : cp)
-        if (f.dst) bpp += f.b;
-      // consecutive ranges are copied together until a group holds
-      // kMinCopyBytes (each copy call costs host time; small batches get
-      // fewer, larger copies); the last range closes the last group
+      // consecutive ranges are copied together until a group holds min_copy
+      // bytes; the last range closes the last group
+      const size_t bpp = row_bytes;  // bytes copied per pair
+      const size_t min_copy = std::clamp((size_t)h0.n_pairs * bpp / 4, kMinCopyBytes, kMaxCopyBytes);
       int64_t ga = -1;
       for (int j = 0; j < np; j++) {
         const int64_t a = pair_at(h0.n_items * cum[j] / cum[np]), e = pair_at(h0.n_items * cum[j + 1] / cum[np]);
@@ -1016,7 +1104,7 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
         }
         if (ga < 0) ga = a;
         const bool last = j == np - 1;
-        if (!last && (size_t)(e - ga) * bpp < kMinCopyBytes) continue;
+        if (!last && (size_t)(e - ga) * bpp < min_copy) continue;
         if (last) CUDA_TRY(c, cudaEventRecord(c->ev_cl[0], c->cstream));
         if (e > ga)
           for (const auto &f : cp)
@@ -1029,10 +1117,11 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
         ga = -1;
       }
     }
-    CUDA_TRY(c, cudaStreamWaitEvent(c->cstream, c->ev[4], 0));
+    CUDA_TRY(c, cudaStreamWaitEvent(c->cstream, c->ev[3], 0));
     CUDA_TRY(c, cudaEventRecord(c->ev[5], c->cstream));
   }
   CUDA_TRY(c, cudaMemcpyAsync(c->h_ctr + 1, ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, st));
+  if (!pipelined) CUDA_TRY(c, cudaEventRecord(c->ev[5], st));
   CUDA_TRY(c, cudaStreamSynchronize(st));
   if (pipelined) CUDA_TRY(c, cudaStreamSynchronize(c->cstream));
   const DevCounters h = c->h_ctr[1];
@@ -1045,6 +1134,9 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
   const int64_t np = (int64_t)h.n_pairs;
   if (pipelined) {
     // copied above
+  } else if (small_out) {
+    for (const auto &f : sm_out)
+      if (f.dst) std::memcpy(f.dst, static_cast<char *>(c->h_small) + f.at, f.row * (size_t)np);
   } else if (!dev_out && !direct && np > 0) {
     struct { void *dst; void *src; size_t b; } cp[] = {
         {out->node, c->p_node.p, 4}, {out->prim, c->p_prim.p, 4}, {out->verdict, c->p_verdict.p, 1},
@@ -1054,29 +1146,18 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
     for (int i = 0; i < n_copy; i++)
       if (cp[i].dst) CUDA_TRY(c, cudaMemcpyAsync(cp[i].dst, cp[i].src, cp[i].b * np, cudaMemcpyDeviceToHost, st));
   }
-  if (!pipelined) {
+  if (!pipelined && !small_out && !dev_out) {
     CUDA_TRY(c, cudaEventRecord(c->ev[5], st));
     CUDA_TRY(c, cudaStreamSynchronize(st));
   }
-  float ms = 0;
-  cudaEventElapsedTime(&ms, c->ev[1], c->ev[2]); c->timings[0] = ms;
-  cudaEventElapsedTime(&ms, c->ev[2], c->ev[3]); c->timings[1] = ms;
-  cudaEventElapsedTime(&ms, c->ev[3], c->ev[4]); c->timings[2] = ms;
-  float t_in = 0, t_out = 0;
-  cudaEventElapsedTime(&t_in, c->ev[0], c->ev[1]);
-  cudaEventElapsedTime(&t_out, c->ev[4], c->ev[5]);
-  c->timings[3] = t_in + t_out;
+  c->timings_due = true;
+  if (pipelined) read_timings(c);
   if (pipelined && last_bytes >= (1u << 20) && np > 0 && c->timings[1] > 0) {
     // the next call's range decay: this call's copy time (at the rate of its
     // last range, whose copies run after the check) over its check time
     float cl = 0;
     if (cudaEventElapsedTime(&cl, c->ev_cl[0], c->ev_cl[1]) == cudaSuccess && cl > 0) {
-      size_t bpp = 0;  // bytes copied per pair
-      const size_t b1[7] = {4, 4, 1, 2, (size_t)es_bytes * nx, 4, 1};
-      void *d1[7] = {out->node, out->prim, out->verdict, out->first_invalid, out->end_state, out->min_gap, out->flags};
-      for (int i = 0; i < 7; i++)
-        if (d1[i]) bpp += b1[i];
-      const double copy_ms = (double)bpp * (double)np * (double)cl / (double)last_bytes;
+      const double copy_ms = (double)row_bytes * (double)np * (double)cl / (double)last_bytes;
       c->pipe_decay = std::min(1.0, std::max(0.75, copy_ms / (double)c->timings[1]));
     }
   }
@@ -1574,6 +1655,7 @@ extern "C" int dpg_check_pairs(dpg_ctx *c, const dpg_expand_opts *opts, int64_t 
                                     " pairs have node >= N or prim >= P (left unchecked)");
   if (h.status == DPG_ERR_ABORTED) return fail(c, DPG_ERR_ABORTED, "check_pairs: aborted");
   float ms = 0;
+  c->timings_due = false;
   cudaEventElapsedTime(&ms, c->ev[1], c->ev[2]);
   c->timings[0] = ms;
   cudaEventElapsedTime(&ms, c->ev[2], c->ev[3]);

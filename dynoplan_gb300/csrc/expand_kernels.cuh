@@ -599,6 +599,182 @@ static __global__ void __launch_bounds__(256) nn_emit(int P, int64_t W, int64_t 
   }
 }
 
+// ------------------------------------------------------- small batches ---
+// Up to kSmallNodes nodes (a popped node, a round of the search): every step
+// above has a few microseconds of work at most, so their launches and
+// dependent table reads were the whole time.  Two kernels replace the seven:
+//   small_ball   thread per primitive (in length order): keys of the nodes in
+//                shared memory, the membership words of its primitive, their
+//                count and the FP64 decisions; block 0 also writes the nodes'
+//                states and offsets for the check
+//   small_emit   a block per 256 positions adds up the counts before it (all
+//                of them: P is a few thousand words in L2), then writes the
+//                bases, the item table, the counters and the pair lists
+// Same membership tests, order and counts as nn_mask ... nn_emit.  Ball stage,
+// car1, one node against 5,000 primitives: 15 us, quad2d, 32 against 10,000: 31 us
+// (nn_mask form: 66 and 86 us).  The line of 128 nodes: a thread walks the nodes
+// one by one, so its time grows with them (128 nodes: car1 42 us, quadrotor 53,
+// against 66 and 89), while nn_mask's does not up to about two blocks an SM.
+constexpr int kSmallNodes = 128;
+constexpr int kSmallMaxP = 32768;  // small_emit's blocks each read every count
+
+template <int KIND>
+__global__ void __launch_bounds__(128) small_ball(RobotParams rp, PrimView pv, NodeView nv, const double *x_in,
+                                                  double *x_out, float4 w32, float radius, double radius64, float band,
+                                                  uint32_t *mask, uint32_t *cnt) {
+  using R = Robot<KIND>;
+  __shared__ float nk[R::KEYD][kSmallNodes];
+  const int N = (int)nv.N, W = (N + 31) / 32;
+  for (int n = threadIdx.x; n < N; n += blockDim.x) {
+    const double *x = x_in + (int64_t)n * R::NX;
+#pragma unroll
+    for (int i = 0; i < R::KEYD; i++) {
+      const int c = R::key_comp(i);
+      const bool angle = (KIND != DPG_ROBOT_QUAD3D) && c == 2 || (KIND == DPG_ROBOT_CAR1 && c == 3);
+      nk[i][n] = angle ? wrap_pi_f64(x[c]) : (float)x[c];
+    }
+    if (blockIdx.x == 0) {
+#pragma unroll
+      for (int i = 0; i < R::POSD; i++) nv.off32[i * nv.N + n] = (float)x[i];
+#pragma unroll
+      for (int i = 0; i < R::VELOFF; i++) nv.off32[(R::POSD + i) * nv.N + n] = (float)x[R::vel_comp(i)];
+      if (x_out)
+#pragma unroll
+        for (int i = 0; i < R::NX; i++) x_out[(int64_t)n * R::NX + i] = x[i];
+    }
+  }
+  __syncthreads();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= pv.P) return;
+  const int p = pv.order[i];
+  float sk[R::KEYD];
+#pragma unroll
+  for (int k = 0; k < R::KEYD; k++) sk[k] = pv.key32[(int64_t)k * pv.P + p];
+  const float kc = pv.kconst32[p];
+  uint32_t members = 0, rechecks = 0;
+  for (int w = 0; w < W; w++) {
+    uint32_t word = 0;
+    const int nn = min(32, N - 32 * w);
+    for (int b = 0; b < nn; b++) {
+      float q[R::KEYD];
+#pragma unroll
+      for (int k = 0; k < R::KEYD; k++) q[k] = nk[k][32 * w + b];
+      const float d = key_dist32<KIND>(w32, q, sk, 1, kc);
+      bool in = d <= radius;
+      if (fabsf(d - radius) <= band) {  // decide in FP64
+        in = key_dist64<KIND>(rp, x_in + (int64_t)(32 * w + b) * R::NX, pv.st64 + pv.krow[p] * R::NX) <= radius64;
+        rechecks++;
+      }
+      if (in) word |= 1u << b;
+    }
+    mask[(int64_t)i * W + w] = word;
+    members += __popc(word);
+  }
+  cnt[i] = members | rechecks << 16;
+}
+
+static __global__ void __launch_bounds__(256) small_emit(int P, int W, const int32_t *order, const uint32_t *mask,
+                                                         const uint32_t *cnt, int64_t cap, uint32_t *pair_node,
+                                                         uint32_t *pair_prim, unsigned long long *ord_pbase,
+                                                         unsigned long long *ord_ibase, uint32_t *item_pos,
+                                                         DevCounters *ctr) {
+  __shared__ uint32_t part[8][5];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // sums over the positions before this warp's and over all of them
+  const int w0 = blockIdx.x * 256 + 32 * warp;  // the warp's first position
+  uint32_t before = 0, before_i = 0, all = 0, all_i = 0, rechecks = 0;
+  for (int i = threadIdx.x; i < P; i += 256) {
+    const uint32_t c = cnt[i], n = c & 0xffffu, items = (n + 31) / 32;
+    all += n;
+    all_i += items;
+    rechecks += c >> 16;
+    if (i < (int)blockIdx.x * 256) {
+      before += n;
+      before_i += items;
+    }
+  }
+  before = __reduce_add_sync(kFull, before);
+  before_i = __reduce_add_sync(kFull, before_i);
+  all = __reduce_add_sync(kFull, all);
+  all_i = __reduce_add_sync(kFull, all_i);
+  rechecks = __reduce_add_sync(kFull, rechecks);
+  if (lane == 0) {
+    part[warp][0] = before;
+    part[warp][1] = before_i;
+    part[warp][2] = all;
+    part[warp][3] = all_i;
+    part[warp][4] = rechecks;
+  }
+  __syncthreads();
+  before = before_i = all = all_i = rechecks = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    before += part[k][0];
+    before_i += part[k][1];
+    all += part[k][2];
+    all_i += part[k][3];
+    rechecks += part[k][4];
+  }
+  __syncthreads();
+  const bool overflow = (int64_t)all > cap;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    DevCounters c{};
+    c.n_pairs = all;
+    c.n_items = overflow ? 0 : all_i;
+    c.n_overflow = overflow ? 1 : 0;
+    c.n_ball_recheck = rechecks;
+    *ctr = c;
+    ord_pbase[P] = all;
+    ord_ibase[P] = all_i;
+  }
+  // this position's bases: prefix within the block
+  const int i = w0 + lane;
+  const uint32_t n = i < P ? cnt[i] & 0xffffu : 0u, items = (n + 31) / 32;
+  uint32_t pn = n, pi = items;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t a = __shfl_up_sync(kFull, pn, d), b = __shfl_up_sync(kFull, pi, d);
+    if (lane >= d) {
+      pn += a;
+      pi += b;
+    }
+  }
+  if (lane == 31) {
+    part[warp][0] = pn;
+    part[warp][1] = pi;
+  }
+  __syncthreads();
+  for (int k = 0; k < warp; k++) {
+    before += part[k][0];
+    before_i += part[k][1];
+  }
+  const uint32_t base = before + pn - n, ibase = before_i + pi - items;
+  if (i < P) {
+    ord_pbase[i] = base;
+    ord_ibase[i] = ibase;
+  }
+  // the warp writes its positions' pairs and items, a word of nodes at a time
+  const int p = i < P ? order[i] : 0;
+  const uint32_t first = i < P ? mask[(int64_t)i * W] : 0u;
+  for (unsigned m = __ballot_sync(kFull, n > 0); m; m &= m - 1) {
+    const int k = __ffs(m) - 1;
+    uint32_t at = __shfl_sync(kFull, base, k);
+    const uint32_t ik = __shfl_sync(kFull, ibase, k), mk = __shfl_sync(kFull, items, k);
+    const uint32_t pk = __shfl_sync(kFull, (uint32_t)p, k);
+    const uint32_t word0 = __shfl_sync(kFull, first, k);
+    for (int w = 0; w < W; w++) {
+      const uint32_t word = w == 0 ? word0 : mask[(int64_t)(w0 + k) * W + w];
+      const uint32_t pos = at + __popc(word & ((1u << lane) - 1u));
+      if (((word >> lane) & 1u) && (int64_t)pos < cap) {
+        pair_node[pos] = (uint32_t)(32 * w + lane);
+        pair_prim[pos] = pk;
+      }
+      at += __popc(word);
+    }
+    if (!overflow && lane < (int)mk) item_pos[ik + lane] = (uint32_t)(w0 + k);
+  }
+}
+
 // --------------------------------------------------- upload-time tables ---
 
 // Canonical FP64 rollout of every primitive from its stored start with its
