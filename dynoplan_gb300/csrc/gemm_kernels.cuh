@@ -387,12 +387,15 @@ struct EpiBiasGelu {
     if (actT) store_transposed16(actT, ldt, row, c0, h);
   }
 };
-// out = acc + bias (FP32), first n_valid columns
+// out = acc + bias (FP32), first n_valid columns of the first `rows` rows (the
+// GEMM's row count is padded to its tile; out holds no more than these)
 struct EpiBias {
   const float *bias;
   float *out;
   int ld, n_valid;
+  int64_t rows;
   __device__ void operator()(int row, int c0, const float *v) const {
+    if (row >= rows) return;
 #pragma unroll
     for (int j = 0; j < 16; j++)
       if (c0 + j < n_valid) out[(int64_t)row * ld + c0 + j] = v[j] + bias[c0 + j];

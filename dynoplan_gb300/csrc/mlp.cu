@@ -286,7 +286,7 @@ cudaError_t forward_rows(dpg_mlp *M, int64_t B, bool train, float *out, cudaStre
     if (e != cudaSuccess) return e;
     in = M->H[l];
   }
-  return launch_gemm(kMlpOutPad, M->H[2], M->W16[3], (int)Bp, kMlpHidden, 1, EpiBias{M->w[DPG_MLP_B4], out, 2, 2},
+  return launch_gemm(kMlpOutPad, M->H[2], M->W16[3], (int)Bp, kMlpHidden, 1, EpiBias{M->w[DPG_MLP_B4], out, 2, 2, B},
                      M->err, st);
 }
 
