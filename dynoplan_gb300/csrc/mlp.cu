@@ -31,17 +31,19 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// tensor map of a row-major bf16 matrix [rows x k] read in boxes of
-// 64 columns (one 128-byte swizzle row) x box_rows rows
-bool make_kmajor_map(CUtensorMap *m, const void *ptr, uint64_t rows, uint64_t k, uint32_t box_rows) {
+// tensor map of a row-major bf16 matrix [rows x k] read in boxes of box_k
+// columns (64: one 128-byte swizzle row, 32: one 64-byte swizzle row) x box_rows
+// rows
+bool make_kmajor_map(CUtensorMap *m, const void *ptr, uint64_t rows, uint64_t k, uint32_t box_rows,
+                     uint32_t box_k = kGemmKChunk) {
   const EncodeTiledFn fn = encode_tiled();
   if (!fn || (reinterpret_cast<uintptr_t>(ptr) & 15) || k % kGemmKChunk) return false;
   const cuuint64_t dims[2] = {k, rows};
   const cuuint64_t strides[1] = {k * sizeof(__nv_bfloat16)};
-  const cuuint32_t box[2] = {(cuuint32_t)kGemmKChunk, box_rows};
+  const cuuint32_t box[2] = {box_k, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, box_k == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -211,7 +213,7 @@ struct dpg_mlp {
   float *out = nullptr, *loss = nullptr;
   int *err = nullptr;
   int step = 0;
-  int fused = 2;  // forward kernel: 2 mlp_forward_fused2, 1 mlp_forward_fused, 0 layer GEMMs
+  int fused = 2;  // forward kernel: 2 mlp_forward_pair, 1 mlp_forward_fused, 0 layer GEMMs
   int sm_count = 0;
   // training-step inputs copied to fixed buffers, hyper-parameters in device
   // memory [lr, ctg_weight, 1 - b1^t, 1 - b2^t]: the step is captured once
@@ -223,6 +225,11 @@ struct dpg_mlp {
   const void *graph_feat = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   double last_ms = 0, last_flops = 0;
+  bool ms_due = false;  // e0 and e1 hold the last call's time (read when asked for)
+  // weight maps of the forward kernels, [0]: chunks of 64 columns, [1]: of kFwdK
+  CUtensorMap tw[2][4];
+  bool maps = false;
+  int *h_err = nullptr, *d_err = nullptr;  // the forward's error word, mapped page-locked memory
 };
 
 namespace {
@@ -343,9 +350,21 @@ int dpg_mlp_create(dpg_mlp **out, int device, int n_prims, int64_t max_rows, uin
   ok = ok && dalloc(&M->in_node, R) == cudaSuccess && dalloc(&M->in_prim, R) == cudaSuccess &&
        dalloc(&M->in_target, 2 * R) == cudaSuccess && dalloc(&M->hp, 4) == cudaSuccess &&
        cudaHostAlloc(&M->hp_host, 4 * sizeof(float), cudaHostAllocDefault) == cudaSuccess;
+  ok = ok && cudaHostAlloc(&M->h_err, sizeof(int), cudaHostAllocMapped) == cudaSuccess &&
+       cudaHostGetDevicePointer(&M->d_err, M->h_err, 0) == cudaSuccess;
   if (!ok) {
     dpg_mlp_destroy(M);
     return DPG_ERR_OOM;
+  }
+  // (without the driver's tensor maps the forward runs the layer GEMMs)
+  M->maps = cudaFuncSetAttribute(mlp_forward_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem) == cudaSuccess &&
+            cudaFuncSetAttribute(mlp_forward_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmem) == cudaSuccess;
+  for (int v = 0; v < 2; v++) {
+    const uint32_t bk = v ? kFwdK : kGemmKChunk;  // columns of a weight chunk
+    M->maps = M->maps && make_kmajor_map(&M->tw[v][0], M->W16[0], kMlpHidden, kMlpIn, kMlpHidden, bk) &&
+              make_kmajor_map(&M->tw[v][1], M->W16[1], kMlpHidden, kMlpHidden, kMlpHidden, bk) &&
+              make_kmajor_map(&M->tw[v][2], M->W16[2], kMlpHidden, kMlpHidden, kMlpHidden, bk) &&
+              make_kmajor_map(&M->tw[v][3], M->W16[3], kMlpOutPad, kMlpHidden, kMlpOutPad);
   }
   cudaStream_t st = M->stream;
   cudaMemsetAsync(M->err, 0, sizeof(int), st);
@@ -397,6 +416,7 @@ void dpg_mlp_destroy(dpg_mlp *M) {
                   M->out,   M->loss, M->err, M->in_node, M->in_prim, M->in_target, M->hp};
   for (void *b : bufs) cudaFree(b);
   if (M->hp_host) cudaFreeHost(M->hp_host);
+  if (M->h_err) cudaFreeHost(M->h_err);
   if (M->graph) cudaGraphExecDestroy(M->graph);
   if (M->e0) cudaEventDestroy(M->e0);
   if (M->e1) cudaEventDestroy(M->e1);
@@ -433,30 +453,21 @@ int dpg_mlp_forward(dpg_mlp *M, const void *node_feat_dev, const uint32_t *node_
   cudaSetDevice(M->device);
   cudaStream_t st = M->stream;
   const auto *nf = static_cast<const __nv_bfloat16 *>(node_feat_dev);
-  cudaMemsetAsync(M->err, 0, sizeof(int), st);
+  *(volatile int *)M->h_err = 0;
+  const bool fused = M->fused && n > 0 && M->maps;
+  if (!fused) cudaMemsetAsync(M->err, 0, sizeof(int), st);
   cudaEventRecord(M->e0, st);
   double flops = 0;
-  CUtensorMap tw[4];
-  const bool fused = M->fused && n > 0 && make_kmajor_map(&tw[0], M->W16[0], kMlpHidden, kMlpIn, kMlpHidden) &&
-                     make_kmajor_map(&tw[1], M->W16[1], kMlpHidden, kMlpHidden, kMlpHidden) &&
-                     make_kmajor_map(&tw[2], M->W16[2], kMlpHidden, kMlpHidden, kMlpHidden) &&
-                     make_kmajor_map(&tw[3], M->W16[3], kMlpOutPad, kMlpHidden, kMlpOutPad);
   if (fused) {  // one persistent kernel, one CTA per SM
     FusedArgs fa{nf, M->emb16, node_dev, prim_dev, M->w[DPG_MLP_B1], M->w[DPG_MLP_B2], M->w[DPG_MLP_B3],
-                 M->w[DPG_MLP_B4], out_dev, n, M->err};
+                 M->w[DPG_MLP_B4], out_dev, n, M->d_err};
     const int64_t tiles = (n + 127) / 128;
     const unsigned grid = (unsigned)std::min<int64_t>(tiles, std::max(M->sm_count, 1));
-    if (M->fused == 2) {  // warp-specialised: epilogues overlap the next layer's MMAs
-      if (cudaFuncSetAttribute(mlp_forward_fused2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFused2Smem) !=
-          cudaSuccess)
-        return DPG_ERR_CUDA;
-      mlp_forward_fused2<<<grid, kFused2Threads, kFused2Smem, st>>>(tw[0], tw[1], tw[2], tw[3], fa);
-    } else {
-      if (cudaFuncSetAttribute(mlp_forward_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmem) !=
-          cudaSuccess)
-        return DPG_ERR_CUDA;
+    const CUtensorMap *tw = M->tw[M->fused == 2];
+    if (M->fused == 2)  // warp-specialised: epilogues overlap the other tile's MMAs
+      mlp_forward_pair<<<grid, kFwdThreads, kFwdSmem, st>>>(tw[0], tw[1], tw[2], M->W16[3], fa);
+    else
       mlp_forward_fused<<<grid, kFusedThreads, kFusedSmem, st>>>(tw[0], tw[1], tw[2], tw[3], fa);
-    }
     if (cudaGetLastError() != cudaSuccess) return DPG_ERR_CUDA;
     flops = forward_flops(pad128(n));
   }
@@ -470,10 +481,9 @@ int dpg_mlp_forward(dpg_mlp *M, const void *node_feat_dev, const uint32_t *node_
   }
   cudaEventRecord(M->e1, st);
   if (cudaStreamSynchronize(st) != cudaSuccess) return DPG_ERR_CUDA;
-  float ms = 0;
-  cudaEventElapsedTime(&ms, M->e0, M->e1);
-  M->last_ms = ms;
+  M->ms_due = true;
   M->last_flops = flops;
+  if (fused) return *(volatile int *)M->h_err ? DPG_ERR_TIMEOUT : DPG_OK;
   return check_err(M);
 }
 
@@ -597,9 +607,7 @@ int dpg_mlp_train_step(dpg_mlp *M, const void *node_feat_dev, const uint32_t *no
   cudaMemcpyAsync(&hl, M->loss, sizeof(float), cudaMemcpyDeviceToHost, st);
   if (cudaStreamSynchronize(st) != cudaSuccess) return DPG_ERR_CUDA;
   if (loss) *loss = hl / (float)B;
-  float ms = 0;
-  cudaEventElapsedTime(&ms, M->e0, M->e1);
-  M->last_ms = ms;
+  M->ms_due = true;
   // forward + the two backward GEMMs per layer
   M->last_flops = 3.0 * forward_flops(pad128(B));
   return check_err(M);
@@ -614,6 +622,13 @@ int dpg_mlp_set_fused(dpg_mlp *M, int fused) {
 
 int dpg_mlp_last_timing(const dpg_mlp *M, double *ms, double *flops) {
   if (!M) return DPG_ERR_ARG;
+  if (M->ms_due) {
+    dpg_mlp *m = const_cast<dpg_mlp *>(M);
+    float t = 0;
+    cudaEventElapsedTime(&t, m->e0, m->e1);
+    m->last_ms = t;
+    m->ms_due = false;
+  }
   if (ms) *ms = M->last_ms;
   if (flops) *flops = M->last_flops;
   return DPG_OK;

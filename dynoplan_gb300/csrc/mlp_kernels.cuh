@@ -553,70 +553,139 @@ static __global__ void __launch_bounds__(kFusedThreads, 1)
 
 
 // ---------------------------------------------------------------------------
-// The same forward, warp-specialised so that the input gather and each
-// layer's epilogue overlap the MMAs.  Warps 0-15 run the epilogues, warp 16
-// (one lane) streams W1..W3 by TMA through a 3-stage ring of 64-column
-// K-chunks (10 chunks a tile, each stage freed as its MMAs complete), warp
-// 17 (one lane) issues the MMAs, warps 18-25 gather the next tile's input
-// rows into their own buffer while the current tile is computed.  The
-// epilogue of layer l writes H_l one 64-column k-block at a time, every warp
-// taking 16 columns of its lane quarter, and each finished k-block releases
-// the MMAs of layer l+1 over it (mbarrier hready[j], 512 arrivals); layers
-// alternate between two TMEM accumulators of 256 columns (512 allocated),
-// so layer l+1 accumulates while layer l's accumulator is still being read.
-// H_l is written over H_{l-1} in place: layer l's MMAs are complete before
-// its epilogue writes (accfull), and layer l+1 reads only k-blocks already
-// written.  The input buffer is refilled once the tile's layer-0 MMAs are
-// complete (xfree).  Every wait is bounded: on expiry the kernel sets *err,
-// waits (bounded) for its copies and MMAs in flight, frees TMEM and returns.
-constexpr int kFused2Threads = 832;  // 16 epilogue warps + TMA warp + MMA warp + 8 gather warps
-constexpr int kF2EpiThreads = 512;
-constexpr int kF2GatherThreads = 256;
-constexpr int kF2Stages = 3;
-constexpr uint32_t kXBytes = 128 * kMlpIn * 2;  // 32 KB: the input rows of a tile
-constexpr size_t kFused2Smem = 1024 + kXBytes + kActBytes + kF2Stages * kWChunk + kW4Bytes + 256;
+// The same forward, warp-specialised, with two tiles in flight per CTA: while
+// the epilogue warps turn one tile's accumulator into its next activations,
+// the tensor cores run the other tile's layer.  Each of the two tile slots has
+// 64 KB of shared memory (128 rows x 256 bf16, SW128 K-major) for the input
+// rows and the activations, each written over the last, and 256 columns of
+// TMEM.  Warps 0-15 run the epilogues, warp 16 (one lane) streams W1..W3 by TMA
+// through a ring of 32-column K-chunks, warp 17 issues the MMAs, warps 18-21
+// gather input rows, a thread a row, and write the outputs.  Order of the work,
+// for the MMAs and the epilogues alike: layer 1 of slots 0 and 1, layer 2 of
+// both, layer 3 of both, then the next two tiles.
+//
+// Layer l + 1 of a slot starts once the epilogue has read layer l's accumulator
+// and written its activations (hready), layer 1 of the next tile once layer 3's
+// accumulator was read (accfree) and the slot refilled (xready), which starts
+// once the layer-3 MMAs have read the activations (xfree).  H3 stays in
+// registers: the two outputs are dot products with the two rows of W4, summed
+// over the four column groups by the gather warps before they refill the slot.
+// Biases and W4 are in shared memory (read through L1, a layer's epilogue took
+// 5,800 clocks instead of 3,350): with chunks of 32 columns (64-byte swizzle)
+// the ring needs 80 KB, which leaves the room, and N = 256 keeps the input
+// operand's reads at one a k-step.
+// The epilogue's FP32 arithmetic is packed two columns an instruction
+// (fma.rn.f32x2); with 16 tanh a clock an SM it needs 2,048 clocks a layer
+// (measured 2,600 to 3,000 with its hand-over), the MMAs 2,048 (768 for layer
+// 1, whose columns past 96 are zero and left out; measured 3,000 to 4,000 while
+// both slots' weights stream from L2, which bounds the kernel now).
+// 1,048,576 pairs: 0.38 ms, 0.45 of the measured bf16 peak (one tile in
+// flight, two accumulators alternating by layer: 0.596 ms, 0.29); 65,536 pairs
+// 36 us (53), one tile 17 us (19).  Measured beside it: eight epilogue warps a
+// slot 5 % slower; chunks of 128 rows x 64 columns (N = 128) 20 % slower.
+// Every wait is bounded: on expiry the kernel sets *err, waits (bounded) for its
+// copies and MMAs in flight, frees TMEM and returns.
+constexpr int kFwdThreads = 704;  // 16 epilogue warps + TMA warp + MMA warp + 4 gather warps
+constexpr int kFwdEpiWarps = 16;
+constexpr int kFwdGatherThreads = 128;
+constexpr int kFwdStages = 5;
+constexpr int kFwdK = 32;                              // columns of a weight chunk
+constexpr uint32_t kFwdChunk = kMlpHidden * kFwdK * 2;  // 256 rows x 32 bf16 = 16 KB
+// biases of layers 1-3, W4's two rows (FP32), partial outputs [slot][column group][row]
+constexpr uint32_t kFwdConst = (3 + 2) * kMlpHidden * 4, kFwdPart = 2 * 4 * 128 * 8;
+constexpr size_t kFwdSmem = 1024 + 2 * kActBytes + kFwdStages * kFwdChunk + kFwdConst + kFwdPart + 256;
 
-static __global__ void __launch_bounds__(kFused2Threads, 1)
-    mlp_forward_fused2(const __grid_constant__ CUtensorMap tw1, const __grid_constant__ CUtensorMap tw2,
-                       const __grid_constant__ CUtensorMap tw3, const __grid_constant__ CUtensorMap tw4, FusedArgs a) {
+// two FP32 values in one 64-bit register
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// gelu (gemm_kernels.cuh) of two values, with its roundings
+__device__ __forceinline__ uint64_t gelu2(uint64_t z) {
+  const uint64_t one = pack2(1.f, 1.f);
+  const uint64_t f = fma2(mul2(pack2(kGeluB, kGeluB), z), z, one);
+  float u0, u1;
+  unpack2(mul2(mul2(pack2(kGeluA, kGeluA), z), f), u0, u1);
+  return mul2(mul2(pack2(0.5f, 0.5f), z), add2(one, pack2(tanh_fast(u0), tanh_fast(u1))));
+}
+// two values rounded to bf16 (the first in the low half)
+__device__ __forceinline__ uint32_t to_bf16x2(uint64_t v) {
+  float x, y;
+  unpack2(v, x, y);
+  const __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
+  return *reinterpret_cast<const uint32_t *>(&p);
+}
+__device__ __forceinline__ uint64_t from_bf16x2(uint32_t w) {
+  return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+
+static __global__ void __launch_bounds__(kFwdThreads, 1)
+    mlp_forward_pair(const __grid_constant__ CUtensorMap tw1, const __grid_constant__ CUtensorMap tw2,
+                     const __grid_constant__ CUtensorMap tw3, const __nv_bfloat16 *__restrict__ w4, FusedArgs a) {
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = umma::smem_u32(smem_raw);
-  unsigned char *xin = smem_raw + ((1024 - (raw & 1023)) & 1023);
-  unsigned char *act = xin + kXBytes;
-  unsigned char *wst = act + kActBytes;             // kF2Stages weight stages
-  unsigned char *w4 = wst + kF2Stages * kWChunk;    // resident W4, 4 k-blocks of 16 rows
-  uint64_t *wfull = reinterpret_cast<uint64_t *>(w4 + kW4Bytes);  // [kF2Stages]
-  uint64_t *wempty = wfull + kF2Stages;                           // [kF2Stages]
-  uint64_t *hready = wempty + kF2Stages;                          // [4]
-  uint64_t *w4full = hready + 4;
-  uint64_t *xready = w4full + 1;
-  uint64_t *xfree = xready + 1;
-  uint64_t *accfull = xfree + 1;
-  uint64_t *drain = accfull + 1;
+  unsigned char *act = smem_raw + ((1024 - (raw & 1023)) & 1023);  // two slots
+  unsigned char *wst = act + 2 * kActBytes;                        // weight stages
+  float *sbias = reinterpret_cast<float *>(wst + kFwdStages * kFwdChunk);       // [3][256]
+  float *sw4 = sbias + 3 * kMlpHidden;                                          // [2][256]
+  float2 *spart = reinterpret_cast<float2 *>(sw4 + 2 * kMlpHidden);             // [slot][group][128]
+  uint64_t *wfull = reinterpret_cast<uint64_t *>(spart + 2 * 4 * 128);          // [stages]
+  uint64_t *wempty = wfull + kFwdStages;                                       // [stages]
+  uint64_t *hready = wempty + kFwdStages;                                      // [2]
+  uint64_t *xready = hready + 2;                                               // [2]
+  uint64_t *xfree = xready + 2;                                                // [2]
+  uint64_t *accfull = xfree + 2;                                               // [2]
+  uint64_t *accfree = accfull + 2;                                             // [2]
+  uint64_t *pready = accfree + 2;                                              // [2]
+  uint64_t *drain = pready + 2;
   uint32_t *tslot = reinterpret_cast<uint32_t *>(drain + 1);
-  __shared__ __align__(16) float sbias[3][kMlpHidden];
-  __shared__ int s_bad, s_consumed, s_w4_done;
+  volatile int *bad = reinterpret_cast<volatile int *>(tslot + 1), *consumed = bad + 1, *mma_done = bad + 2;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t n_tiles = (a.B + 127) / 128;
-  for (int i = tid; i < 3 * kMlpHidden; i += kFused2Threads)
-    sbias[i / kMlpHidden][i % kMlpHidden] = (i < kMlpHidden ? a.b1 : (i < 2 * kMlpHidden ? a.b2 : a.b3))[i % kMlpHidden];
+  // tile of slot s in iteration i
+  auto tile_at = [&](int i, int s) { return blockIdx.x + (int64_t)(2 * i + s) * gridDim.x; };
   constexpr uint32_t kIdesc = umma::idesc_bf16_f32(128, kMlpHidden);
-  constexpr uint32_t kIdesc4 = umma::idesc_bf16_f32(128, kMlpOutPad);
+  for (int i = tid; i < 5 * kMlpHidden; i += kFwdThreads) {
+    const int l = i / kMlpHidden, c = i % kMlpHidden;
+    sbias[i] = l < 3 ? (l == 0 ? a.b1 : l == 1 ? a.b2 : a.b3)[c] : __bfloat162float(w4[(l - 3) * kMlpHidden + c]);
+  }
   if (tid == 0) {
-    for (int s = 0; s < kF2Stages; s++) {
+    for (int s = 0; s < kFwdStages; s++) {
       umma::mbar_init(&wfull[s], 1);
       umma::mbar_init(&wempty[s], 1);
     }
-    for (int j = 0; j < 4; j++) umma::mbar_init(&hready[j], kF2EpiThreads);
-    umma::mbar_init(w4full, 1);
-    umma::mbar_init(xready, kF2GatherThreads);
-    umma::mbar_init(xfree, 1);
-    umma::mbar_init(accfull, 1);
+    for (int s = 0; s < 2; s++) {
+      umma::mbar_init(&hready[s], kFwdEpiWarps);
+      umma::mbar_init(&pready[s], kFwdEpiWarps);
+      umma::mbar_init(&xready[s], kFwdGatherThreads / 32);
+      umma::mbar_init(&xfree[s], 1);
+      umma::mbar_init(&accfull[s], 1);
+      umma::mbar_init(&accfree[s], kFwdEpiWarps);
+    }
     umma::mbar_init(drain, 1);
     umma::mbar_fence_init();
-    s_bad = 0;
-    s_consumed = 0;
-    s_w4_done = 0;
+    *bad = 0;
+    *consumed = 0;
+    *mma_done = 0;
   }
   if (warp == 0) {
     umma::tmem_alloc(tslot, 512);
@@ -626,169 +695,233 @@ static __global__ void __launch_bounds__(kFused2Threads, 1)
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tmem = *tslot;
-  volatile int *bad = &s_bad;
 
   if (warp == 16) {
-    // ---- TMA producer: W4 once, then W1 (2 chunks), W2, W3 (4 each) per tile
+    // ---- TMA producer: W1 (3 chunks: the used columns), W2, W3 (8 each), for each slot's tile
     if (lane == 0 && blockIdx.x < n_tiles) {
       const void *wmap[3] = {&tw1, &tw2, &tw3};
-      umma::mbar_arrive_expect_tx(w4full, kW4Bytes);
-      for (int j = 0; j < 4; j++) umma::tma_load_2d(w4 + j * (kMlpOutPad * 128), &tw4, 64 * j, 0, w4full);
       int cnt = 0;
       bool ok = true;
-      for (int64_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x)
+      for (int i = 0; tile_at(i, 0) < n_tiles && ok; i++)
         for (int l = 0; l < 3 && ok; l++)
-          for (int j = 0; j < (l == 0 ? kMlpIn : kMlpHidden) / 64; j++, cnt++) {
-            const int s = cnt % kF2Stages;
-            if ((cnt >= kF2Stages && !umma::mbar_wait(&wempty[s], ((cnt / kF2Stages) - 1) & 1)) || *bad) {
-              *bad = 1;
-              ok = false;
-              break;
+          for (int s = 0; s < 2 && ok; s++) {
+            if (tile_at(i, s) >= n_tiles) continue;
+            for (int j = 0; j < (l == 0 ? kMlpNodeFeat + kMlpEmb : kMlpHidden) / kFwdK; j++, cnt++) {
+              const int st = cnt % kFwdStages;
+              if ((cnt >= kFwdStages && !umma::mbar_wait(&wempty[st], ((cnt / kFwdStages) - 1) & 1)) || *bad) {
+                *bad = 1;
+                ok = false;
+                break;
+              }
+              umma::mbar_arrive_expect_tx(&wfull[st], kFwdChunk);
+              umma::tma_load_2d(wst + st * kFwdChunk, wmap[l], kFwdK * j, 0, &wfull[st]);
             }
-            umma::mbar_arrive_expect_tx(&wfull[s], kWChunk);
-            umma::tma_load_2d(wst + s * kWChunk, wmap[l], 64 * j, 0, &wfull[s]);
           }
       // Copies still in flight land before the block's memory goes: once the
-      // MMA thread has stopped (it publishes s_w4_done; waited for at most
+      // MMA thread has stopped (it publishes mma_done; waited for at most
       // ~2 s of SM clock, far beyond any batch), the loads it did not consume
       // are waited for, bounded.
       const long long t0 = clock64();
-      while (*(volatile int *)&s_w4_done == 0 && clock64() - t0 < 4000000000ll) {
+      while (*mma_done == 0 && clock64() - t0 < 4000000000ll) {
       }
-      if (*bad) {
-        const int cons = *(volatile int *)&s_consumed;
-        for (int i = cons; i < cnt; i++) umma::mbar_wait(&wfull[i % kF2Stages], (i / kF2Stages) & 1, 1u << 20);
-      }
-      if (*(volatile int *)&s_w4_done != 2) umma::mbar_wait(w4full, 0, 1u << 20);  // W4 never waited for
+      if (*bad)
+        for (int i = *consumed; i < cnt; i++) umma::mbar_wait(&wfull[i % kFwdStages], (i / kFwdStages) & 1, 1u << 20);
     }
   } else if (warp == 17) {
-    // ---- MMA issuer
-    if (lane == 0) {
-      int cnt = 0, it = 0;
-      bool w4_ready = false, ok = true, issued_any = false;
-      for (int64_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, it++) {
-        if (!umma::mbar_wait(xready, it & 1) || *bad) { ok = false; break; }
-        for (int l = 0; l < 4 && ok; l++) {
-          const uint32_t acc = tmem + 256u * (uint32_t)(l & 1);
-          const uint32_t a0 = umma::smem_u32(l == 0 ? xin : act);
-          const int chunks = l == 0 ? kMlpIn / 64 : kMlpHidden / 64;
-          if (l == 3 && !w4_ready) {
-            if (!umma::mbar_wait(w4full, 0)) { ok = false; break; }
-            w4_ready = true;
-          }
-          for (int j = 0; j < chunks; j++) {
-            if (l > 0 && !umma::mbar_wait(&hready[j], (it * 3 + l - 1) & 1)) { ok = false; break; }
-            if (l < 3) {
-              if (!umma::mbar_wait(&wfull[cnt % kF2Stages], (cnt / kF2Stages) & 1)) { ok = false; break; }
-              *(volatile int *)&s_consumed = cnt + 1;
-            }
-            if (*bad) { ok = false; break; }
-            umma::fence_after_sync();
-            const uint32_t ak = a0 + j * (128 * 128);
-            const uint32_t b0 = l < 3 ? umma::smem_u32(wst + (cnt % kF2Stages) * kWChunk)
-                                      : umma::smem_u32(w4 + j * (kMlpOutPad * 128));
+    // ---- MMA issuer: the whole warp walks the schedule, so that the
+    // descriptors are warp-uniform, and an elected lane issues (a wait and four
+    // MMAs: 360 clocks of issue this way, 510 from one lane's branch)
+    bool ok = true, issued_any = false;
+    uint32_t st = 0, parity = 0;  // the next weight stage, parity of its next completion
+    int cnt = 0;
+    const uint64_t a_desc = umma::sdesc_kmajor_sw128(umma::smem_u32(act));
+    const uint64_t b_desc = umma::sdesc_kmajor_sw64(umma::smem_u32(wst));
+    auto layer = [&](auto first, int s) -> bool {
+      constexpr bool kFirst = decltype(first)::value;
+      const uint64_t ad = a_desc + s * (kActBytes >> 4);
+      const uint32_t acc = tmem + 256u * (uint32_t)s;
 #pragma unroll
-            for (int kk = 0; kk < 4; kk++)
-              umma::mma_bf16(acc, umma::sdesc_kmajor_sw128(ak + kk * 32), umma::sdesc_kmajor_sw128(b0 + kk * 32),
-                             l < 3 ? kIdesc : kIdesc4, (j > 0 || kk > 0) ? 1u : 0u);
-            issued_any = true;
-            if (l < 3) {
-              umma::commit(&wempty[cnt % kF2Stages]);
-              cnt++;
-            }
-          }
-          if (!ok) break;
-          if (l == 0) umma::commit(xfree);  // the input buffer may be refilled once these MMAs are done
-          umma::commit(accfull);
+      for (int j = 0; j < (kFirst ? kMlpNodeFeat + kMlpEmb : kMlpHidden) / kFwdK; j++) {
+        if (!umma::mbar_wait_warp(&wfull[st], parity)) return false;
+        umma::fence_after_sync();
+        const uint64_t bd = b_desc + st * (kFwdChunk >> 4);
+        if (umma::elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < kFwdK / 16; kk++)  // the input's k-blocks of 64 columns hold two chunks
+            umma::mma_bf16(acc, ad + (j >> 1) * (128 * 128 >> 4) + 4 * (j & 1) + 2 * kk, bd + 2 * kk, kIdesc,
+                           (j > 0 || kk > 0) ? 1u : 0u);
+          umma::commit(&wempty[st]);
+        }
+        __syncwarp();
+        cnt++;
+        if (++st == kFwdStages) {
+          st = 0;
+          parity ^= 1u;
         }
       }
-      if (!ok) *bad = 1;
-      if (issued_any) {  // the MMAs issued are complete before the memory goes
-        umma::commit(drain);
-        umma::mbar_wait(drain, 0, 1u << 20);
-      }
-      *(volatile int *)&s_consumed = cnt;
+      return true;
+    };
+    for (int i = 0; tile_at(i, 0) < n_tiles && ok; i++)
+      for (int l = 0; l < 3 && ok; l++)
+        for (int s = 0; s < 2 && ok; s++) {
+          if (tile_at(i, s) >= n_tiles) continue;
+          if (__any_sync(0xffffffffu, *bad) ||
+              (l == 0 ? !umma::mbar_wait_warp(&xready[s], i & 1) || (i > 0 && !umma::mbar_wait_warp(&accfree[s], (i - 1) & 1))
+                      : !umma::mbar_wait_warp(&hready[s], (2 * i + l - 1) & 1))) {
+            ok = false;
+            break;
+          }
+          issued_any = true;
+          ok = l == 0 ? layer(std::true_type{}, s) : layer(std::false_type{}, s);
+          if (!ok) break;
+          if (umma::elect_one()) {
+            if (l == 2) umma::commit(&xfree[s]);  // the slot may be refilled once these MMAs are done
+            umma::commit(&accfull[s]);
+          }
+          __syncwarp();
+        }
+    if (!ok && lane == 0) *bad = 1;
+    if (issued_any) {  // the MMAs issued are complete before the memory goes
+      if (umma::elect_one()) umma::commit(drain);
+      __syncwarp();
+      umma::mbar_wait_warp(drain, 0, 1u << 20);
+    }
+    if (lane == 0) {
+      *consumed = cnt;
       __threadfence_block();
-      *(volatile int *)&s_w4_done = w4_ready ? 2 : 1;
+      *mma_done = 1;
     }
   } else if (warp >= 18) {
-    // ---- gather warps: the input rows of each tile into xin, once the
-    // previous tile's layer-0 MMAs have read it
-    const int gt = tid - 18 * 32;
-    int it = 0;
-    for (int64_t t = blockIdx.x; t < n_tiles && !*bad; t += gridDim.x, it++) {
-      if (it > 0 && !umma::mbar_wait(xfree, (it - 1) & 1)) { *bad = 1; break; }
-      // two threads a row: the row's indices once, then its eight 16-byte
-      // chunks (node features 0-9, embedding 10-11, zero 12-15) loaded
-      // together before any store
-      static_assert(kF2GatherThreads == 256 && kMlpIn == 128, "two gather threads per row, 8 chunks each");
-      const int r = gt >> 1, c0 = 8 * (gt & 1);
-      const int64_t b = t * 128 + r;
-      uint4 v[8];
+    // ---- gather warps, a thread a row: the outputs of the slot's last tile,
+    // then the input row of its next one (node features and embedding, 16-byte
+    // chunks 0-9 and 10-11, loaded before the waits)
+    static_assert(kFwdGatherThreads == 128 && kMlpNodeFeat == 80 && kMlpEmb == 16, "a gather thread a row, 12 chunks");
+    const int r = tid - 18 * 32;
+    const float b40 = __ldg(a.b4), b41 = __ldg(a.b4 + 1);
+    // (decisions to stop are the same for a whole warp)
+    for (int i = 0; tile_at(i - 1, 0) < n_tiles && !__any_sync(0xffffffffu, *bad); i++)  // (i = 0: always)
+      for (int s = 0; s < 2; s++) {
+        const bool more = tile_at(i, s) < n_tiles;
+        const int64_t b = tile_at(i, s) * 128 + r;
+        uint4 v[12];
 #pragma unroll
-      for (int k = 0; k < 8; k++) v[k] = make_uint4(0, 0, 0, 0);
-      if (b < a.B) {
-        const uint4 *nf = reinterpret_cast<const uint4 *>(a.node_feat + (int64_t)a.node[b] * kMlpNodeFeat);
-        const uint4 *em = reinterpret_cast<const uint4 *>(a.emb + (int64_t)a.prim[b] * kMlpEmb);
+        for (int k = 0; k < 12; k++) v[k] = make_uint4(0, 0, 0, 0);
+        if (more && b < a.B) {
+          const uint4 *nf = reinterpret_cast<const uint4 *>(a.node_feat + (int64_t)a.node[b] * kMlpNodeFeat);
+          const uint4 *em = reinterpret_cast<const uint4 *>(a.emb + (int64_t)a.prim[b] * kMlpEmb);
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-          const int c = c0 + k;
-          if (c < kMlpNodeFeat / 8) v[k] = nf[c];
-          else if (c < (kMlpNodeFeat + kMlpEmb) / 8) v[k] = em[c - kMlpNodeFeat / 8];
+          for (int k = 0; k < 12; k++) v[k] = k < 10 ? nf[k] : em[k - 10];
         }
-      }
+        if (i > 0 && tile_at(i - 1, s) < n_tiles) {
+          if (!__all_sync(0xffffffffu, umma::mbar_wait(&pready[s], (i - 1) & 1))) {
+            *bad = 1;
+            break;
+          }
+          float2 o = make_float2(b40, b41);
 #pragma unroll
-      for (int k = 0; k < 8; k++) *reinterpret_cast<uint4 *>(xin + umma::kmajor_offset(128, r, c0 + k)) = v[k];
-      umma::fence_proxy_async_smem();
-      umma::mbar_arrive(xready);
-    }
+          for (int g = 0; g < 4; g++) {
+            const float2 p = spart[512 * s + 128 * g + r];
+            o.x += p.x;
+            o.y += p.y;
+          }
+          const int64_t ob = tile_at(i - 1, s) * 128 + r;
+          if (ob < a.B) {
+            a.out[ob * 2] = o.x;
+            a.out[ob * 2 + 1] = o.y;
+          }
+        }
+        if (!more) continue;
+        // (pready follows accfull of layer 3, so the slot's MMAs are done: xfree is there too)
+        if (!__all_sync(0xffffffffu, i == 0 || umma::mbar_wait(&xfree[s], (i - 1) & 1))) {
+          *bad = 1;
+          break;
+        }
+#pragma unroll
+        for (int k = 0; k < 12; k++)
+          *reinterpret_cast<uint4 *>(act + s * kActBytes + umma::kmajor_offset(128, r, k)) = v[k];
+        umma::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) umma::mbar_arrive(&xready[s]);
+      }
   } else {
-    // ---- epilogue warps: per layer H_l by k-blocks, then the outputs
-    const int q = warp & 3, h = warp >> 2, row = 32 * q + lane;
-    const uint32_t lane_addr = tmem + ((uint32_t)(32 * q) << 16);
-    int it = 0;
-    for (int64_t t = blockIdx.x; t < n_tiles && !*bad; t += gridDim.x, it++) {
-      const int64_t m0 = t * 128;
-      bool ok = true;
-      for (int l = 0; l < 3 && ok; l++) {
-        if (!umma::mbar_wait(accfull, (it * 4 + l) & 1)) { *bad = 1; ok = false; break; }
-        umma::fence_after_sync();
-        const uint32_t acc = 256u * (uint32_t)(l & 1);
-        const float *bias = sbias[l];
-        for (int j = 0; j < 4; j++) {
-          const int c0 = 64 * j + 16 * h;
-          float v[16];
-          umma::tmem_ld16(lane_addr + acc + c0, v);
-          __align__(16) __nv_bfloat162 hb[8];
+    // ---- epilogue warps: H1, H2, then the partial outputs.  Warp w:
+    // accumulator lanes 32 (w % 4) .., columns 64 (w / 4) ..
+    const int q = warp & 3, cg = warp >> 2, row = 32 * q + lane;
+    bool ok = true;
+    for (int i = 0; tile_at(i, 0) < n_tiles && ok && !__any_sync(0xffffffffu, *bad); i++)
+      for (int l = 0; l < 3 && ok; l++)
+        for (int s = 0; s < 2; s++) {
+          if (tile_at(i, s) >= n_tiles) continue;
+          if (!__all_sync(0xffffffffu, umma::mbar_wait(&accfull[s], (3 * i + l) & 1))) {
+            ok = false;
+            break;
+          }
+          const uint32_t src = tmem + ((uint32_t)(32 * q) << 16) + 256u * (uint32_t)s + 64u * (uint32_t)cg;
+          unsigned char *slot = act + s * kActBytes;
+          umma::fence_after_sync();
+          const float4 *bias = reinterpret_cast<const float4 *>(sbias + kMlpHidden * l + 64 * cg);
+          uint64_t a0 = pack2(0.f, 0.f), a1 = a0;
+          uint32_t r[2][16];  // this block's values and the next one's, in flight
+          umma::tmem_ld16_async(src, r[0]);
 #pragma unroll
-          for (int k = 0; k < 8; k++)
-            hb[k] = __floats2bfloat162_rn(gelu(v[2 * k] + bias[c0 + 2 * k]), gelu(v[2 * k + 1] + bias[c0 + 2 * k + 1]));
-          *reinterpret_cast<uint4 *>(act + umma::kmajor_offset(128, row, c0 / 8)) = reinterpret_cast<const uint4 *>(hb)[0];
-          *reinterpret_cast<uint4 *>(act + umma::kmajor_offset(128, row, c0 / 8 + 1)) =
-              reinterpret_cast<const uint4 *>(hb)[1];
-          umma::fence_proxy_async_smem();
-          umma::fence_before_sync();
-          umma::mbar_arrive(&hready[j]);
+          for (int j = 0; j < 4; j++) {
+            const int c0 = 64 * cg + 16 * j;
+            float4 bv[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) bv[k] = bias[4 * j + k];
+            uint32_t *v = r[j & 1];
+            umma::tmem_wait16(v);
+            if (j < 3) umma::tmem_ld16_async(src + 16u * (j + 1), r[(j + 1) & 1]);
+            uint64_t g[8];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              auto f = [&](int e) { return __uint_as_float(v[4 * k + e]); };
+              g[2 * k] = gelu2(add2(pack2(f(0), f(1)), pack2(bv[k].x, bv[k].y)));
+              g[2 * k + 1] = gelu2(add2(pack2(f(2), f(3)), pack2(bv[k].z, bv[k].w)));
+            }
+            uint32_t hb[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) hb[k] = to_bf16x2(g[k]);
+            if (l < 2) {
+              *reinterpret_cast<uint4 *>(slot + umma::kmajor_offset(128, row, c0 / 8)) = make_uint4(hb[0], hb[1], hb[2], hb[3]);
+              *reinterpret_cast<uint4 *>(slot + umma::kmajor_offset(128, row, c0 / 8 + 1)) =
+                  make_uint4(hb[4], hb[5], hb[6], hb[7]);
+            } else {  // the two outputs: rows 0 and 1 of W4
+#pragma unroll
+              for (int k = 0; k < 4; k++) {
+                const float4 w0 = *reinterpret_cast<const float4 *>(sw4 + c0 + 4 * k);
+                const float4 w1 = *reinterpret_cast<const float4 *>(sw4 + kMlpHidden + c0 + 4 * k);
+                const uint64_t h0 = from_bf16x2(hb[2 * k]), h1 = from_bf16x2(hb[2 * k + 1]);
+                a0 = fma2(h0, pack2(w0.x, w0.y), a0);
+                a1 = fma2(h0, pack2(w1.x, w1.y), a1);
+                a0 = fma2(h1, pack2(w0.z, w0.w), a0);
+                a1 = fma2(h1, pack2(w1.z, w1.w), a1);
+              }
+            }
+          }
+          if (l < 2) {
+            umma::fence_proxy_async_smem();
+            umma::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) umma::mbar_arrive(&hready[s]);
+          } else {
+            float x0, y0, x1, y1;
+            unpack2(a0, x0, y0);
+            unpack2(a1, x1, y1);
+            spart[512 * s + 128 * cg + row] = make_float2(x0 + y0, x1 + y1);
+            umma::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+              umma::mbar_arrive(&accfree[s]);
+              umma::mbar_arrive(&pready[s]);
+            }
+          }
         }
-      }
-      if (!ok) break;
-      if (!umma::mbar_wait(accfull, (it * 4 + 3) & 1)) { *bad = 1; break; }
-      umma::fence_after_sync();
-      if (h == 0) {
-        float v[16];
-        umma::tmem_ld16(lane_addr + 256u, v);
-        const int64_t b = m0 + row;
-        if (b < a.B) {
-          a.out[b * 2] = v[0] + a.b4[0];
-          a.out[b * 2 + 1] = v[1] + a.b4[1];
-        }
-      }
-      umma::fence_before_sync();
-    }
+    if (!ok) *bad = 1;
   }
   umma::fence_before_sync();
   __syncthreads();
-  if (tid == 0 && s_bad) atomicExch(a.err, 1);
+  if (tid == 0 && *bad) atomicExch(a.err, 1);
   umma::fence_after_sync();
   if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }

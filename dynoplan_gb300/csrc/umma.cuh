@@ -72,6 +72,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity, uint32_t
   return false;
 }
 
+// The same by all 32 lanes of a warp, with one answer for the warp.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *b, uint32_t parity, uint32_t limit = 1u << 22) {
+  for (uint32_t i = 0; i < limit; i++)
+    if (__any_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
+  return false;
+}
+// one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\nselp.b32 %0, 1, 0, q;\n}" : "=r"(p));
+  return p != 0;
+}
+
 // ---- descriptors -----------------------------------------------------------
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups
 // 1024 bytes apart (stride byte offset), descriptor version 1.
@@ -82,6 +95,16 @@ __device__ __forceinline__ uint64_t sdesc_kmajor_sw128(uint32_t saddr) {
   d |= (uint64_t)(1024 >> 4) << 32;          // stride byte offset
   d |= (uint64_t)1 << 46;                    // version
   d |= (uint64_t)2 << 61;                    // 128-byte swizzle
+  return d;
+}
+// The same with the 64-byte swizzle: rows of 64 bytes, 8-row groups 512 bytes apart.
+__device__ __forceinline__ uint64_t sdesc_kmajor_sw64(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(512 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)4 << 61;  // 64-byte swizzle
   return d;
 }
 // Instruction descriptor of kind::f16: BF16 A and B (K-major), FP32 D, M x N.
@@ -123,6 +146,24 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// The same load without its wait, and the wait: r is valid after
+// tmem_wait16(r), so a load can be in flight while the last one's values are
+// worked on.
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t *r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait16(uint32_t *r) {  // (the operands keep the uses behind the wait)
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
 }
 
 // 32 lanes x 32 consecutive columns (one wait for 32 values)

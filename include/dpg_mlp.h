@@ -81,11 +81,11 @@ int dpg_mlp_train_step(dpg_mlp *mlp, const void *node_feat_dev, const uint32_t *
 
 /* Forward kernels: fused 1 runs the whole MLP per 128-row tile in one
  * persistent tcgen05 kernel (activations kept in shared memory, weights
- * streamed by TMA); fused 2 (default) is the same kernel warp-specialised
- * (a TMA warp, an MMA warp, 16 epilogue warps) so that each layer's
- * epilogue overlaps the next layer's MMAs; fused 0 runs the layer-by-layer
- * GEMMs the training step uses.  Same arithmetic (bf16 operands, FP32
- * accumulation in the same order, same epilogue). */
+ * streamed by TMA); fused 2 (default) is warp-specialised with two tiles in
+ * flight (a TMA warp, an MMA warp, 16 epilogue warps, 4 gather warps) so that
+ * one tile's epilogue overlaps the other's MMAs; fused 0 runs the
+ * layer-by-layer GEMMs the training step uses.  Same arithmetic (bf16 operands
+ * and activations, FP32 accumulation, same epilogue). */
 int dpg_mlp_set_fused(dpg_mlp *mlp, int fused);
 
 /* device time of the last forward / train step (ms) and the FLOPs it ran */
