@@ -202,15 +202,10 @@ struct dpg_mlp {
   // to K = 64), emb16 the embedding table
   __nv_bfloat16 *W16[4] = {}, *WT16[4] = {}, *emb16 = nullptr;
   // activations and backward buffers (rows_pad rows)
-  __nv_bfloat16 *X = nullptr, *H[3] = {}, *dZa = nullptr, *dZb = nullptr, *dY = nullptr, *T1 = nullptr,
-                *T2 = nullptr;
-  // training: the activations and loss gradient transposed ([cols x rows_pad],
-  // the K-major operands of the weight-gradient GEMMs), written by the
-  // producing kernels; T2 holds X^T, T1 the current layer's dZ^T
-  __nv_bfloat16 *HT[3] = {}, *dYT = nullptr;
-  float *dpart = nullptr;  // per-warp partial bias gradients [rows_pad / 32 x 256]
+  __nv_bfloat16 *X = nullptr, *H[3] = {}, *dZ[3] = {}, *dY = nullptr, *T1 = nullptr;
   __nv_bfloat16 *G[3] = {};  // gelu'(pre-activation) of layers 1-3 (training)
-  float *out = nullptr, *loss = nullptr;
+  float *out = nullptr;
+  double *loss = nullptr;
   int *err = nullptr;
   int step = 0;
   int fused = 2;  // forward kernel: 2 mlp_forward_pair, 1 mlp_forward_fused, 0 layer GEMMs
@@ -281,14 +276,13 @@ template <class T> cudaError_t dalloc(T **p, size_t count) {
   return cudaMalloc((void **)p, sizeof(T) * std::max<size_t>(count, 1));
 }
 
-// forward of rows [0, B) of the assembled X; keeps gelu'(Z) (bf16) and the
-// activations transposed (HT) when train
+// forward of rows [0, B) of the assembled X; keeps gelu'(Z) (bf16) when train
 cudaError_t forward_rows(dpg_mlp *M, int64_t B, bool train, float *out, cudaStream_t st) {
   const int64_t Bp = pad128(B);
   cudaError_t e;
   const __nv_bfloat16 *in = M->X;
   for (int l = 0; l < 3; l++) {
-    EpiBiasGelu epi{M->w[2 * l + 1], train ? M->G[l] : nullptr, M->H[l], kMlpHidden, train ? M->HT[l] : nullptr, Bp};
+    EpiBiasGelu epi{M->w[2 * l + 1], train ? M->G[l] : nullptr, M->H[l], kMlpHidden};
     e = launch_gemm(kMlpHidden, in, M->W16[l], (int)Bp, kIn[l], 1, epi, M->err, st);
     if (e != cudaSuccess) return e;
     in = M->H[l];
@@ -336,16 +330,13 @@ int dpg_mlp_create(dpg_mlp **out, int device, int n_prims, int64_t max_rows, uin
     ok = dalloc(&M->W16[l], (size_t)kOut[l] * kIn[l]) == cudaSuccess &&
          dalloc(&M->WT16[l], l < 3 ? (size_t)kOut[l] * kIn[l] : (size_t)kMlpHidden * kDY) == cudaSuccess;
   ok = ok && dalloc(&M->emb16, (size_t)n_prims * kMlpEmb) == cudaSuccess &&
-       dalloc(&M->X, (size_t)R * kMlpIn) == cudaSuccess && dalloc(&M->dZa, (size_t)R * kMlpHidden) == cudaSuccess &&
-       dalloc(&M->dZb, (size_t)R * kMlpHidden) == cudaSuccess && dalloc(&M->dY, (size_t)R * kDY) == cudaSuccess &&
-       dalloc(&M->T1, (size_t)R * kMlpHidden) == cudaSuccess && dalloc(&M->T2, (size_t)R * kMlpHidden) == cudaSuccess &&
+       dalloc(&M->X, (size_t)R * kMlpIn) == cudaSuccess && dalloc(&M->dY, (size_t)R * kDY) == cudaSuccess &&
+       dalloc(&M->T1, (size_t)kMlpOutPad * kMlpHidden) == cudaSuccess &&
        dalloc(&M->out, (size_t)R * 2) == cudaSuccess && dalloc(&M->loss, 1) == cudaSuccess &&
        dalloc(&M->err, 1) == cudaSuccess;
   for (int l = 0; l < 3 && ok; l++)
     ok = dalloc(&M->H[l], (size_t)R * kMlpHidden) == cudaSuccess && dalloc(&M->G[l], (size_t)R * kMlpHidden) == cudaSuccess &&
-         dalloc(&M->HT[l], (size_t)R * kMlpHidden) == cudaSuccess;
-  ok = ok && dalloc(&M->dYT, (size_t)R * kMlpOutPad) == cudaSuccess &&
-       dalloc(&M->dpart, (size_t)(R / 32) * kMlpHidden) == cudaSuccess;
+         dalloc(&M->dZ[l], (size_t)R * kMlpHidden) == cudaSuccess;
   ok = ok && cudaEventCreate(&M->e0) == cudaSuccess && cudaEventCreate(&M->e1) == cudaSuccess;
   ok = ok && dalloc(&M->in_node, R) == cudaSuccess && dalloc(&M->in_prim, R) == cudaSuccess &&
        dalloc(&M->in_target, 2 * R) == cudaSuccess && dalloc(&M->hp, 4) == cudaSuccess &&
@@ -408,12 +399,9 @@ void dpg_mlp_destroy(dpg_mlp *M) {
   for (int l = 0; l < 3; l++) {
     cudaFree(M->H[l]);
     cudaFree(M->G[l]);
-    cudaFree(M->HT[l]);
+    cudaFree(M->dZ[l]);
   }
-  cudaFree(M->dYT);
-  cudaFree(M->dpart);
-  void *bufs[] = {M->emb16, M->X,   M->dZa,     M->dZb,     M->dY,     M->T1,  M->T2,
-                  M->out,   M->loss, M->err, M->in_node, M->in_prim, M->in_target, M->hp};
+  void *bufs[] = {M->emb16, M->X, M->dY, M->T1, M->out, M->loss, M->err, M->in_node, M->in_prim, M->in_target, M->hp};
   for (void *b : bufs) cudaFree(b);
   if (M->hp_host) cudaFreeHost(M->hp_host);
   if (M->h_err) cudaFreeHost(M->h_err);
@@ -475,7 +463,7 @@ int dpg_mlp_forward(dpg_mlp *M, const void *node_feat_dev, const uint32_t *node_
     const int64_t B = std::min(M->max_rows, n - r0), Bp = pad128(B);
     const int64_t chunks = Bp * (kMlpIn / 8);
     mlp_assemble<<<(unsigned)((chunks + 255) / 256), 256, 0, st>>>(nf, M->emb16, node_dev + r0, prim_dev + r0, B, Bp,
-                                                                    M->X, nullptr);
+                                                                    M->X);
     if (forward_rows(M, B, false, out_dev + 2 * r0, st) != cudaSuccess) return DPG_ERR_CUDA;
     flops += forward_flops(Bp);
   }
@@ -493,51 +481,48 @@ int dpg_mlp_forward(dpg_mlp *M, const void *node_feat_dev, const uint32_t *node_
 // fixed input buffers and the hyper-parameters from M->hp (capturable).
 static cudaError_t enqueue_train(dpg_mlp *M, const __nv_bfloat16 *nf, int64_t B, cudaStream_t st) {
   const int64_t Bp = pad128(B);
-  // split-K of the weight-gradient GEMMs (K = the batch): about one CTA per SM
-  auto split_for = [&](int rows) {
-    const int tiles = (rows + 127) / 128;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(std::max(M->sm_count, 1) / tiles, Bp / 512));
-  };
   cudaMemsetAsync(M->err, 0, sizeof(int), st);
-  cudaMemsetAsync(M->loss, 0, sizeof(float), st);
+  cudaMemsetAsync(M->loss, 0, sizeof(double), st);
   for (int i = 0; i < DPG_MLP_NPARAM; i++) cudaMemsetAsync(M->g[i], 0, sizeof(float) * M->n[i], st);
   const int64_t chunks = Bp * (kMlpIn / 8);
-  mlp_assemble<<<(unsigned)((chunks + 255) / 256), 256, 0, st>>>(nf, M->emb16, M->in_node, M->in_prim, B, Bp, M->X,
-                                                                  M->T2);
+  mlp_assemble<<<(unsigned)((chunks + 255) / 256), 256, 0, st>>>(nf, M->emb16, M->in_node, M->in_prim, B, Bp, M->X);
   cudaError_t e = forward_rows(M, B, true, M->out, st);
   if (e != cudaSuccess) return e;
-  mlp_loss<<<(unsigned)((Bp + 255) / 256), 256, 0, st>>>(M->out, M->in_target, B, Bp, M->hp, M->dY, M->loss, M->dYT,
+  mlp_loss<<<(unsigned)((Bp + 255) / 256), 256, 0, st>>>(M->out, M->in_target, B, Bp, M->hp, M->dY, M->loss,
                                                           M->g[DPG_MLP_B4]);
-  // the transposed operands and the bias gradients come from the kernels that
-  // produce the activations and dZ (Bp is a multiple of 128: whole warps of rows)
-  auto bias_grad = [&](int which) {  // the partial column sums of the last dZ into g[which]
-    sum_rows_f32<<<dim3(kMlpHidden / 32, 32), 256, 0, st>>>(M->dpart, Bp / 32, kMlpHidden, kMlpHidden, M->g[which]);
-  };
-  // layer 4: dW4 = dY^T H3 (16 rows), dZ3 = (dY W4) * gelu'(Z3) with dZ3^T and db3
-  e = launch_gemm(kMlpHidden, M->dYT, M->HT[2], kMlpOutPad, (int)Bp, split_for(kMlpOutPad),
-                  EpiAtomicF32{M->g[DPG_MLP_W4], kMlpHidden, kMlpHidden}, M->err, st);
+  // dZ3 = (dY W4) gelu'(Z3), dZ2, dZ1
+  e = launch_gemm(kMlpHidden, M->dY, M->WT16[3], (int)Bp, kDY, 1, EpiGeluGrad{M->G[2], M->dZ[2], kMlpHidden}, M->err, st);
+  for (int l = 2; l >= 1 && e == cudaSuccess; l--)
+    e = launch_gemm(kMlpHidden, M->dZ[l], M->WT16[l], (int)Bp, kMlpHidden, 1,
+                    EpiGeluGrad{M->G[l - 1], M->dZ[l - 1], kMlpHidden}, M->err, st);
+  // only the embedding columns 80..95 of dX are needed: rows 80..95 of W1^T
   if (e == cudaSuccess)
-    e = launch_gemm(kMlpHidden, M->dY, M->WT16[3], (int)Bp, kDY, 1,
-                    EpiGeluGrad{M->G[2], M->dZa, kMlpHidden, M->T1, Bp, M->dpart}, M->err, st);
-  if (e == cudaSuccess) bias_grad(DPG_MLP_B3);
-  __nv_bfloat16 *dz = M->dZa, *dz_next = M->dZb;
-  for (int l = 2; l >= 0 && e == cudaSuccess; l--) {  // layers 3, 2, 1: dZ^T in T1
-    const __nv_bfloat16 *h_inT = l > 0 ? M->HT[l - 1] : M->T2;
-    e = launch_gemm(kIn[l], M->T1, h_inT, kMlpHidden, (int)Bp, split_for(kMlpHidden),
-                    EpiAtomicF32{M->g[2 * l], kIn[l], kIn[l]},
-                    M->err, st);
-    if (e != cudaSuccess) break;
-    if (l > 0)
-      e = launch_gemm(kMlpHidden, dz, M->WT16[l], (int)Bp, kMlpHidden, 1,
-                      EpiGeluGrad{M->G[l - 1], dz_next, kMlpHidden, M->T1, Bp, M->dpart}, M->err, st);
-    if (e == cudaSuccess && l > 0) bias_grad(2 * (l - 1) + 1);
-    else
-      // only the embedding columns 80..95 of dX are needed: rows 80..95 of W1^T
-      e = launch_gemm(kMlpEmb, dz, M->WT16[0] + (size_t)kMlpNodeFeat * kMlpHidden, (int)Bp, kMlpHidden, 1,
-                      EpiEmbGrad{M->in_prim, M->g[DPG_MLP_EMB], B}, M->err, st);
-    std::swap(dz, dz_next);
-  }
+    e = launch_gemm(kMlpEmb, M->dZ[0], M->WT16[0] + (size_t)kMlpNodeFeat * kMlpHidden, (int)Bp, kMlpHidden, 1,
+                    EpiEmbGrad{M->in_prim, M->g[DPG_MLP_EMB], B}, M->err, st);
   if (e != cudaSuccess) return e;
+  // weight and bias gradients: the layers share the SMs by the bytes they read
+  WgradArgs wa{};
+  const int64_t n_chunks = Bp / 64;
+  const int weight[4] = {6, 8, 8, 5};  // blocks of 64 columns a chunk
+  int cta = 0;
+  for (int l = 0; l < 4; l++) {
+    WgradJob &j = wa.job[l];
+    const __nv_bfloat16 *a = l < 3 ? M->dZ[l] : M->H[2], *b = l == 0 ? M->X : l < 3 ? M->H[l - 1] : M->dY;
+    if (!make_kmajor_map(&j.a, a, (uint64_t)Bp, kMlpHidden, 64) ||
+        !make_kmajor_map(&j.b, b, (uint64_t)Bp, l == 0 ? kMlpIn : l < 3 ? kMlpHidden : kDY, 64))
+      return cudaErrorNotSupported;
+    j.g = M->g[2 * l];
+    j.db = l < 3 ? M->g[2 * l + 1] : nullptr;
+    j.ld = l < 3 ? kIn[l] : kMlpHidden;
+    j.n = l == 0 ? kMlpNodeFeat + kMlpEmb : l < 3 ? kMlpHidden : kMlpOutPad;
+    j.transposed = l == 3;
+    j.cta0 = cta;
+    j.ctas = (int)std::max<int64_t>(1, std::min<int64_t>(n_chunks, (int64_t)std::max(M->sm_count, 4) * weight[l] / 27));
+    cta += j.ctas;
+  }
+  e = cudaFuncSetAttribute(mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem);
+  if (e != cudaSuccess) return e;
+  mlp_wgrad<<<cta, kWgThreads, kWgSmem, st>>>(wa, n_chunks, M->err);
   // Adam on every parameter and the bf16 operand copies, one launch
   static_assert(kAdamSegs == DPG_MLP_NPARAM, "one Adam segment per parameter");
   AdamArgs aa{};
@@ -603,10 +588,10 @@ int dpg_mlp_train_step(dpg_mlp *M, const void *node_feat_dev, const uint32_t *no
     return DPG_ERR_CUDA;
   }
   cudaEventRecord(M->e1, st);
-  float hl = 0;
-  cudaMemcpyAsync(&hl, M->loss, sizeof(float), cudaMemcpyDeviceToHost, st);
+  double hl = 0;
+  cudaMemcpyAsync(&hl, M->loss, sizeof(double), cudaMemcpyDeviceToHost, st);
   if (cudaStreamSynchronize(st) != cudaSuccess) return DPG_ERR_CUDA;
-  if (loss) *loss = hl / (float)B;
+  if (loss) *loss = (float)(hl / (double)B);
   M->ms_due = true;
   // forward + the two backward GEMMs per layer
   M->last_flops = 3.0 * forward_flops(pad128(B));

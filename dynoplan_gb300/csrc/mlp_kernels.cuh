@@ -139,17 +139,13 @@ __global__ void __launch_bounds__(8 * kFeatNodes) mlp_node_features(NodeView nv,
   store8(feat + n * kMlpNodeFeat + 16 + 8 * t, make_uint4(w[0], w[1], w[2], w[3]), vec);
 }
 
-// X[b] = [node_feat[node[b]] | emb[prim[b]]], one thread per 16-byte chunk
-// Thread per (8-column chunk c, row b), rows fastest; when XT is set the
-// rows are also written transposed (XT[col * B_pad + b]: consecutive threads
-// store consecutive rows of a column).
+// X[b] = [node_feat[node[b]] | emb[prim[b]] | 0], one thread per 16-byte chunk
 static __global__ void mlp_assemble(const __nv_bfloat16 *node_feat, const __nv_bfloat16 *emb, const uint32_t *node,
-                             const uint32_t *prim, int64_t B, int64_t B_pad, __nv_bfloat16 *X,
-                             __nv_bfloat16 *XT) {
+                                    const uint32_t *prim, int64_t B, int64_t B_pad, __nv_bfloat16 *X) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int c = (int)(i / B_pad);
-  const int64_t b = i - (int64_t)c * B_pad;
-  if (c >= kMlpIn / 8) return;
+  const int64_t b = i / (kMlpIn / 8);
+  const int c = (int)(i % (kMlpIn / 8));
+  if (b >= B_pad) return;
   uint4 v = make_uint4(0, 0, 0, 0);
   if (b < B) {
     if (c < kMlpNodeFeat / 8)
@@ -157,12 +153,7 @@ static __global__ void mlp_assemble(const __nv_bfloat16 *node_feat, const __nv_b
     else if (c < (kMlpNodeFeat + kMlpEmb) / 8)
       v = reinterpret_cast<const uint4 *>(emb + (int64_t)prim[b] * kMlpEmb)[c - kMlpNodeFeat / 8];
   }
-  reinterpret_cast<uint4 *>(X + b * kMlpIn)[c] = v;
-  if (XT) {
-    const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&v);
-#pragma unroll
-    for (int j = 0; j < 8; j++) XT[(int64_t)(8 * c + j) * B_pad + b] = h[j];
-  }
+  reinterpret_cast<uint4 *>(X)[i] = v;
 }
 
 __device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
@@ -171,12 +162,10 @@ __device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + __expf(-
 // loss = mean_b [softplus(l) - y l  +  0.5 w (c - t)^2]; dY (bf16, B x 64,
 // columns >= 2 zero) = d loss / d [l, c]; loss accumulated into *loss_sum
 // (ctg_weight = hp[1]: the step's hyper-parameters live in device memory so a
-// captured training step can be replayed with new values)
-// When dYT is set, also the first kMlpOutPad columns of dY transposed
-// (dYT[j * B_pad + b]) and the head's bias gradient (column sums of the bf16
-// dY, two non-zero columns) added into db.
+// captured training step can be replayed with new values), and the head's bias
+// gradient (column sums of the bf16 dY, two non-zero columns) added into db.
 static __global__ void mlp_loss(const float *out, const float *target, int64_t B, int64_t B_pad, const float *hp,
-                         __nv_bfloat16 *dY, float *loss_sum, __nv_bfloat16 *dYT, float *db) {
+                         __nv_bfloat16 *dY, double *loss_sum, float *db) {
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const float ctg_weight = hp[1];
   float l = 0.f, g0 = 0.f, g1 = 0.f;
@@ -200,10 +189,6 @@ static __global__ void mlp_loss(const float *out, const float *target, int64_t B
     uint4 *dst = reinterpret_cast<uint4 *>(dY + b * 64);
 #pragma unroll
     for (int j = 0; j < 8; j++) dst[j] = reinterpret_cast<const uint4 *>(row)[j];
-    if (dYT) {
-#pragma unroll
-      for (int j = 0; j < kMlpOutPad; j++) dYT[j * B_pad + b] = row[j];
-    }
     g0 = __bfloat162float(row[0]);
     g1 = __bfloat162float(row[1]);
   }
@@ -213,26 +198,18 @@ static __global__ void mlp_loss(const float *out, const float *target, int64_t B
     g1 += __shfl_down_sync(0xffffffffu, g1, o);
   }
   if ((threadIdx.x & 31) == 0) {
-    if (l != 0.f) atomicAdd(loss_sum, l);
+    if (l != 0.f) atomicAdd(loss_sum, (double)l);
     if (db && g0 != 0.f) atomicAdd(db, g0);
     if (db && g1 != 0.f) atomicAdd(db + 1, g1);
   }
 }
 
 // dZ = dH * gelu'(Z) (gelu' kept in bf16 by the forward epilogue): the
-// epilogue of dH = dZnext * W.  Optionally also
-// dZ transposed (dzT[col * ldt + row], the K-major operand of the
-// weight-gradient GEMM) and partial bias gradients: the column sums of the
-// bf16 dZ over each warp's 32 rows, stored (no atomics) at row
-// 4 blockIdx.x + (warp % 4) of dpart [M / 32 x ld], summed by sum_rows_f32.
-// The partial sums need whole warps of rows: M a multiple of 128.
+// epilogue of dH = dZnext * W.
 struct EpiGeluGrad {
   const __nv_bfloat16 *dgelu;
   __nv_bfloat16 *dz;
   int ld;
-  __nv_bfloat16 *dzT = nullptr;
-  int64_t ldt = 0;
-  float *dpart = nullptr;
   __device__ void operator()(int row, int c0, const float *v) const {
     __align__(16) __nv_bfloat16 h[16], d[16];
     const uint4 *gd = reinterpret_cast<const uint4 *>(dgelu + (int64_t)row * ld + c0);
@@ -243,21 +220,6 @@ struct EpiGeluGrad {
     uint4 *dst = reinterpret_cast<uint4 *>(dz + (int64_t)row * ld + c0);
     dst[0] = reinterpret_cast<const uint4 *>(h)[0];
     dst[1] = reinterpret_cast<const uint4 *>(h)[1];
-    float *prow = dpart ? dpart + ((int64_t)blockIdx.x * 4 + ((threadIdx.x >> 5) & 3)) * ld + c0 : nullptr;
-    if (dzT) {  // the transposed store also sums the staged columns
-      store_transposed16(dzT, ldt, row, c0, h, prow);
-    } else if (prow) {
-      const int lane = threadIdx.x & 31;
-      float mine = 0.f;  // lane j < 16 keeps column c0 + j
-#pragma unroll
-      for (int j = 0; j < 16; j++) {
-        float t = __bfloat162float(h[j]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (lane == j) mine = t;
-      }
-      if (lane < 16) prow[lane] = mine;
-    }
   }
 };
 
@@ -290,27 +252,173 @@ static __global__ void transpose_bf16(const __nv_bfloat16 *in, __nv_bfloat16 *ou
   }
 }
 
-// out[j] += sum_r part[r * ld + j] for j < n.  Block = 32 columns x 8 warps;
-// gridDim.y splits the rows; one atomic per (block, column).
-static __global__ void __launch_bounds__(256) sum_rows_f32(const float *part, int64_t rows, int ld, int n,
-                                                           float *out) {
-  __shared__ float red[8][33];
-  const int j = blockIdx.x * 32 + (threadIdx.x & 31), sg = threadIdx.x >> 5;
-  const int64_t per = (rows + gridDim.y - 1) / gridDim.y;
-  const int64_t r0 = blockIdx.y * per, r1 = min(rows, r0 + per);
-  float s = 0.f;
-  if (j < n) {
-#pragma unroll 4
-    for (int64_t r = r0 + sg; r < r1; r += 8) s += part[r * ld + j];
+// ---------------------------------------------------------------------------
+// Weight and bias gradients of all four layers in one launch:
+//   g[m][n] += sum_b a[b][m] b[b][n]      a, b bf16 row-major, a row per pair
+// (layers 1-3: a = dZ, b = the layer's input; layer 4: a = H3, b = dY, stored
+// transposed).  The contraction runs over the rows, so both operands are read
+// MN-major straight from the row-major activations (boxes of 64 rows x 64
+// columns by TMA): no transposed copies are written.  A layer's CTAs take
+// ranges of 64-row chunks; a CTA holds the whole gradient, two M = 128 tiles of
+// up to 256 columns, in TMEM, so each operand is read once, and adds it to g at
+// the end (float4 atomics).  Warps 4-7 sum the columns of a (the bias
+// gradients) from the staged tiles while the tensor cores use them.
+// Bound by reading the operands (2 x 33.5 MB a hidden layer at 65,536 rows):
+// all four layers 48 us; as transposed copies written by the layers'
+// epilogues (another 230 MB) and a split-K launch per layer 155 us, without the
+// writes.  Every wait is bounded, as above.
+struct alignas(128) WgradJob {
+  CUtensorMap a, b;  // boxes of 64 columns x 64 rows
+  float *g, *db;     // db: column sums of a (may be null)
+  int ld, n;         // row stride of g; columns of b used (multiple of 16)
+  int transposed;    // g[n][m] (the two non-zero columns of dY) instead of g[m][n]
+  int cta0, ctas;    // the layer's CTAs
+};
+struct alignas(128) WgradArgs {
+  WgradJob job[4];
+};
+constexpr int kWgThreads = 256, kWgStages = 3;
+constexpr uint32_t kWgBlock = 64 * 128;        // 64 rows x 64 columns
+constexpr uint32_t kWgStage = 8 * kWgBlock;    // a: 256 columns, b: up to 256
+constexpr size_t kWgSmem = 1024 + kWgStages * kWgStage + 256;
+
+static __global__ void __launch_bounds__(kWgThreads, 1) mlp_wgrad(const __grid_constant__ WgradArgs A, int64_t n_chunks,
+                                                                  int *err) {
+  extern __shared__ unsigned char smem_raw[];
+  const uint32_t raw = umma::smem_u32(smem_raw);
+  unsigned char *base = smem_raw + ((1024 - (raw & 1023)) & 1023);
+  uint64_t *full = reinterpret_cast<uint64_t *>(base + kWgStages * kWgStage);
+  uint64_t *empty = full + kWgStages, *done = empty + kWgStages;
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
+  volatile int *bad = reinterpret_cast<volatile int *>(tslot + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int ji = 0;
+  while (ji < 3 && (int)blockIdx.x >= A.job[ji].cta0 + A.job[ji].ctas) ji++;
+  const WgradJob &J = A.job[ji];
+  const int64_t rel = (int)blockIdx.x - J.cta0;
+  const int64_t c0 = n_chunks * rel / J.ctas, c1 = n_chunks * (rel + 1) / J.ctas;
+  const int n = (int)(c1 - c0), b_blocks = (J.n + 63) / 64;
+  const uint32_t bytes = (4 + b_blocks) * kWgBlock;
+  if (tid == 0) {
+    for (int s = 0; s < kWgStages; s++) {
+      umma::mbar_init(&full[s], 1);
+      umma::mbar_init(&empty[s], J.db ? 5 : 1);  // the MMAs, and the four summing warps
+    }
+    umma::mbar_init(done, 1);
+    umma::mbar_fence_init();
+    *bad = 0;
   }
-  red[sg][threadIdx.x & 31] = s;
+  if (warp == 0) {
+    umma::tmem_alloc(tslot, 512);
+    umma::tmem_relinquish();
+  }
+  umma::fence_before_sync();
   __syncthreads();
-  if (sg == 0 && j < n) {
-    float t = 0.f;
+  umma::fence_after_sync();
+  const uint32_t tmem = *tslot;
+
+  int loads = 0;  // (thread 0) chunks whose loads were issued
+  if (tid == 0) {
+    for (int i = 0; i < n; i++) {
+      const int s = i % kWgStages;
+      if ((i >= kWgStages && !umma::mbar_wait(&empty[s], ((i / kWgStages) - 1) & 1)) || *bad) {
+        *bad = 1;
+        break;
+      }
+      unsigned char *st = base + s * kWgStage;
+      const int row = (int)(64 * (c0 + i));
+      umma::mbar_arrive_expect_tx(&full[s], bytes);
+      for (int k = 0; k < 4; k++) umma::tma_load_2d(st + k * kWgBlock, &J.a, 64 * k, row, &full[s]);
+      for (int k = 0; k < b_blocks; k++) umma::tma_load_2d(st + (4 + k) * kWgBlock, &J.b, 64 * k, row, &full[s]);
+      loads = i + 1;
+    }
+  } else if (warp == 1) {
+    const uint32_t idesc = umma::idesc_bf16_f32(128, J.n) | umma::kIdescMnMajorAB;
+    const uint64_t ad = umma::sdesc_mnmajor_sw128(umma::smem_u32(base), kWgBlock);
+    const uint64_t bd = ad + (4 * kWgBlock >> 4);
+    uint32_t s = 0, parity = 0;
+    bool ok = true;
+    for (int i = 0; i < n && ok; i++) {
+      if (!umma::mbar_wait_warp(&full[s], parity)) {
+        ok = false;
+        break;
+      }
+      umma::fence_after_sync();
+      const uint64_t so = s * (kWgStage >> 4);
+      if (umma::elect_one()) {
 #pragma unroll
-    for (int k = 0; k < 8; k++) t += red[k][threadIdx.x];
-    atomicAdd(out + j, t);
+        for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+          for (int kk = 0; kk < 4; kk++)  // 16 rows a step
+            umma::mma_bf16(tmem + 256u * mt, ad + so + mt * (2 * kWgBlock >> 4) + kk * (2048 >> 4),
+                           bd + so + kk * (2048 >> 4), idesc, (i > 0 || kk > 0) ? 1u : 0u);
+        umma::commit(&empty[s]);
+      }
+      __syncwarp();
+      if (++s == kWgStages) {
+        s = 0;
+        parity ^= 1u;
+      }
+    }
+    if (!ok && lane == 0) *bad = 1;
+    if (umma::elect_one()) umma::commit(done);  // once every MMA issued above is complete
+    __syncwarp();
+  } else if (warp >= 4 && J.db) {
+    // column sums of a: a thread two columns (word w of block k), over the rows
+    const int k = warp - 4;
+    float s0 = 0.f, s1 = 0.f;
+    bool ok = true;
+    for (int i = 0; i < n && ok; i++) {
+      const int s = i % kWgStages;
+      ok = umma::mbar_wait_warp(&full[s], (i / kWgStages) & 1);
+      if (!ok) break;
+      const unsigned char *t = base + s * kWgStage + k * kWgBlock;
+#pragma unroll 16
+      for (int r = 0; r < 64; r++) {
+        const uint32_t v = *reinterpret_cast<const uint32_t *>(t + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + 4 * (lane & 3));
+        s0 += __uint_as_float(v << 16);
+        s1 += __uint_as_float(v & 0xffff0000u);
+      }
+      __syncwarp();
+      if (lane == 0) umma::mbar_arrive(&empty[s]);
+    }
+    if (!ok) {
+      if (lane == 0) *bad = 1;
+    } else if (n > 0) {
+      atomicAdd(J.db + 64 * k + 2 * lane, s0);
+      atomicAdd(J.db + 64 * k + 2 * lane + 1, s1);
+    }
   }
+  __syncwarp();
+  const bool fin = umma::mbar_wait(done, 0);
+  const bool failed = __syncthreads_or(!fin || *bad);
+  if (failed) {
+    if (tid == 0) {
+      atomicExch(err, 1);
+      // copies still in flight land before the block's shared memory goes
+      for (int i = max(0, loads - kWgStages); i < loads; i++)
+        umma::mbar_wait(&full[i % kWgStages], (i / kWgStages) & 1, 1u << 20);
+    }
+  } else if (n > 0) {
+    umma::fence_after_sync();
+    const int q = warp & 3, mt = warp >> 2, m = 128 * mt + 32 * q + lane;
+    const uint32_t src = tmem + ((uint32_t)(32 * q) << 16) + 256u * (uint32_t)mt;
+    for (int k = 0; k < J.n; k += 16) {
+      float v[16];
+      umma::tmem_ld16(src + k, v);
+      if (J.transposed) {
+        atomicAdd(J.g + m, v[0]);
+        atomicAdd(J.g + J.ld + m, v[1]);
+      } else {
+        float4 *dst = reinterpret_cast<float4 *>(J.g + (int64_t)m * J.ld + k);
+#pragma unroll
+        for (int j = 0; j < 4; j++) atomicAdd(dst + j, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
+      }
+    }
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
 
 // Adam over every parameter in one launch: segment s is elements

@@ -107,6 +107,21 @@ __device__ __forceinline__ uint64_t sdesc_kmajor_sw64(uint32_t saddr) {
   d |= (uint64_t)4 << 61;  // 64-byte swizzle
   return d;
 }
+// MN-major with the 128-byte swizzle: the tile is stored as blocks of 64
+// columns (M or N), a block's rows (K) 128 bytes each in the same swizzle,
+// 8-row groups 1024 bytes apart (stride byte offset), the next 64 columns
+// block_bytes on (leading byte offset) -- what a TMA box of 64 columns of a
+// row-major [K x MN] matrix leaves.
+__device__ __forceinline__ uint64_t sdesc_mnmajor_sw128(uint32_t saddr, uint32_t block_bytes) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+  d |= (uint64_t)(block_bytes >> 4) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+constexpr uint32_t kIdescMnMajorAB = (1u << 15) | (1u << 16);  // A and B MN-major
 // Instruction descriptor of kind::f16: BF16 A and B (K-major), FP32 D, M x N.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
   return (1u << 4)                       // D format F32
