@@ -204,8 +204,8 @@ struct dpg_mlp {
   // activations and backward buffers (rows_pad rows)
   __nv_bfloat16 *X = nullptr, *H[3] = {}, *dZ[3] = {}, *dY = nullptr, *T1 = nullptr;
   __nv_bfloat16 *G[3] = {};  // gelu'(pre-activation) of layers 1-3 (training)
-  float *out = nullptr;
-  double *loss = nullptr;
+  double *loss = nullptr;  // one allocation: the loss, then the gradients g[]
+  size_t sums_bytes = 0;
   int *err = nullptr;
   int step = 0;
   int fused = 2;  // forward kernel: 2 mlp_forward_pair, 1 mlp_forward_fused, 0 layer GEMMs
@@ -276,8 +276,8 @@ template <class T> cudaError_t dalloc(T **p, size_t count) {
   return cudaMalloc((void **)p, sizeof(T) * std::max<size_t>(count, 1));
 }
 
-// forward of rows [0, B) of the assembled X; keeps gelu'(Z) (bf16) when train
-cudaError_t forward_rows(dpg_mlp *M, int64_t B, bool train, float *out, cudaStream_t st) {
+// hidden layers of rows [0, B) of the assembled X; keeps gelu'(Z) (bf16) when train
+cudaError_t hidden_rows(dpg_mlp *M, int64_t B, bool train, cudaStream_t st) {
   const int64_t Bp = pad128(B);
   cudaError_t e;
   const __nv_bfloat16 *in = M->X;
@@ -287,6 +287,13 @@ cudaError_t forward_rows(dpg_mlp *M, int64_t B, bool train, float *out, cudaStre
     if (e != cudaSuccess) return e;
     in = M->H[l];
   }
+  return cudaSuccess;
+}
+// .. and the head's outputs
+cudaError_t forward_rows(dpg_mlp *M, int64_t B, float *out, cudaStream_t st) {
+  const int64_t Bp = pad128(B);
+  const cudaError_t e = hidden_rows(M, B, false, st);
+  if (e != cudaSuccess) return e;
   return launch_gemm(kMlpOutPad, M->H[2], M->W16[3], (int)Bp, kMlpHidden, 1, EpiBias{M->w[DPG_MLP_B4], out, 2, 2, B},
                      M->err, st);
 }
@@ -323,16 +330,25 @@ int dpg_mlp_create(dpg_mlp **out, int device, int n_prims, int64_t max_rows, uin
   bool ok = cudaStreamCreateWithFlags(&M->stream, cudaStreamDefault) == cudaSuccess;
   for (int i = 0; i < DPG_MLP_NPARAM && ok; i++) {
     M->n[i] = sizes[i];
-    ok = dalloc(&M->w[i], sizes[i]) == cudaSuccess && dalloc(&M->g[i], sizes[i]) == cudaSuccess &&
-         dalloc(&M->m[i], sizes[i]) == cudaSuccess && dalloc(&M->v[i], sizes[i]) == cudaSuccess;
+    ok = dalloc(&M->w[i], sizes[i]) == cudaSuccess && dalloc(&M->m[i], sizes[i]) == cudaSuccess &&
+         dalloc(&M->v[i], sizes[i]) == cudaSuccess;
   }
+  // the loss and the gradients, cleared by one memset each step (256-byte aligned parts)
+  M->sums_bytes = 256;
+  size_t g_at[DPG_MLP_NPARAM];
+  for (int i = 0; i < DPG_MLP_NPARAM; i++) {
+    g_at[i] = M->sums_bytes;
+    M->sums_bytes += (sizeof(float) * (size_t)sizes[i] + 255) / 256 * 256;
+  }
+  ok = ok && dalloc(&M->loss, M->sums_bytes / sizeof(double)) == cudaSuccess;
+  for (int i = 0; i < DPG_MLP_NPARAM && ok; i++)
+    M->g[i] = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(M->loss) + g_at[i]);
   for (int l = 0; l < 4 && ok; l++)
     ok = dalloc(&M->W16[l], (size_t)kOut[l] * kIn[l]) == cudaSuccess &&
          dalloc(&M->WT16[l], l < 3 ? (size_t)kOut[l] * kIn[l] : (size_t)kMlpHidden * kDY) == cudaSuccess;
   ok = ok && dalloc(&M->emb16, (size_t)n_prims * kMlpEmb) == cudaSuccess &&
        dalloc(&M->X, (size_t)R * kMlpIn) == cudaSuccess && dalloc(&M->dY, (size_t)R * kDY) == cudaSuccess &&
        dalloc(&M->T1, (size_t)kMlpOutPad * kMlpHidden) == cudaSuccess &&
-       dalloc(&M->out, (size_t)R * 2) == cudaSuccess && dalloc(&M->loss, 1) == cudaSuccess &&
        dalloc(&M->err, 1) == cudaSuccess;
   for (int l = 0; l < 3 && ok; l++)
     ok = dalloc(&M->H[l], (size_t)R * kMlpHidden) == cudaSuccess && dalloc(&M->G[l], (size_t)R * kMlpHidden) == cudaSuccess &&
@@ -359,6 +375,8 @@ int dpg_mlp_create(dpg_mlp **out, int device, int n_prims, int64_t max_rows, uin
   }
   cudaStream_t st = M->stream;
   cudaMemsetAsync(M->err, 0, sizeof(int), st);
+  cudaMemsetAsync(M->loss, 0, M->sums_bytes, st);
+  cudaMemsetAsync(M->dY, 0, sizeof(__nv_bfloat16) * R * kDY, st);  // columns 16.. stay zero
   const float stdv[DPG_MLP_NPARAM] = {1.f / sqrtf(96.f), 0, 1.f / 16.f, 0, 1.f / 16.f, 0, 1.f / 16.f, 0, 0.5f};
   for (int i = 0; i < DPG_MLP_NPARAM; i++) {
     const int64_t n = M->n[i];
@@ -371,7 +389,6 @@ int dpg_mlp_create(dpg_mlp **out, int device, int n_prims, int64_t max_rows, uin
       cudaMemsetAsync(M->w[i], 0, sizeof(float) * n, st);
     cudaMemsetAsync(M->m[i], 0, sizeof(float) * n, st);
     cudaMemsetAsync(M->v[i], 0, sizeof(float) * n, st);
-    cudaMemsetAsync(M->g[i], 0, sizeof(float) * n, st);
   }
   for (int i = 0; i < DPG_MLP_NPARAM; i++) refresh_bf16(M, i, st);
   if (cudaStreamSynchronize(st) != cudaSuccess) {
@@ -388,7 +405,6 @@ void dpg_mlp_destroy(dpg_mlp *M) {
   if (M->stream) cudaStreamSynchronize(M->stream);
   for (int i = 0; i < DPG_MLP_NPARAM; i++) {
     cudaFree(M->w[i]);
-    cudaFree(M->g[i]);
     cudaFree(M->m[i]);
     cudaFree(M->v[i]);
   }
@@ -401,7 +417,7 @@ void dpg_mlp_destroy(dpg_mlp *M) {
     cudaFree(M->G[l]);
     cudaFree(M->dZ[l]);
   }
-  void *bufs[] = {M->emb16, M->X, M->dY, M->T1, M->out, M->loss, M->err, M->in_node, M->in_prim, M->in_target, M->hp};
+  void *bufs[] = {M->emb16, M->X, M->dY, M->T1, M->loss, M->err, M->in_node, M->in_prim, M->in_target, M->hp};
   for (void *b : bufs) cudaFree(b);
   if (M->hp_host) cudaFreeHost(M->hp_host);
   if (M->h_err) cudaFreeHost(M->h_err);
@@ -464,7 +480,7 @@ int dpg_mlp_forward(dpg_mlp *M, const void *node_feat_dev, const uint32_t *node_
     const int64_t chunks = Bp * (kMlpIn / 8);
     mlp_assemble<<<(unsigned)((chunks + 255) / 256), 256, 0, st>>>(nf, M->emb16, node_dev + r0, prim_dev + r0, B, Bp,
                                                                     M->X);
-    if (forward_rows(M, B, false, out_dev + 2 * r0, st) != cudaSuccess) return DPG_ERR_CUDA;
+    if (forward_rows(M, B, out_dev + 2 * r0, st) != cudaSuccess) return DPG_ERR_CUDA;
     flops += forward_flops(Bp);
   }
   cudaEventRecord(M->e1, st);
@@ -482,14 +498,14 @@ int dpg_mlp_forward(dpg_mlp *M, const void *node_feat_dev, const uint32_t *node_
 static cudaError_t enqueue_train(dpg_mlp *M, const __nv_bfloat16 *nf, int64_t B, cudaStream_t st) {
   const int64_t Bp = pad128(B);
   cudaMemsetAsync(M->err, 0, sizeof(int), st);
-  cudaMemsetAsync(M->loss, 0, sizeof(double), st);
-  for (int i = 0; i < DPG_MLP_NPARAM; i++) cudaMemsetAsync(M->g[i], 0, sizeof(float) * M->n[i], st);
+  cudaMemsetAsync(M->loss, 0, M->sums_bytes, st);  // the loss and every gradient
   const int64_t chunks = Bp * (kMlpIn / 8);
   mlp_assemble<<<(unsigned)((chunks + 255) / 256), 256, 0, st>>>(nf, M->emb16, M->in_node, M->in_prim, B, Bp, M->X);
-  cudaError_t e = forward_rows(M, B, true, M->out, st);
+  cudaError_t e = hidden_rows(M, B, true, st);
+  if (e == cudaSuccess)
+    e = launch_gemm(kMlpOutPad, M->H[2], M->W16[3], (int)Bp, kMlpHidden, 1,
+                    EpiHeadLoss{M->w[DPG_MLP_B4], M->in_target, M->hp, B, M->dY, M->loss, M->g[DPG_MLP_B4]}, M->err, st);
   if (e != cudaSuccess) return e;
-  mlp_loss<<<(unsigned)((Bp + 255) / 256), 256, 0, st>>>(M->out, M->in_target, B, Bp, M->hp, M->dY, M->loss,
-                                                          M->g[DPG_MLP_B4]);
   // dZ3 = (dY W4) gelu'(Z3), dZ2, dZ1
   e = launch_gemm(kMlpHidden, M->dY, M->WT16[3], (int)Bp, kDY, 1, EpiGeluGrad{M->G[2], M->dZ[2], kMlpHidden}, M->err, st);
   for (int l = 2; l >= 1 && e == cudaSuccess; l--)

@@ -159,73 +159,60 @@ static __global__ void mlp_assemble(const __nv_bfloat16 *node_feat, const __nv_b
 __device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
 __device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + __expf(-x)); }
 
-// loss = mean_b [softplus(l) - y l  +  0.5 w (c - t)^2]; dY (bf16, B x 64,
-// columns >= 2 zero) = d loss / d [l, c]; loss accumulated into *loss_sum
-// (ctg_weight = hp[1]: the step's hyper-parameters live in device memory so a
-// captured training step can be replayed with new values), and the head's bias
-// gradient (column sums of the bf16 dY, two non-zero columns) added into db.
-static __global__ void mlp_loss(const float *out, const float *target, int64_t B, int64_t B_pad, const float *hp,
-                         __nv_bfloat16 *dY, double *loss_sum, float *db) {
-  const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const float ctg_weight = hp[1];
-  float l = 0.f, g0 = 0.f, g1 = 0.f;
-  if (b < B_pad) {
-    __align__(16) __nv_bfloat16 row[64];
-#pragma unroll
-    for (int j = 0; j < 64; j++) row[j] = __float2bfloat16_rn(0.f);
-    if (b < B) {  // a NaN target leaves its head out of the loss
-      const float lg = out[b * 2], ct = out[b * 2 + 1];
-      const float y = target[b * 2], t = target[b * 2 + 1];
+// The training step's head: [l, c] = acc + bias, then
+//   loss = mean_b [softplus(l) - y l  +  0.5 w (c - t)^2]
+// (a NaN target leaves its head out of the loss).  Writes dY = d loss / d [l, c]
+// (bf16, rows of 64; columns 0-15 of every row, the others are zero from the
+// start) and adds the loss to *loss_sum and the column sums of dY, the head's
+// bias gradient, to db.  The step's hyper-parameters [lr, w, ..] live in device
+// memory, so that a captured step can be replayed with new values.  (A launch
+// of its own for the loss took 10.7 us at 65,536 rows, the head's GEMM 11.9.)
+struct EpiHeadLoss {
+  static constexpr bool kPrefetch = false;
+  const float *bias, *target, *hp;
+  int64_t B;
+  __nv_bfloat16 *dY;
+  double *loss_sum;
+  float *db;
+  __device__ void operator()(int row, int c0, const float *v) const {  // c0 = 0, whole warps
+    const float w = hp[1];
+    float l = 0.f, g0 = 0.f, g1 = 0.f;
+    uint32_t d[8] = {};
+    if (row < B) {
+      const float lg = v[0] + bias[0], ct = v[1] + bias[1];
+      const float2 yt = reinterpret_cast<const float2 *>(target)[row];
       const float inv = 1.f / (float)B;
-      if (!isnan(y)) {
-        l += softplus(lg) - y * lg;
-        row[0] = __float2bfloat16_rn((sigmoid(lg) - y) * inv);
+      __nv_bfloat162 g = __floats2bfloat162_rn(0.f, 0.f);
+      if (!isnan(yt.x)) {
+        l += softplus(lg) - yt.x * lg;
+        g.x = __float2bfloat16_rn((sigmoid(lg) - yt.x) * inv);
       }
-      if (!isnan(t)) {
-        l += 0.5f * ctg_weight * (ct - t) * (ct - t);
-        row[1] = __float2bfloat16_rn(ctg_weight * (ct - t) * inv);
+      if (!isnan(yt.y)) {
+        l += 0.5f * w * (ct - yt.y) * (ct - yt.y);
+        g.y = __float2bfloat16_rn(w * (ct - yt.y) * inv);
       }
+      d[0] = *reinterpret_cast<const uint32_t *>(&g);
+      g0 = __bfloat162float(g.x);
+      g1 = __bfloat162float(g.y);
     }
-    uint4 *dst = reinterpret_cast<uint4 *>(dY + b * 64);
-#pragma unroll
-    for (int j = 0; j < 8; j++) dst[j] = reinterpret_cast<const uint4 *>(row)[j];
-    g0 = __bfloat162float(row[0]);
-    g1 = __bfloat162float(row[1]);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    l += __shfl_down_sync(0xffffffffu, l, o);
-    g0 += __shfl_down_sync(0xffffffffu, g0, o);
-    g1 += __shfl_down_sync(0xffffffffu, g1, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (l != 0.f) atomicAdd(loss_sum, (double)l);
-    if (db && g0 != 0.f) atomicAdd(db, g0);
-    if (db && g1 != 0.f) atomicAdd(db + 1, g1);
-  }
-}
-
-// dZ = dH * gelu'(Z) (gelu' kept in bf16 by the forward epilogue): the
-// epilogue of dH = dZnext * W.
-struct EpiGeluGrad {
-  const __nv_bfloat16 *dgelu;
-  __nv_bfloat16 *dz;
-  int ld;
-  __device__ void operator()(int row, int c0, const float *v) const {
-    __align__(16) __nv_bfloat16 h[16], d[16];
-    const uint4 *gd = reinterpret_cast<const uint4 *>(dgelu + (int64_t)row * ld + c0);
-    reinterpret_cast<uint4 *>(d)[0] = gd[0];
-    reinterpret_cast<uint4 *>(d)[1] = gd[1];
-#pragma unroll
-    for (int j = 0; j < 16; j++) h[j] = __float2bfloat16_rn(v[j] * __bfloat162float(d[j]));
-    uint4 *dst = reinterpret_cast<uint4 *>(dz + (int64_t)row * ld + c0);
-    dst[0] = reinterpret_cast<const uint4 *>(h)[0];
-    dst[1] = reinterpret_cast<const uint4 *>(h)[1];
+    store32(dY + (int64_t)row * 64, d);
+    for (int o = 16; o > 0; o >>= 1) {
+      l += __shfl_down_sync(0xffffffffu, l, o);
+      g0 += __shfl_down_sync(0xffffffffu, g0, o);
+      g1 += __shfl_down_sync(0xffffffffu, g1, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      if (l != 0.f) atomicAdd(loss_sum, (double)l);
+      if (g0 != 0.f) atomicAdd(db, g0);
+      if (g1 != 0.f) atomicAdd(db + 1, g1);
+    }
   }
 };
 
 // dE[prim[b]] += dX[b, 80:96]: the epilogue of the 16-column product
 // dZ1 * W1[:, 80:96] (the embedding part of the layer-1 input gradient)
 struct EpiEmbGrad {
+  static constexpr bool kPrefetch = false;
   const uint32_t *prim;
   float *demb;
   int64_t B;
@@ -702,49 +689,6 @@ constexpr uint32_t kFwdChunk = kMlpHidden * kFwdK * 2;  // 256 rows x 32 bf16 = 
 // biases of layers 1-3, W4's two rows (FP32), partial outputs [slot][column group][row]
 constexpr uint32_t kFwdConst = (3 + 2) * kMlpHidden * 4, kFwdPart = 2 * 4 * 128 * 8;
 constexpr size_t kFwdSmem = 1024 + 2 * kActBytes + kFwdStages * kFwdChunk + kFwdConst + kFwdPart + 256;
-
-// two FP32 values in one 64-bit register
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-// gelu (gemm_kernels.cuh) of two values, with its roundings
-__device__ __forceinline__ uint64_t gelu2(uint64_t z) {
-  const uint64_t one = pack2(1.f, 1.f);
-  const uint64_t f = fma2(mul2(pack2(kGeluB, kGeluB), z), z, one);
-  float u0, u1;
-  unpack2(mul2(mul2(pack2(kGeluA, kGeluA), z), f), u0, u1);
-  return mul2(mul2(pack2(0.5f, 0.5f), z), add2(one, pack2(tanh_fast(u0), tanh_fast(u1))));
-}
-// two values rounded to bf16 (the first in the low half)
-__device__ __forceinline__ uint32_t to_bf16x2(uint64_t v) {
-  float x, y;
-  unpack2(v, x, y);
-  const __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
-  return *reinterpret_cast<const uint32_t *>(&p);
-}
-__device__ __forceinline__ uint64_t from_bf16x2(uint32_t w) {
-  return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-}
 
 static __global__ void __launch_bounds__(kFwdThreads, 1)
     mlp_forward_pair(const __grid_constant__ CUtensorMap tw1, const __grid_constant__ CUtensorMap tw2,
