@@ -253,11 +253,11 @@ static void launch_ball(const dpg_ctx *c, const PrimView &pv, const NodeView &nv
       const float h1 = half(KIND == DPG_ROBOT_CAR1 ? rp.w[2] : rp.w[3], KIND == DPG_ROBOT_CAR1);
       cudaMemsetAsync(mask, 0, sizeof(uint32_t) * (size_t)P * Wpad, st);
       if (P <= kGridSmemP) {
-        nn_grid<KIND, true><<<(unsigned)B, kNNThreads, sizeof(uint32_t) * P, st>>>(
+        nn_grid<KIND, true><<<(unsigned)B, kGridThreads, sizeof(uint32_t) * P, st>>>(
             rp, pv, nv, c->kg, w32, (float)radius, radius, (float)ball_band, h0, h1, Wpad, mask, cnt, ctr);
       } else {
         cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (size_t)B * P, st);
-        nn_grid<KIND, false><<<(unsigned)B, kNNThreads, 0, st>>>(rp, pv, nv, c->kg, w32, (float)radius, radius,
+        nn_grid<KIND, false><<<(unsigned)B, kGridThreads, 0, st>>>(rp, pv, nv, c->kg, w32, (float)radius, radius,
                                                                  (float)ball_band, h0, h1, Wpad, mask, cnt, ctr);
       }
       done = true;

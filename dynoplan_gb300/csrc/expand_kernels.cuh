@@ -208,6 +208,28 @@ __global__ void __launch_bounds__(256) node_tiles(const double *x64, int64_t N, 
   for (int c = threadIdx.x; c < kOrderCells; c += 256) out[c] = hist[c];
 }
 
+// sum of v over the threads before this one (a block of 1024); total: over all
+template <class T>
+__device__ __forceinline__ T block_prefix(T v, T *ws, T &total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto incl = [&](T x) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const T y = __shfl_up_sync(kFull, x, o);
+      if (lane >= o) x += y;
+    }
+    return x;
+  };
+  const T mine = incl(v);
+  if (lane == 31) ws[warp] = mine;
+  __syncthreads();
+  const T sums = incl(ws[lane]);
+  total = __shfl_sync(kFull, sums, 31);
+  const T before = __shfl_sync(kFull, sums, max(warp - 1, 0));
+  __syncthreads();  // ws may be written again
+  return (warp ? before : T(0)) + mine - v;
+}
+
 // single block: start = exclusive prefix of cnt over n cells
 static __global__ void __launch_bounds__(1024) cell_scan(int n, const uint32_t *cnt, uint32_t *start) {
   __shared__ uint32_t part[1024];
@@ -363,7 +385,7 @@ struct KeyGrid {
 
 __host__ __device__ __forceinline__ int kg_clamp(int c, int n) { return c < 0 ? 0 : (c >= n ? n - 1 : c); }
 
-// Ball membership through the key grid: thread per node, each node tests the
+// Ball membership through the key grid: kGridLanes lanes per node, each node tests the
 // primitives of the cells within h0 / h1 (the radius plus the band over the
 // component's weight, widened; negative = the whole range) of its key, with
 // the same FP32 test and FP64 band decision as nn_mask, so the bitmask and
@@ -371,8 +393,13 @@ __host__ __device__ __forceinline__ int kg_clamp(int c, int n) { return c < 0 ? 
 // their bit with atomicOr.  cnt[b][p] is counted in shared memory when
 // SCNT (P <= kGridSmemP), else by global atomics into a zeroed cnt.
 constexpr int kGridSmemP = 12288;
+// Bound by the latency of the table loads and the atomics: with a thread a node
+// (four loads in flight) a batch of 10,000-30,000 nodes left the SMs a few warps
+// each; ball stage of 10,000 unicycle nodes x 1,000 primitives 117 us with one
+// lane, 105 with two, 97 with four; 100,000 cars x 5,000: 277, 285, 260.
+constexpr int kGridLanes = 4, kGridThreads = kNNThreads * kGridLanes;
 template <int KIND, bool SCNT>
-__global__ void __launch_bounds__(kNNThreads) nn_grid(RobotParams rp, PrimView pv, NodeView nv, KeyGrid kg,
+__global__ void __launch_bounds__(kGridThreads) nn_grid(RobotParams rp, PrimView pv, NodeView nv, KeyGrid kg,
                                                       float4 w32, float radius, double radius64, float band,
                                                       float h0, float h1, int64_t Wpad, uint32_t *mask, uint32_t *cnt,
                                                       DevCounters *ctr) {
@@ -385,9 +412,9 @@ __global__ void __launch_bounds__(kNNThreads) nn_grid(RobotParams rp, PrimView p
     for (int t = threadIdx.x; t < pv.P; t += blockDim.x) scnt[t] = 0;
     __syncthreads();
   }
-  const int lane = threadIdx.x & 31;
-  const int64_t w = (int64_t)blockIdx.x * (kNNThreads / 32) + (threadIdx.x >> 5);
-  const int64_t n = w * 32 + lane;
+  const int64_t n = (int64_t)blockIdx.x * kNNThreads + threadIdx.x / kGridLanes;
+  const int64_t w = n >> 5;
+  const uint32_t sub = threadIdx.x % kGridLanes;
   unsigned long long rechecks = 0;
   if (n < nv.N) {
     float nk[2];
@@ -411,33 +438,27 @@ __global__ void __launch_bounds__(kNNThreads) nn_grid(RobotParams rp, PrimView p
       }
     }
     const double *xn = nv.x64 + n * R::NX;
-    const uint32_t bit = 1u << lane;
+    const uint32_t bit = 1u << (n & 31);
     for (int a = a0; a <= a1; a++) {
       const int ca = ((a % kg.n0) + kg.n0) % kg.n0;
       for (int b = b0; b <= b1;) {  // runs of cells contiguous in the row
         const int cb = kPer1 ? ((b % kg.n1) + kg.n1) % kg.n1 : b;
         const int last = kPer1 ? min(b1, b + (kg.n1 - 1 - cb)) : b1;
         const uint32_t s = kg.start[ca * kg.n1 + cb], e = kg.start[ca * kg.n1 + cb + (last - b) + 1];
-        for (uint32_t i = s; i < e; i += 4) {  // four table loads in flight
-          float4 t[4];
-#pragma unroll
-          for (int u = 0; u < 4; u++) t[u] = i + u < e ? kg.tab[i + u] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            if (i + u >= e) break;
-            const float sk[2] = {t[u].x, t[u].y};
-            const float d = key_dist32<KIND>(w32, nk, sk, 1, t[u].z);
-            bool in = d <= radius;
-            const int p = __float_as_int(t[u].w);
-            if (fabsf(d - radius) <= band) {  // decide in FP64
-              in = key_dist64<KIND>(rp, xn, pv.st64 + pv.krow[p] * R::NX) <= radius64;
-              rechecks++;
-            }
-            if (in) {
-              atomicOr(&mask[(int64_t)p * Wpad + w], bit);
-              if (SCNT) atomicAdd(&scnt[p], 1u);
-              else atomicAdd(&cnt[(int64_t)blockIdx.x * pv.P + p], 1u);
-            }
+        for (uint32_t i = s + sub; i < e; i += kGridLanes) {
+          const float4 t = kg.tab[i];
+          const float sk[2] = {t.x, t.y};
+          const float d = key_dist32<KIND>(w32, nk, sk, 1, t.z);
+          bool in = d <= radius;
+          const int p = __float_as_int(t.w);
+          if (fabsf(d - radius) <= band) {  // decide in FP64
+            in = key_dist64<KIND>(rp, xn, pv.st64 + pv.krow[p] * R::NX) <= radius64;
+            rechecks++;
+          }
+          if (in) {
+            atomicOr(&mask[(int64_t)p * Wpad + w], bit);
+            if (SCNT) atomicAdd(&scnt[p], 1u);
+            else atomicAdd(&cnt[(int64_t)blockIdx.x * pv.P + p], 1u);
           }
         }
         b = last + 1;
@@ -449,7 +470,7 @@ __global__ void __launch_bounds__(kNNThreads) nn_grid(RobotParams rp, PrimView p
     for (int t = threadIdx.x; t < pv.P; t += blockDim.x) cnt[(int64_t)blockIdx.x * pv.P + t] = scnt[t];
   }
   for (int o = 16; o > 0; o >>= 1) rechecks += __shfl_down_sync(kFull, rechecks, o);
-  if (lane == 0 && rechecks) atomicAdd(&ctr->n_ball_recheck, rechecks);
+  if ((threadIdx.x & 31) == 0 && rechecks) atomicAdd(&ctr->n_ball_recheck, rechecks);
 }
 
 // per primitive: cnt[b][p] -> exclusive prefix over b; tot[p] = total.
@@ -479,50 +500,54 @@ static __global__ void __launch_bounds__(256) nn_prefix(int P, int B, uint32_t *
 }
 
 // Single block: bases of each primitive's pair segment and of its work
-// items, in the order of decreasing primitive length.
+// items, in the order of decreasing primitive length.  kScanRun positions a
+// thread, their counts in flight together, one prefix over the block for 8,192
+// positions (14.3 us for 5,000 primitives with dependent loads and a prefix
+// through shared memory).
+constexpr int kScanRun = 8;
 static __global__ void __launch_bounds__(1024) scan_totals(int P, const int32_t *order, const uint32_t *tot,
                                                     unsigned long long *pbase,
                                                     unsigned long long *ord_pbase,
                                                     unsigned long long *ord_ibase, int64_t cap,
                                                     DevCounters *ctr) {
-  __shared__ unsigned long long sp[1024], si[1024];
-  const int t = threadIdx.x, T = blockDim.x;
-  const int per = (P + T - 1) / T;
-  const int b = t * per, e = min(P, b + per);
-  unsigned long long a = 0, c = 0;
-  for (int i = b; i < e; i++) {
-    const uint32_t v = tot[order[i]];
-    a += v;
-    c += (v + 31) / 32;
+  __shared__ unsigned long long wp[32], wi[32];
+  unsigned long long np = 0, ni = 0;  // pairs and items of the positions done
+  for (int64_t base = 0; base < P; base += 1024 * kScanRun) {
+    const int64_t i0 = base + (int64_t)threadIdx.x * kScanRun;
+    int p[kScanRun];
+    uint32_t v[kScanRun];
+    unsigned long long a = 0, b = 0, ta, tb;
+#pragma unroll
+    for (int k = 0; k < kScanRun; k++) p[k] = i0 + k < P ? order[i0 + k] : -1;
+#pragma unroll
+    for (int k = 0; k < kScanRun; k++) v[k] = p[k] >= 0 ? tot[p[k]] : 0u;
+#pragma unroll
+    for (int k = 0; k < kScanRun; k++) {
+      a += v[k];
+      b += ((unsigned long long)v[k] + 31) / 32;
+    }
+    a = np + block_prefix(a, wp, ta);
+    b = ni + block_prefix(b, wi, tb);
+#pragma unroll
+    for (int k = 0; k < kScanRun; k++) {
+      if (p[k] >= 0) {
+        ord_pbase[i0 + k] = a;
+        ord_ibase[i0 + k] = b;
+        pbase[p[k]] = a;
+      }
+      a += v[k];
+      b += ((unsigned long long)v[k] + 31) / 32;
+    }
+    np += ta;
+    ni += tb;
   }
-  sp[t] = a;
-  si[t] = c;
-  __syncthreads();
-  for (int off = 1; off < T; off <<= 1) {  // inclusive Hillis-Steele
-    unsigned long long va = 0, vc = 0;
-    if (t >= off) { va = sp[t - off]; vc = si[t - off]; }
-    __syncthreads();
-    sp[t] += va;
-    si[t] += vc;
-    __syncthreads();
-  }
-  unsigned long long ra = sp[t] - a, rc = si[t] - c;
-  for (int i = b; i < e; i++) {
-    const int p = order[i];
-    const uint32_t v = tot[p];
-    ord_pbase[i] = ra;
-    ord_ibase[i] = rc;
-    pbase[p] = ra;
-    ra += v;
-    rc += (v + 31) / 32;
-  }
-  if (t == T - 1) {
-    ord_pbase[P] = sp[T - 1];
-    ord_ibase[P] = si[T - 1];
-    ctr->n_pairs = sp[T - 1];
-    const bool overflow = (int64_t)sp[T - 1] > cap;
+  if (threadIdx.x == 0) {
+    ord_pbase[P] = np;
+    ord_ibase[P] = ni;
+    ctr->n_pairs = np;
+    const bool overflow = (int64_t)np > cap;
     ctr->n_overflow = overflow ? 1 : 0;
-    ctr->n_items = overflow ? 0 : si[T - 1];
+    ctr->n_items = overflow ? 0 : ni;
     for (int i = 0; i < kMaxSub; i++) ctr->next_sub[i] = 0;
   }
 }
