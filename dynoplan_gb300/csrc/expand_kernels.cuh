@@ -29,6 +29,7 @@
 #include <cfloat>
 #include <cstdint>
 
+#include "f32x2.cuh"
 #include "robots.cuh"
 
 namespace dpg {
@@ -292,13 +293,55 @@ __device__ __forceinline__ float key_dist32(const float4 w, const float *nk,
   } else if constexpr (KIND == DPG_ROBOT_QUAD2D) {
     return kc + w.y * so2w(nk[0], sk[0]) + w.w * fabsf(nk[1] - sk[stride]);
   } else {
-    float dq = fabsf(nk[0] * sk[0] + nk[1] * sk[stride] + nk[2] * sk[2 * stride] +
-                     nk[3] * sk[3 * stride]);
+    // (the roundings are pinned: quad_dist2 has the same)
+    float dq = fabsf(fmaf(nk[3], sk[3 * stride], fmaf(nk[2], sk[2 * stride], fmaf(nk[0], sk[0], nk[1] * sk[stride]))));
     dq = fminf(dq, 1.0f);
     const float a = nk[4] - sk[4 * stride], b = nk[5] - sk[5 * stride],
                 c = nk[6] - sk[6 * stride];
     return kc + w.y * acosf(dq) + w.w * sqrtf(a * a + b * b + c * c);
   }
+}
+
+// The quadrotor's distance to two primitives at once, approximately: acos by
+// Abramowitz & Stegun 4.4.45 (error below 7e-5) and approximate square roots.
+// key[i], kc: the primitives' key components and constants in pairs; nk2: the
+// node's, twice (the velocity negated).  Given weights that are not negative it
+// is within quad_margin of key_dist32 wherever that matters: near the radius no
+// term is above it, and further out the rounding grows slower than the distance.
+// Pairs within the margin, about one in a hundred, take key_dist32.  Bound by
+// this arithmetic: for 50,000 nodes x 5,000 primitives the ball stage took
+// 1.13 ms with acosf and exact roots for every pair, 0.46 ms with this.
+__device__ __forceinline__ float sqrt_fast(float x) {
+  float y;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ uint64_t quad_dist2(uint64_t wy, uint64_t ww, const uint64_t *nk2, const uint64_t *key,
+                                               uint64_t kc) {
+  const uint64_t dq = fma2(nk2[3], key[3], fma2(nk2[2], key[2], fma2(nk2[0], key[0], mul2(nk2[1], key[1]))));
+  const uint64_t x = dq & 0x7fffffff7fffffffull;
+  float t0, t1, s0, s1;
+  unpack2(fma2(x, pack2(-1.f, -1.f), pack2(1.f, 1.f)), t0, t1);
+  uint64_t p = fma2(x, pack2(-0.0187293f, -0.0187293f), pack2(0.0742610f, 0.0742610f));
+  p = fma2(x, p, pack2(-0.2121144f, -0.2121144f));
+  p = fma2(x, p, pack2(1.5707288f, 1.5707288f));
+  const uint64_t ac = mul2(pack2(sqrt_fast(fmaxf(t0, 0.f)), sqrt_fast(fmaxf(t1, 0.f))), p);
+  const uint64_t a = add2(nk2[4], key[4]), b = add2(nk2[5], key[5]), c = add2(nk2[6], key[6]);
+  unpack2(fma2(c, c, fma2(b, b, mul2(a, a))), s0, s1);
+  return fma2(ww, pack2(sqrt_fast(s0), sqrt_fast(s1)), fma2(wy, ac, kc));
+}
+// bit b of lane l's word -> bit l of lane b's
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
+#pragma unroll
+  for (int j = 16; j > 0; j >>= 1) {
+    const uint32_t m = j == 16 ? 0x0000ffffu : j == 8 ? 0x00ff00ffu : j == 4 ? 0x0f0f0f0fu : j == 2 ? 0x33333333u : 0x55555555u;
+    const uint32_t y = __shfl_xor_sync(kFull, x, j);
+    x = lane & j ? (x & ~m) | ((y >> j) & m) : (x & m) | ((y & m) << j);
+  }
+  return x;
+}
+__device__ __forceinline__ float quad_margin(const float4 w, float radius, float band) {
+  return w.y >= 0.f && w.w >= 0.f ? band + 1e-4f * w.y + 1e-5f * fabsf(radius) : INFINITY;
 }
 
 // Ball membership of 256 nodes (blockIdx.x) against the primitives of
@@ -313,8 +356,8 @@ __global__ void __launch_bounds__(kNNThreads) nn_mask(RobotParams rp, PrimView p
                                                       int64_t Wpad, int tiles_per_y, uint32_t *mask, uint32_t *cnt,
                                                       DevCounters *ctr) {
   using R = Robot<KIND>;
-  __shared__ float sk[R::KEYD * kNNTile];
-  __shared__ float skc[kNNTile];
+  __shared__ __align__(16) float sk[R::KEYD * kNNTile];
+  __shared__ __align__(16) float skc[kNNTile];
   __shared__ uint32_t scnt[kNNThreads / 32][kNNTile];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t w = (int64_t)blockIdx.x * (kNNThreads / 32) + warp;  // bitmask word
@@ -324,6 +367,15 @@ __global__ void __launch_bounds__(kNNThreads) nn_mask(RobotParams rp, PrimView p
 #pragma unroll
   for (int i = 0; i < R::KEYD; i++) nk[i] = live ? nv.key32[i * nv.N + n] : 0.f;
   unsigned long long rechecks = 0;
+  [[maybe_unused]] uint64_t nk2[7], wy2 = 0, ww2 = 0;
+  [[maybe_unused]] float margin = 0.f;
+  if constexpr (KIND == DPG_ROBOT_QUAD3D) {
+#pragma unroll
+    for (int i = 0; i < 7; i++) nk2[i] = i < 4 ? pack2(nk[i], nk[i]) : pack2(-nk[i], -nk[i]);
+    wy2 = pack2(w32.y, w32.y);
+    ww2 = pack2(w32.w, w32.w);
+    margin = quad_margin(w32, radius, band);
+  }
 
   const int p_begin = blockIdx.y * tiles_per_y * kNNTile;
   const int p_end = min(pv.P, p_begin + tiles_per_y * kNNTile);
@@ -335,25 +387,59 @@ __global__ void __launch_bounds__(kNNThreads) nn_mask(RobotParams rp, PrimView p
       for (int i = 0; i < R::KEYD; i++) sk[i * kNNTile + t] = pv.key32[i * pv.P + p0 + t];
       skc[t] = pv.kconst32[p0 + t];
     }
+    if (KIND == DPG_ROBOT_QUAD3D)  // past the last primitive: outside
+      for (int t = tp + threadIdx.x; t < (tp + 3) / 4 * 4; t += blockDim.x) {
+#pragma unroll
+        for (int i = 0; i < R::KEYD; i++) sk[i * kNNTile + t] = 0.f;
+        skc[t] = INFINITY;
+      }
     __syncthreads();
+    // the decision on the tile's primitive j: FP32, in FP64 near the radius
+    auto exact = [&](int j) {
+      const float d = key_dist32<KIND>(w32, nk, &sk[j], kNNTile, skc[j]);
+      if (!(fabsf(d - radius) <= band)) return d <= radius;
+      rechecks++;
+      return key_dist64<KIND>(rp, nv.x64 + n * R::NX, pv.st64 + pv.krow[p0 + j] * R::NX) <= radius64;
+    };
     for (int j0 = 0; j0 < tp; j0 += 32) {
       uint32_t mine = 0;
       const int jn = min(32, tp - j0);
-      for (int jj = 0; jj < jn; jj++) {
-        const int j = j0 + jj;
-        bool in = false;
-        if (live) {
-          const float d = key_dist32<KIND>(w32, nk, &sk[j], kNNTile, skc[j]);
-          in = d <= radius;
-          if (fabsf(d - radius) <= band) {  // decide in FP64
-            const int p = p0 + j;
-            const double d64 = key_dist64<KIND>(rp, nv.x64 + n * R::NX, pv.st64 + pv.krow[p] * R::NX);
-            in = d64 <= radius64;
-            rechecks++;
+      if constexpr (KIND == DPG_ROBOT_QUAD3D) {
+        // bit j: this node against primitive j0 + j, as far as quad_dist2 tells
+        uint32_t in = 0, unsure = 0;
+#pragma unroll
+        for (int jj = 0; jj < 32; jj += 4) {
+          if (jj >= jn) break;
+          const int j = j0 + jj;
+          ulonglong2 k4[7];
+#pragma unroll
+          for (int i = 0; i < 7; i++) k4[i] = *reinterpret_cast<const ulonglong2 *>(&sk[i * kNNTile + j]);
+          const ulonglong2 c4 = *reinterpret_cast<const ulonglong2 *>(&skc[j]);
+          const uint64_t ka[7] = {k4[0].x, k4[1].x, k4[2].x, k4[3].x, k4[4].x, k4[5].x, k4[6].x};
+          const uint64_t kb[7] = {k4[0].y, k4[1].y, k4[2].y, k4[3].y, k4[4].y, k4[5].y, k4[6].y};
+          float d[4];
+          unpack2(quad_dist2(wy2, ww2, nk2, ka, c4.x), d[0], d[1]);
+          unpack2(quad_dist2(wy2, ww2, nk2, kb, c4.y), d[2], d[3]);
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            if (d[u] <= radius) in |= 1u << (jj + u);
+            if (!(fabsf(d[u] - radius) > margin)) unsure |= 1u << (jj + u);
           }
         }
-        const uint32_t word = __ballot_sync(kFull, in);
-        if (lane == jj) mine = word;
+        if (jn < 32) unsure &= (1u << jn) - 1u;
+        if (!live) in = unsure = 0;
+        in &= ~unsure;
+        for (; unsure; unsure &= unsure - 1) {
+          const int j = __ffs(unsure) - 1;
+          if (exact(j0 + j)) in |= 1u << j;
+        }
+        __syncwarp();
+        mine = transpose32(in, lane);
+      } else {
+        for (int jj = 0; jj < jn; jj++) {
+          const uint32_t word = __ballot_sync(kFull, live && exact(j0 + jj));
+          if (lane == jj) mine = word;
+        }
       }
       const int p = p0 + j0 + lane;
       if (p < pv.P && w * 32 < nv.N) mask[(int64_t)p * Wpad + w] = mine;

@@ -17,6 +17,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include "f32x2.cuh"
 #include "umma.cuh"
 
 namespace dpg {
@@ -336,31 +337,6 @@ __device__ __forceinline__ float gelu_grad(float z) {
   const float t = tanh_fast(kGeluA * z * fmaf(kGeluB * z, z, 1.0f));
   const float du = kGeluA * fmaf(3.0f * kGeluB * z, z, 1.0f);
   return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * du;
-}
-
-// two FP32 values in one 64-bit register
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
 }
 
 // gelu and gelu_grad of two values, with the roundings of the forms above
