@@ -470,6 +470,80 @@ template <class T> struct DVec {  // growable device array
   }
 };
 
+// growable page-locked array (contents lost when it grows), mapped for kernels
+template <class T> struct HVec {
+  T *p = nullptr, *dev = nullptr;
+  size_t cap = 0;
+  ~HVec() { drop(); }
+  void drop() {
+    if (!p) return;
+    cudaDeviceSynchronize();  // copies from or to it are done
+    cudaFreeHost(p);
+    p = nullptr;
+    cap = 0;
+  }
+  bool reserve(size_t n) {
+    if (n <= cap) return true;
+    const size_t nc = std::max<size_t>(n, cap * 2 + 1024);
+    drop();
+    if (cudaHostAlloc(&p, sizeof(T) * nc, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(&dev, p, 0) != cudaSuccess)
+      return false;
+    cap = nc;
+    return true;
+  }
+};
+
+// A round's query answers in one page-locked buffer: the lists' lengths, then
+// per query offsets and counts, then the lists.  pack_answers writes them
+// there, so that the host waits once instead of for nine copies.
+struct Answers {
+  unsigned long long *fill;  // [2]
+  int64_t *off_tab, *off_self;
+  double *lbt_tab, *lbt_self;
+  int *cnt_tab, *cnt_all, *cnt_self, *ids_tab, *ids_self;
+};
+static size_t answers_at(unsigned char *b, int Q, int64_t cap_tab, int64_t cap_self, Answers &a) {
+  size_t at = 0;
+  auto take = [&](auto *&q, size_t n) {
+    q = reinterpret_cast<std::remove_reference_t<decltype(q)>>(b + at);
+    at += sizeof(*q) * n;
+  };
+  take(a.fill, 2);  // (the 8-byte types first)
+  take(a.off_tab, Q);
+  take(a.off_self, Q);
+  take(a.lbt_tab, cap_tab);
+  take(a.lbt_self, cap_self);
+  take(a.cnt_tab, Q);
+  take(a.cnt_all, Q);
+  take(a.cnt_self, Q);
+  take(a.ids_tab, cap_tab);
+  take(a.ids_self, cap_self);
+  return at;
+}
+static __global__ void pack_answers(Answers in, Answers out, int Q, unsigned long long cap_tab,
+                                    unsigned long long cap_self) {
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  const unsigned long long nt = in.fill[0], ns = in.fill[1];
+  if (i0 < 2) out.fill[i0] = in.fill[i0];
+  for (int64_t i = i0; i < Q; i += step) {
+    out.off_tab[i] = in.off_tab[i];
+    out.off_self[i] = in.off_self[i];
+    out.cnt_tab[i] = in.cnt_tab[i];
+    out.cnt_all[i] = in.cnt_all[i];
+    out.cnt_self[i] = in.cnt_self[i];
+  }
+  if (nt > cap_tab || ns > cap_self) return;  // the host grows the lists and repeats the queries
+  for (int64_t i = i0; i < (int64_t)nt; i += step) {
+    out.ids_tab[i] = in.ids_tab[i];
+    out.lbt_tab[i] = in.lbt_tab[i];
+  }
+  for (int64_t i = i0; i < (int64_t)ns; i += step) {
+    out.ids_self[i] = in.ids_self[i];
+    out.lbt_self[i] = in.lbt_self[i];
+  }
+}
+
 }  // namespace
 
 
@@ -532,8 +606,8 @@ extern "C" int dpg_search(dpg_ctx *c, const dpg_search_opts *o, const double *st
     if (!cell.reserve(std::max(n, 1)) || !sorted.reserve(std::max(n, 1)) ||
         !rows_out.reserve((size_t)std::max(n, 1) * nx))
       return false;
-    cudaMemset(cnt.p, 0, sizeof(int) * n_cells);
-    cudaMemset(fill.p, 0, sizeof(int) * n_cells);
+    cudaMemsetAsync(cnt.p, 0, sizeof(int) * n_cells, 0);
+    cudaMemsetAsync(fill.p, 0, sizeof(int) * n_cells, 0);
     with_kind_s(r.kind, [&](auto Kd) {
       constexpr int KIND = decltype(Kd)::value;
       if (n > 0) grid_count<KIND><<<(n + 255) / 256, 256>>>(grid, rows, n, cell.p, cnt.p);
@@ -547,17 +621,26 @@ extern "C" int dpg_search(dpg_ctx *c, const dpg_search_opts *o, const double *st
   // the table's g values as uploaded with each node: never below a node's
   // current g (g only decreases), so the rewire filter against them is exact
   DVec<float> gsnap;
+  HVec<double> up64;
+  HVec<float> up32;
   size_t uploaded = 0;
   auto sync_table = [&]() -> bool {
     const size_t n = nodes.size();
     if (!t64.reserve(n * nx) || !t32.reserve(n * nx) || !gsnap.reserve(n)) return false;
     if (n > uploaded) {
-      std::vector<float> f(xs.begin() + uploaded * nx, xs.end()), gs(n - uploaded);
-      for (size_t i = uploaded; i < n; i++) gs[i - uploaded] = nodes[i].g;
-      cudaMemcpy(t64.p + uploaded * nx, xs.data() + uploaded * nx, sizeof(double) * (n - uploaded) * nx,
-                 cudaMemcpyHostToDevice);
-      cudaMemcpy(t32.p + uploaded * nx, f.data(), sizeof(float) * f.size(), cudaMemcpyHostToDevice);
-      cudaMemcpy(gsnap.p + uploaded, gs.data(), sizeof(float) * gs.size(), cudaMemcpyHostToDevice);
+      // (page-locked, so that the copies are only queued; the round's wait for
+      // its answers comes before the next use)
+      const size_t m = n - uploaded;
+      if (!up64.reserve(m * nx) || !up32.reserve(m * (nx + 1))) return false;
+      float *gs = up32.p + m * nx;
+      for (size_t i = 0; i < m * nx; i++) {
+        up64.p[i] = xs[uploaded * nx + i];
+        up32.p[i] = (float)up64.p[i];
+      }
+      for (size_t i = 0; i < m; i++) gs[i] = nodes[uploaded + i].g;
+      cudaMemcpyAsync(t64.p + uploaded * nx, up64.p, sizeof(double) * m * nx, cudaMemcpyHostToDevice, 0);
+      cudaMemcpyAsync(t32.p + uploaded * nx, up32.p, sizeof(float) * m * nx, cudaMemcpyHostToDevice, 0);
+      cudaMemcpyAsync(gsnap.p + uploaded, gs, sizeof(float) * m, cudaMemcpyHostToDevice, 0);
       uploaded = n;
       return sort_by_cell(t32.p, (int)n, tab_cnt, tab_start, tab_fill, tab_cell, tab_sorted, tab_rows);
     }
@@ -585,8 +668,9 @@ extern "C" int dpg_search(dpg_ctx *c, const dpg_search_opts *o, const double *st
   DVec<double> q64, b64, prep, goal_d, gq, lbt_tab, lbt_self;
   DVec<float> gpop_d;
   DVec<int> cand, cnt_all;
-  std::vector<int> cnp;
-  std::vector<double> prep_h;
+  HVec<int> cnp;
+  HVec<double> prep_h;
+  HVec<unsigned char> answers;
   if (!goal_d.reserve(nx)) return DPG_ERR_OOM;
   cudaMemcpy(goal_d.p, goal, sizeof(double) * nx, cudaMemcpyHostToDevice);
   DVec<float> q32;
@@ -599,6 +683,7 @@ extern "C" int dpg_search(dpg_ctx *c, const dpg_search_opts *o, const double *st
   std::vector<uint32_t> h_node, h_prim;
   std::vector<uint8_t> h_verdict;
   std::vector<int16_t> h_fi;
+  std::vector<uint64_t> bits;
   int solution = -1;
   int status = DPG_SEARCH_EMPTY_QUEUE;
   const float4 w32 = make_float4((float)r.w[0], (float)r.w[1], (float)r.w[2], (float)r.w[3]);
@@ -655,12 +740,30 @@ extern "C" int dpg_search(dpg_ctx *c, const dpg_search_opts *o, const double *st
     res->expand_ms += elapsed_ms() - te0;
     res->checked_pairs += eo.n_pairs;
 
-    // valid motions per batch node, in expand_lazy's order
+    // valid motions per batch node, in expand_lazy's order: a bit per motion,
+    // eight verdicts looked at together (a branch per pair and a sort per node
+    // took a quarter of a search with 8 million pairs)
+    static_assert(DPG_VALID == 0, "zero bytes are searched for");
+    const size_t words = ((size_t)P + 63) / 64;
+    bits.assign((size_t)B * words, 0);
+    auto mark = [&](int64_t i) {
+      bits[h_node[i] * words + (h_prim[i] >> 6)] |= (uint64_t)1 << (h_prim[i] & 63);
+    };
+    int64_t i8 = 0;
+    for (; i8 + 8 <= eo.n_pairs; i8 += 8) {
+      uint64_t v;
+      std::memcpy(&v, &h_verdict[i8], 8);
+      const uint64_t low = 0x7f7f7f7f7f7f7f7full;
+      for (uint64_t z = ~(((v & low) + low) | v | low); z; z &= z - 1)  // 0x80 in each zero byte
+        mark(i8 + (__builtin_ctzll(z) >> 3));
+    }
+    for (; i8 < eo.n_pairs; i8++)
+      if (h_verdict[i8] == DPG_VALID) mark(i8);
     std::vector<std::vector<int>> per_node(B);
-    for (int64_t i = 0; i < eo.n_pairs; i++)
-      if (h_verdict[i] == DPG_VALID) per_node[h_node[i]].push_back((int)h_prim[i]);
     for (int b = 0; b < B; b++) {
-      std::sort(per_node[b].begin(), per_node[b].end());
+      for (size_t w = 0; w < words; w++)
+        for (uint64_t z = bits[b * words + w]; z; z &= z - 1)
+          per_node[b].push_back((int)(64 * w) + __builtin_ctzll(z));
       if (o->shuffle) std::shuffle(per_node[b].begin(), per_node[b].end(), rng);
     }
     // the batch's states and g when popped on the device (successor
@@ -716,10 +819,10 @@ extern "C" int dpg_search(dpg_ctx *c, const dpg_search_opts *o, const double *st
       if (!q64.reserve((size_t)Q * nx) || !q32.reserve((size_t)Q * nx) || !cand.reserve(2 * (size_t)Q) ||
           !prep.reserve((size_t)Q * prow) || !gq.reserve(Q))
         return DPG_ERR_OOM;
-      cnp.resize(2 * (size_t)Q);
-      std::copy(c_node.begin(), c_node.end(), cnp.begin());
-      std::copy(c_prim.begin(), c_prim.end(), cnp.begin() + Q);
-      cudaMemcpy(cand.p, cnp.data(), sizeof(int) * cnp.size(), cudaMemcpyHostToDevice);
+      if (!cnp.reserve(2 * (size_t)Q) || !prep_h.reserve((size_t)Q * prow)) return DPG_ERR_OOM;
+      std::copy(c_node.begin(), c_node.end(), cnp.p);
+      std::copy(c_prim.begin(), c_prim.end(), cnp.p + Q);
+      cudaMemcpyAsync(cand.p, cnp.p, sizeof(int) * 2 * Q, cudaMemcpyHostToDevice, 0);
       with_kind_s(r.kind, [&](auto Kd) {
         constexpr int KIND = decltype(Kd)::value;
         prepare_successors<KIND><<<(Q + 127) / 128, 128>>>(
@@ -727,8 +830,8 @@ extern "C" int dpg_search(dpg_ctx *c, const dpg_search_opts *o, const double *st
             static_cast<const int32_t *>(c->len.p), b64.p, gpop_d.p, cand.p, cand.p + Q, Q, goal_d.p, goal_tol,
             o->cost_delta_factor, prep.p, gq.p, q64.p, q32.p);
       });
-      prep_h.resize((size_t)Q * prow);
-      if (cudaMemcpy(prep_h.data(), prep.p, sizeof(double) * prep_h.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
+      if (cudaMemcpyAsync(prep_h.p, prep.p, sizeof(double) * Q * prow, cudaMemcpyDeviceToHost, 0) != cudaSuccess ||
+          cudaStreamSynchronize(0) != cudaSuccess)
         return DPG_ERR_CUDA;
       c_x.resize((size_t)Q * nx);
       c_chosen.resize(Q);
@@ -736,7 +839,7 @@ extern "C" int dpg_search(dpg_ctx *c, const dpg_search_opts *o, const double *st
       c_lbtpar.resize(Q);
       c_hlbt.resize(Q);
       for (int q = 0; q < Q; q++) {
-        const double *row = &prep_h[(size_t)q * prow];
+        const double *row = prep_h.p + (size_t)q * prow;
         std::memcpy(&c_x[(size_t)q * nx], row, sizeof(double) * nx);
         c_chosen[q] = (int)row[nx];
         c_cost[q] = row[nx + 1];
@@ -760,12 +863,14 @@ extern "C" int dpg_search(dpg_ctx *c, const dpg_search_opts *o, const double *st
       // filter (all of them are counted for the novelty test) and every
       // earlier successor of the round within the radius, each with its time
       // lower bound, in packed lists (a run per query, offsets from the device)
-      std::vector<int> ct(Q), ca(Q), cs(Q), it, is;
-      std::vector<double> lt, ls;
-      std::vector<int64_t> ot(Q), os(Q);
-      unsigned long long nts[2] = {0, 0};
+      Answers ans{};
       if (!off_tab.reserve(Q) || !off_self.reserve(Q) || !list_fill.reserve(2)) return DPG_ERR_OOM;
       auto query = [&]() {  // a block per query
+        const size_t cap_tab = std::min(ids_tab.cap, lbt_tab.cap), cap_self = std::min(ids_self.cap, lbt_self.cap);
+        if (!answers.reserve(answers_at(nullptr, Q, cap_tab, cap_self, ans))) return false;
+        Answers ans_dev{};
+        answers_at(answers.p, Q, cap_tab, cap_self, ans);
+        answers_at(answers.dev, Q, cap_tab, cap_self, ans_dev);
         cudaMemsetAsync(list_fill.p, 0, sizeof(unsigned long long) * 2);
         with_kind_s(r.kind, [&](auto Kd) {
           constexpr int KIND = decltype(Kd)::value;
@@ -781,36 +886,24 @@ extern "C" int dpg_search(dpg_ctx *c, const dpg_search_opts *o, const double *st
                                                  (int64_t)std::min(ids_self.cap, lbt_self.cap), ids_self.p,
                                                  lbt_self.p);
         });
-        return cudaMemcpy(nts, list_fill.p, sizeof(nts), cudaMemcpyDeviceToHost) == cudaSuccess;
+        const Answers in{list_fill.p, off_tab.p, off_self.p, lbt_tab.p, lbt_self.p,
+                         cnt_tab.p,   cnt_all.p, cnt_self.p, ids_tab.p, ids_self.p};
+        pack_answers<<<64, 256>>>(in, ans_dev, Q, cap_tab, cap_self);
+        return cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess;
       };
       const double tq0 = elapsed_ms();
       if (!ids_tab.reserve(1024) || !lbt_tab.reserve(1024) || !ids_self.reserve(1024) || !lbt_self.reserve(1024) ||
           !query())
         return DPG_ERR_CUDA;
-      if (nts[0] > std::min(ids_tab.cap, lbt_tab.cap) || nts[1] > std::min(ids_self.cap, lbt_self.cap)) {
+      if (ans.fill[0] > std::min(ids_tab.cap, lbt_tab.cap) || ans.fill[1] > std::min(ids_self.cap, lbt_self.cap)) {
         // lists past the capacity: grow them, query again
-        if (!ids_tab.reserve(nts[0]) || !lbt_tab.reserve(nts[0]) || !ids_self.reserve(nts[1]) ||
-            !lbt_self.reserve(nts[1]) || !query())
+        const size_t nt = ans.fill[0], ns = ans.fill[1];
+        if (!ids_tab.reserve(nt) || !lbt_tab.reserve(nt) || !ids_self.reserve(ns) || !lbt_self.reserve(ns) || !query())
           return DPG_ERR_OOM;
       }
-      const int64_t nt = (int64_t)nts[0], ns = (int64_t)nts[1];
-      cudaMemcpy(ct.data(), cnt_tab.p, sizeof(int) * Q, cudaMemcpyDeviceToHost);
-      cudaMemcpy(ca.data(), cnt_all.p, sizeof(int) * Q, cudaMemcpyDeviceToHost);
-      cudaMemcpy(cs.data(), cnt_self.p, sizeof(int) * Q, cudaMemcpyDeviceToHost);
-      cudaMemcpy(ot.data(), off_tab.p, sizeof(int64_t) * Q, cudaMemcpyDeviceToHost);
-      cudaMemcpy(os.data(), off_self.p, sizeof(int64_t) * Q, cudaMemcpyDeviceToHost);
-      it.resize((size_t)nt);
-      is.resize((size_t)ns);
-      lt.resize((size_t)nt);
-      ls.resize((size_t)ns);
-      if (nt) {
-        cudaMemcpy(it.data(), ids_tab.p, sizeof(int) * nt, cudaMemcpyDeviceToHost);
-        cudaMemcpy(lt.data(), lbt_tab.p, sizeof(double) * nt, cudaMemcpyDeviceToHost);
-      }
-      if (ns) {
-        cudaMemcpy(is.data(), ids_self.p, sizeof(int) * ns, cudaMemcpyDeviceToHost);
-        cudaMemcpy(ls.data(), lbt_self.p, sizeof(double) * ns, cudaMemcpyDeviceToHost);
-      }
+      const int *ct = ans.cnt_tab, *ca = ans.cnt_all, *cs = ans.cnt_self, *it = ans.ids_tab, *is = ans.ids_self;
+      const double *lt = ans.lbt_tab, *ls = ans.lbt_self;
+      const int64_t *ot = ans.off_tab, *os = ans.off_self;
       if (cudaGetLastError() != cudaSuccess) return DPG_ERR_CUDA;
       res->query_ms += elapsed_ms() - tq0;
       res->novelty_ms += elapsed_ms() - tn0;
