@@ -55,11 +55,11 @@ L2_FLUSH_BYTES = 512 << 20
 # (profiles/check_pairs_car1_50k.md): sm__inst_executed.avg.per_cycle_active
 # over the SM's 4 issue slots per cycle, and warp instructions per pair.
 CHECK_ISSUE = {
-    2: {"inst_per_cycle": 2.614, "issue_slots": 4, "warp_instructions_per_pair": 879676364 / 4126228,
-        "active_lanes_per_instruction": 17.68},
+    2: {"inst_per_cycle": 3.071, "issue_slots": 4, "warp_instructions_per_pair": 539073772 / 4126602,
+        "active_lanes_per_instruction": 27.08},
 }
 CHECK_TRAFFIC_PER_PAIR = {
-    2: (37.874944e6 + 51.243264e6) / 4126228,  # ncu capture (grouped slot rounds), car1_v0 with 50,000 nodes
+    2: (39.801088e6 + 46.022912e6) / 4126602,  # ncu capture (check_pairs_slots), car1_v0 with 50,000 nodes
 }
 
 

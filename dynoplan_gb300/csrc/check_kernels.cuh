@@ -5,9 +5,10 @@
 // for every in-ball pair of a batch.
 //
 // Work decomposition: persistent warps take (primitive, 32 nodes) items from a
-// device counter, longest primitives first.  The 32 lanes walk the same
-// primitive in lockstep, so the per-state pose rows are warp-broadcast loads
-// and the lanes differ only by their node offset.
+// device counter, longest primitives first.  check_pairs: the 32 lanes walk the
+// same primitive in lockstep, so the per-state pose rows are warp-broadcast
+// loads and the lanes differ only by their node offset.  check_pairs_slots
+// (below, the default) gives every test of the item to a lane of its own.
 //
 // Transform: position_k = canonical_k + p0 (+ k*dt*v0), velocity_k =
 // canonical_k + v0, other components canonical_k.  That is the translation of
@@ -15,7 +16,7 @@
 // shifted start for quad2d / quadrotor (no dynamics term depends on position
 // or velocity); the canonical rollout is FP64, once per upload.
 //
-// Obstacles (shared memory) are culled per lane in two levels, both with a
+// Obstacles (shared memory) are culled in the lockstep walk per lane in two levels, both with a
 // margin of band + slack (+ kGapCap when min_gap is an output) so nothing that
 // could touch the robot, fall in the FP64 band or set min_gap is dropped:
 //   1. against the bounding box of the whole transformed primitive (once per

@@ -12,17 +12,19 @@
 //   nn_prefix       per-primitive exclusive prefix over node tiles
 //   scan_totals     per-primitive bases in length order, work-item bases
 //   nn_emit         pair lists grouped by primitive, nodes in processing order
-//   check_pairs     persistent warps over (primitive, 32 nodes) work items
-//                   (check_kernels.cuh); they also restore the caller's node
-//                   ids of a spatially ordered batch
+//   item_positions  work item -> primitive
+//   check_pairs_slots, check_pairs   persistent warps over (primitive, 32
+//                   nodes) work items (check_kernels.cuh); they also restore
+//                   the caller's node ids of a spatially ordered batch
+// Batches of at most kSmallNodes nodes take small_ball and small_emit in place
+// of all that comes before the check.
 //
 // The reference does this per node with a KD-tree radius query and a
 // per-motion fcl AABB tree (include/dynoplan/dbastar/dbastar.hpp:270-312,
 // src/dbastar/dbastar.cpp:391-490).  Here the pairs of one primitive share
 // every per-state quantity (canonical pose, orientation, action), so a warp
-// walks one primitive for 32 nodes in lockstep: pose rows are broadcast
-// loads, obstacles are broadcast shared-memory reads, and only the node
-// offset differs per lane.
+// takes one primitive for 32 nodes: pose rows are shared by its lanes, and
+// only the node offset differs per lane.
 #pragma once
 
 #include <algorithm>

@@ -66,7 +66,7 @@ template <> struct Robot<DPG_ROBOT_QUAD2D> {
   static constexpr int KEYD = 2;  // theta, w
   static constexpr int CHUNK = 16;  // dt 0.01: ten times the states of the others per second
   static constexpr int CHECK_BLOCKS = 4;
-  static constexpr int SLOT_BLOCKS = 3;  // slot-parallel check: 64 registers a thread
+  static constexpr int SLOT_BLOCKS = 3;  // slot-parallel check: 80 registers a thread
   static constexpr int WINDOW = 8;  // chunks whose slots are listed together
   __host__ __device__ static int key_comp(int i) { return i == 0 ? 2 : 5; }
   __host__ __device__ static int vel_comp(int i) { return 3 + i; }

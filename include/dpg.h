@@ -279,7 +279,8 @@ int dpg_expand_noalloc(dpg_ctx *ctx, const dpg_expand_opts *opts, int64_t N, con
 /* Launch choices of a context (defaults in brackets); dpg_autotune picks
  * them per workload (dpg_tune.h).  Results never depend on them. */
 #define DPG_CHECK_LOCKSTEP 0 /* the 32 lanes of a warp walk their pairs' states and candidates */
-#define DPG_CHECK_SLOTS 1    /* per chunk of states, (lane, candidate) slots spread over the warp */
+#define DPG_CHECK_SLOTS 1    /* (lane, candidate, part, state) tests of a window of states spread over
+                                the warp; up to 512 obstacles, beyond that the walk above */
 typedef struct dpg_tuning {
   int32_t check_variant;       /* DPG_CHECK_* [DPG_CHECK_SLOTS]; FP64_STRICT always walks lockstep */
   int32_t check_blocks_per_sm; /* resident check blocks per SM, 0 = the occupancy maximum [0] */
@@ -306,7 +307,8 @@ int dpg_set_tuning(dpg_ctx *ctx, const dpg_tuning *t);
 
 /* Wait for the context's stream. */
 int dpg_sync(dpg_ctx *ctx);
-/* Raise (1) or clear (0) the abort flag polled by the device work queue. */
+/* Raise (1) or clear (0) the abort flag polled by the device work queue (by a
+ * launch's first warp and with every 64th work item). */
 int dpg_set_abort(dpg_ctx *ctx, int32_t flag);
 
 /* Page-locked host buffers (cudaHostAlloc) for inputs and outputs of
@@ -316,7 +318,8 @@ void *dpg_host_alloc(size_t bytes);
 void dpg_host_free(void *p);
 
 /* Device time of the last dpg_expand, split by stage (milliseconds):
- * t[0] ball scan + compaction, t[1] exact check, t[2] FP64 re-check,
+ * t[0] ball scan + compaction, t[1] exact check (its FP64 decisions are part
+ * of it: t[2] = 0),
  * t[3] host<->device copies.  Returns the number of stages written. */
 int dpg_last_timings(const dpg_ctx *ctx, double *t, int32_t n);
 
