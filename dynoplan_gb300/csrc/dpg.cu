@@ -911,6 +911,20 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
   else if (N > 0 && !opts->x_on_device)
     CUDA_TRY(c, cudaMemcpyAsync(c->x64.p, x, sizeof(double) * nx * N, cudaMemcpyHostToDevice, st));
   const double *x_dev = opts->x_on_device ? x : P_<double>(c->x64);  // the nodes, in the caller's order
+  if (opts->x_on_device && N > 0) {
+    // The kernels read the caller's array to the end of the check, so nodes that
+    // lie in an output of this call, or not on 8 bytes, are read from a copy
+    const uintptr_t lo = reinterpret_cast<uintptr_t>(x), hi = lo + sizeof(double) * nx * (size_t)N;
+    bool copy = lo % sizeof(double) != 0;
+    for (const auto &f : sm_out) {
+      const uintptr_t a = reinterpret_cast<uintptr_t>(f.dst);
+      copy = copy || (f.dst && a < hi && lo < a + f.row * (size_t)std::max<int64_t>(cap, 0));
+    }
+    if (copy) {
+      CUDA_TRY(c, cudaMemcpyAsync(c->x64.p, x, hi - lo, cudaMemcpyDeviceToDevice, st));
+      x_dev = P_<double>(c->x64);
+    }
+  }
   if (!small) CUDA_TRY(c, cudaMemsetAsync(c->d_ctr, 0, sizeof(DevCounters), st));
   CUDA_TRY(c, cudaEventRecord(c->ev[1], st));
 
