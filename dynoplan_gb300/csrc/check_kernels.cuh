@@ -1082,10 +1082,10 @@ __device__ void load_obstacles(const EnvView &ev, void *sm) {
 // the link serves about 150 M such reads a second whatever the SMs do, so a
 // read per item bounded the whole check (car1, 100,000 nodes x 5,000 motions,
 // 260,000 items: 1.73 ms for fetching the items alone, 0.18 ms without the
-// reads).  The launch's first warp reads it, then the warps that draw every
-// kAbortPoll-th item (one read in a few hundred nanoseconds of a full GPU); on
-// an abort they move the launch's item counter past its end.
-constexpr unsigned long long kAbortPoll = 64;
+// reads).  So a warp reads it when it takes up every kAbortPoll-th item of the
+// launch, the first included (one read in a few hundred nanoseconds of a full
+// GPU); on an abort it moves the launch's item counter past its end.
+constexpr uint32_t kAbortPoll = 64;
 constexpr unsigned long long kNoMoreItems = 1ull << 62;
 
 // Persistent warps over (primitive, 32 nodes) work items: item(p, pair, count,
@@ -1123,25 +1123,22 @@ __device__ __forceinline__ void for_items(const CheckArgs &A, Item item_fn) {
   // while the current one is checked.
   const uint32_t warps = gridDim.x * (blockDim.x >> 5), w_id = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   uint32_t next = w_id < n_items - i_lo ? i_lo + w_id : n_items;
-  auto poll_abort = [&]() {
-    if (*A.abort_flag) {
-      A.ctr->status = DPG_ERR_ABORTED;  // every warp's next item lies past the end
-      atomicMax(&A.ctr->next_sub[A.sub], kNoMoreItems);
-      next = n_items;
-    }
-  };
-  auto draw = [&]() {
-    if (lane == 0) {
-      const unsigned long long drawn = atomicAdd(&A.ctr->next_sub[A.sub], 1ull);
-      next = drawn + warps < n_items - i_lo ? i_lo + warps + (uint32_t)drawn : n_items;
-      if (next < n_items && drawn % kAbortPoll == 0) poll_abort();
-    }
-  };
-  if (lane == 0 && w_id == 0 && next < n_items) poll_abort();
   while (true) {
     const uint32_t item = __shfl_sync(kFull, next, 0);
     if (item >= n_items) break;
-    draw();
+    if ((item - i_lo) % kAbortPoll == 0) {
+      int stop = 0;
+      if (lane == 0 && *A.abort_flag) {
+        stop = 1;
+        A.ctr->status = DPG_ERR_ABORTED;  // every warp's next draw lies past the end
+        atomicMax(&A.ctr->next_sub[A.sub], kNoMoreItems);
+      }
+      if (__shfl_sync(kFull, stop, 0)) break;
+    }
+    if (lane == 0) {
+      const unsigned long long drawn = atomicAdd(&A.ctr->next_sub[A.sub], 1ull);
+      next = drawn + warps < n_items - i_lo ? i_lo + warps + (uint32_t)drawn : n_items;
+    }
     if (A.n_ranges > 1) {
       int j = 0;
       while (j + 1 < A.n_ranges && item >= range_end(j)) j++;

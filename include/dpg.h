@@ -307,8 +307,8 @@ int dpg_set_tuning(dpg_ctx *ctx, const dpg_tuning *t);
 
 /* Wait for the context's stream. */
 int dpg_sync(dpg_ctx *ctx);
-/* Raise (1) or clear (0) the abort flag polled by the device work queue (by a
- * launch's first warp and with every 64th work item). */
+/* Raise (1) or clear (0) the abort flag polled by the device work queue (by the
+ * warp that takes up a launch's first work item, and every 64th after it). */
 int dpg_set_abort(dpg_ctx *ctx, int32_t flag);
 
 /* Page-locked host buffers (cudaHostAlloc) for inputs and outputs of
