@@ -67,7 +67,11 @@ template <> struct Robot<DPG_ROBOT_QUAD2D> {
   static constexpr int CHUNK = 16;  // dt 0.01: ten times the states of the others per second
   static constexpr int CHECK_BLOCKS = 4;
   static constexpr int SLOT_BLOCKS = 3;  // slot-parallel check: 80 registers a thread
-  static constexpr int WINDOW = 8;  // chunks whose slots are listed together
+  // chunks whose slots are listed together: shorter among many obstacles, where
+  // lanes meet one early and a longer window's slots do not fit (check kernel, us,
+  // windows of 8 / 4 / 3 / 2: 300 nodes x 10,000 motions, 40 obstacles 145 / 129 /
+  // 131 / 141, 100 of them 289 / 201 / 197 / 215; 32 nodes, 40: 48.8 / 47.1 / 47.1 / 53.6)
+  static constexpr int WINDOW = 3;
   __host__ __device__ static int key_comp(int i) { return i == 0 ? 2 : 5; }
   __host__ __device__ static int vel_comp(int i) { return 3 + i; }
 };

@@ -45,3 +45,28 @@ def test_long_items_start_on_free_warps(dpg_lib, variant, L):
             assert r["n_pairs"] == cap
             times.append(float(np.median(t)))
     assert times[1] < 1.6 * times[0], times
+
+
+@pytest.mark.parametrize("n_obs", [100, 128, 400])
+@pytest.mark.parametrize("kind,P,steps,radius", [(W.QUAD2D, 1500, (20, 150), 0.3), (W.CAR1, 1000, (5, 100), 0.25)])
+def test_slots_among_many_obstacles(dpg_lib, kind, P, steps, radius, n_obs):
+    """The windows' slots must not cost more than a lane walking its own tests: no
+    slower than the lockstep walk (1.7 times as slow for quad2d with windows
+    whose slots did not fit)."""
+    from dynoplan_gb300 import gpu as G
+    m = W.robot_model(kind)
+    prims = W.make_primitives(m, P, *steps, seed=3)
+    env = W.make_env((8.0, 4.0), n_obs, 0.05, 0.25, seed=4)
+    x = W.make_nodes(m, W.Env(env.lo, env.hi, env.obs_lo[:0], env.obs_hi[:0]), 1200, seed=6)
+    x = np.ascontiguousarray(x[np.sort(np.argsort(-W.state_gap(m, env, x))[:300])])  # the freest
+    with G.Context(m) as ctx:
+        ctx.upload_primitives(prims)
+        ctx.upload_env(env)
+        t = {0: [], 1: []}
+        for i in range(14):
+            for v in t:
+                ctx.set_tuning(check_variant=v)
+                ctx.expand(x, radius, capacity=300 * P)
+                if i >= 3:
+                    t[v].append(ctx.timings()[1])
+        assert np.median(t[1]) <= 1.1 * np.median(t[0]), (np.median(t[1]), np.median(t[0]))
