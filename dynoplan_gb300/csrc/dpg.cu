@@ -207,10 +207,13 @@ static int nn_tiles_per_y(int P, int64_t B, int sm_count) {
 // (an expand whose results go to host buffers runs tune.pipe_launches <=
 // kMaxSub check launches, one work-queue counter each)
 
-// smallest group of copy ranges copied together: a quarter of the results, so
-// that a search round's 10 MB leave while they are checked, within these (a
-// copy call costs host time, and below 2 MB more than it hides)
-constexpr size_t kMinCopyBytes = 2u << 20, kMaxCopyBytes = 16u << 20;
+// copy ranges are copied together in groups of a quarter of the results, at most
+// kMaxCopyBytes; results below kSplitBytes in one group after the check: copies
+// to pageable arrays keep the caller until they are done, and each costs some
+// 25 us.  Call, us, one group / quarters: 2,000 cars x 5,000 (9 MB, pageable) 390 /
+// 547, 150 quad2d x 10,000 (11 MB) 414 / 585, 8,000 unicycles x 1,000 (28.5 MB) 527 /
+// 660 and in page-locked arrays 473 / 458, 2,100 cars (26 MB) there 647 / 619
+constexpr size_t kSplitBytes = 20u << 20, kMaxCopyBytes = 16u << 20;
 // results (of N x P pairs) from which a batch under kReorderMin nodes is copied
 // in ranges too: quad2d x 10,000 with every output, copies after the check /
 // in ranges: 32 nodes (13 MB) 238 / 259 us, 64 nodes 388 / 382, 100 nodes
@@ -1105,7 +1108,8 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
       // consecutive ranges are copied together until a group holds min_copy
       // bytes; the last range closes the last group
       const size_t bpp = row_bytes;  // bytes copied per pair
-      const size_t min_copy = std::clamp((size_t)h0.n_pairs * bpp / 4, kMinCopyBytes, kMaxCopyBytes);
+      const size_t total = (size_t)h0.n_pairs * bpp;
+      const size_t min_copy = total < kSplitBytes ? total : std::min(total / 4, kMaxCopyBytes);
       int64_t ga = -1;
       for (int j = 0; j < np; j++) {
         const int64_t a = pair_at(h0.n_items * cum[j] / cum[np]), e = pair_at(h0.n_items * cum[j + 1] / cum[np]);
