@@ -73,9 +73,10 @@ struct dpg_ctx {
   // launch choices (dpg_set_tuning): check variant, blocks per SM, the batch
   // size from which the ball scan uses the key grid, pipelined check launches
   dpg_tuning tune{DPG_CHECK_SLOTS, 0, 2048, 8, DPG_HOST_OUT_PROGRESS};
-  cudaEvent_t ev[6] = {};
-  // stage times of the last call; timings_due: dpg_expand's events hold them
-  // (read when asked for)
+  // events of a call, and of the last dpg_expand that succeeded (exchanged then)
+  cudaEvent_t ev_all[12] = {}, *ev = ev_all, *ev_done = ev_all + 6;
+  // stage times of the last call that succeeded; timings_due: ev_done holds
+  // them (read when asked for)
   double timings[4] = {0, 0, 0, 0};
   bool timings_due = false;
   // resident blocks per SM of the check kernels, as launched before

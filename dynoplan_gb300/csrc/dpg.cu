@@ -359,7 +359,7 @@ int dpg_create(dpg_ctx **out, int device, const dpg_robot_desc *robot) {
     if (cudaHostAlloc(&c->h_small, kSmallX + kSmallBytes, cudaHostAllocMapped) != cudaSuccess) { rc = DPG_ERR_OOM; break; }
     if (cudaHostGetDevicePointer(&c->d_small, c->h_small, 0) != cudaSuccess) { rc = DPG_ERR_CUDA; break; }
     if (cudaHostGetDevicePointer(&c->d_abort, c->h_abort, 0) != cudaSuccess) { rc = DPG_ERR_CUDA; break; }
-    for (auto &e : c->ev)
+    for (auto &e : c->ev_all)
       if (cudaEventCreate(&e) != cudaSuccess) { rc = DPG_ERR_CUDA; break; }
   } while (0);
   if (rc != DPG_OK) {
@@ -401,7 +401,7 @@ void dpg_destroy(dpg_ctx *c) {
   if (c->cstream) cudaStreamDestroy(c->cstream);
   if (c->xstream) cudaStreamDestroy(c->xstream);
   if (c->h_abort) cudaFreeHost(c->h_abort);
-  for (auto &e : c->ev)
+  for (auto &e : c->ev_all)
     if (e) cudaEventDestroy(e);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -673,10 +673,10 @@ int dpg_upload_env(dpg_ctx *c, int32_t dim, const double *lo, const double *hi, 
 // stage times of the last dpg_expand from its events (all complete)
 static void read_timings(dpg_ctx *c) {
   float a = 0, b = 0, t_in = 0, t_out = 0;
-  cudaEventElapsedTime(&a, c->ev[1], c->ev[2]);
-  cudaEventElapsedTime(&b, c->ev[2], c->ev[3]);
-  cudaEventElapsedTime(&t_in, c->ev[0], c->ev[1]);
-  cudaEventElapsedTime(&t_out, c->ev[3], c->ev[5]);
+  cudaEventElapsedTime(&a, c->ev_done[1], c->ev_done[2]);
+  cudaEventElapsedTime(&b, c->ev_done[2], c->ev_done[3]);
+  cudaEventElapsedTime(&t_in, c->ev_done[0], c->ev_done[1]);
+  cudaEventElapsedTime(&t_out, c->ev_done[3], c->ev_done[5]);
   c->timings[0] = a;
   c->timings[1] = b;
   c->timings[2] = 0;
@@ -1170,6 +1170,7 @@ int dpg_expand(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N, const double 
     CUDA_TRY(c, cudaEventRecord(c->ev[5], st));
     CUDA_TRY(c, cudaStreamSynchronize(st));
   }
+  std::swap(c->ev, c->ev_done);
   c->timings_due = true;
   if (pipelined) read_timings(c);
   if (pipelined && last_bytes >= (1u << 20) && np > 0 && c->timings[1] > 0) {
