@@ -309,7 +309,8 @@ __device__ __forceinline__ float key_dist32(const float4 w, const float *nk,
 // key[i], kc: the primitives' key components and constants in pairs; nk2: the
 // node's, twice (the velocity negated).  Given weights that are not negative it
 // is within quad_margin of key_dist32 wherever that matters: near the radius no
-// term is above it, and further out the rounding grows slower than the distance.
+// term (kc's have w.x and w.z) is above it, and further out the rounding grows
+// slower than the distance.
 // Pairs within the margin, about one in a hundred, take key_dist32.  Bound by
 // this arithmetic: for 50,000 nodes x 5,000 primitives the ball stage took
 // 1.13 ms with acosf and exact roots for every pair, 0.46 ms with this.
@@ -343,7 +344,7 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
   return x;
 }
 __device__ __forceinline__ float quad_margin(const float4 w, float radius, float band) {
-  return w.y >= 0.f && w.w >= 0.f ? band + 1e-4f * w.y + 1e-5f * fabsf(radius) : INFINITY;
+  return w.x >= 0.f && w.y >= 0.f && w.z >= 0.f && w.w >= 0.f ? band + 1e-4f * w.y + 1e-5f * fabsf(radius) : INFINITY;
 }
 
 // Ball membership of 256 nodes (blockIdx.x) against the primitives of

@@ -40,3 +40,35 @@ def test_ball_quadrotor(dpg_lib, N, P, radius):
             if nodes is x:
                 ora = ob.expand(wl.robot, wl.prims, wl.env, nodes, radius, fast=True, threads=ob.lib().orc_max_threads())
                 np.testing.assert_array_equal(np.sort(pairs(whole)), np.sort(pairs(ora)))
+
+
+@pytest.mark.parametrize("w", [(-2e4, 0.5, 1.0, 2e4), (1.0, 0.5, -2e4, 2e4), (1.0, -0.5, 1.0, 1.0), (1.0, 0.5, 1.0, -1.0)])
+def test_ball_quadrotor_negative_weights(dpg_lib, w):
+    """With a negative weight the terms of the distance may cancel near the radius
+    (nodes placed there by the rounding of terms of 1e4): exact distances."""
+    import dataclasses
+
+    from dynoplan_gb300 import gpu as G
+    N, P, radius = 1000, 64, 1.0
+    wl = W.make_workload(3, seed=31, N=N, P=P)
+    m = dataclasses.replace(wl.robot, w=w)
+    prims = wl.prims
+    start = np.concatenate([[0], np.cumsum(prims.length)[:-1]])
+    rng = np.random.default_rng(8)
+    s = prims.states[start]
+    s[:, :3], s[:, 7:10] = rng.uniform(0.3, 1.0, (2, P, 3))  # starts that differ in position and velocity
+    prims.states[start] = s
+    p = np.arange(N) % P
+    x = wl.nodes.copy()
+    x[:, 3:13] = s[p, 3:13]  # the orientation is the primitive's: acos 0
+    kc = w[0] * np.linalg.norm(s[p, :3], axis=1) + w[2] * np.linalg.norm(s[p, 7:10], axis=1)
+    gap = np.maximum((radius + rng.uniform(-4e-3, 4e-3, N) - kc) / w[3], 0.0)
+    x[:, 10] += gap
+    with G.Context(m) as ctx:
+        ctx.upload_primitives(prims)
+        ctx.upload_env(wl.env)
+        whole = ctx.expand(x, radius, ball_only=True, capacity=N * P)
+        parts = [ctx.expand(x[i:i + 128], radius, ball_only=True, capacity=N * P) for i in range(0, N, 128)]
+        want = np.concatenate([pairs(r, 128 * k) for k, r in enumerate(parts)])
+        np.testing.assert_array_equal(np.sort(pairs(whole)), np.sort(want))
+        assert whole["n_ball_recheck"] == sum(r["n_ball_recheck"] for r in parts)
