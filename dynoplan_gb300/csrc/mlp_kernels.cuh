@@ -351,7 +351,8 @@ static __global__ void __launch_bounds__(kWgThreads, 1) mlp_wgrad(const __grid_c
     if (umma::elect_one()) umma::commit(done);  // once every MMA issued above is complete
     __syncwarp();
   } else if (warp >= 4 && J.db) {
-    // column sums of a: a thread two columns (word w of block k), over the rows
+    // column sums of a: a thread two columns (word w of block k), over the rows,
+    // 32 at a time (a running sum over a CTA's 1,500 rows loses small ones)
     const int k = warp - 4;
     float s0 = 0.f, s1 = 0.f;
     bool ok = true;
@@ -360,11 +361,17 @@ static __global__ void __launch_bounds__(kWgThreads, 1) mlp_wgrad(const __grid_c
       ok = umma::mbar_wait_warp(&full[s], (i / kWgStages) & 1);
       if (!ok) break;
       const unsigned char *t = base + s * kWgStage + k * kWgBlock;
+#pragma unroll
+      for (int r0 = 0; r0 < 64; r0 += 32) {
+        float p0 = 0.f, p1 = 0.f;
 #pragma unroll 16
-      for (int r = 0; r < 64; r++) {
-        const uint32_t v = *reinterpret_cast<const uint32_t *>(t + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + 4 * (lane & 3));
-        s0 += __uint_as_float(v << 16);
-        s1 += __uint_as_float(v & 0xffff0000u);
+        for (int r = r0; r < r0 + 32; r++) {
+          const uint32_t v = *reinterpret_cast<const uint32_t *>(t + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + 4 * (lane & 3));
+          p0 += __uint_as_float(v << 16);
+          p1 += __uint_as_float(v & 0xffff0000u);
+        }
+        s0 += p0;
+        s1 += p1;
       }
       __syncwarp();
       if (lane == 0) umma::mbar_arrive(&empty[s]);

@@ -38,3 +38,29 @@ def test_gradients(dpg_lib, B):
         if k in ("W4", "b4"):
             g, r = g[:2], r[:2]
         assert np.linalg.norm(g - r) <= 2e-2 * max(np.linalg.norm(r), 1e-12), k
+
+
+def test_bias_gradient_keeps_small_terms(dpg_lib):
+    """db3 = sum_b dZ3[b] with one row of 1 and 65,535 of 2^-26 (weights zero, so
+    that dZ3 = dY / 2 exactly).  Tolerance: a sum of 32 rows, of a CTA's parts
+    (under 64) and of the CTAs (under 64), each addition within half an ulp:
+    (31 + 64 + 64) 2^-24 = 9.5e-6; one running sum over a CTA's rows loses
+    1,400 x 2^-26 = 2.1e-5."""
+    torch = pytest.importorskip("torch")
+    from dynoplan_gb300.surrogate import SHAPES, Surrogate
+    B, P = 65536, 4
+    s = Surrogate(P, max_rows=B, seed=1)
+    for k, shape in SHAPES.items():
+        s.set(k, np.zeros(shape, np.float32))
+    w4 = np.zeros((16, 256), np.float32)
+    w4[1] = 1.0
+    s.set("W4", w4)
+    dz = np.full(B, 2.0 ** -26)
+    dz[0] = 1.0
+    target = np.stack([np.full(B, np.nan), -2.0 * dz * B], 1).astype(np.float32)  # dY = -target / B
+    feat = torch.zeros((1, 80), dtype=torch.bfloat16, device="cuda")
+    zero = torch.zeros(B, dtype=torch.int32, device="cuda")
+    s.train_step(feat, zero, zero, torch.from_numpy(target).cuda(), lr=0.0)
+    g = s.get("b3", grad=True).astype(np.float64)
+    assert np.abs(g / dz.sum() - 1).max() <= (31 + 64 + 64) * 2.0 ** -24
+    s.close()
