@@ -247,8 +247,11 @@ static __global__ void transpose_bf16(const __nv_bfloat16 *in, __nv_bfloat16 *ou
 // MN-major straight from the row-major activations (boxes of 64 rows x 64
 // columns by TMA): no transposed copies are written.  A layer's CTAs take
 // ranges of 64-row chunks; a CTA holds the whole gradient, two M = 128 tiles of
-// up to 256 columns, in TMEM, so each operand is read once, and adds it to g at
-// the end (float4 atomics).  Warps 4-7 sum the columns of a (the bias
+// up to 256 columns, in TMEM, so each operand is read once, and adds it to g
+// (float4 atomics) at the end or after every kWgRun chunks an accumulator: longer
+// runs' error against 64 bits exceeds that of sums over 900 rows (rms of dW3 at
+// 65,536 rows of one sign 2.3e-6, 1.2e-6 with 900 rows, 0.95e-6 with these; a
+// step takes 266 us with them, 256 without).  Warps 4-7 sum the columns of a (the bias
 // gradients) from the staged tiles while the tensor cores use them.
 // Bound by reading the operands (2 x 33.5 MB a hidden layer at 65,536 rows):
 // all four layers 48 us; as transposed copies written by the layers'
@@ -264,7 +267,7 @@ struct alignas(128) WgradJob {
 struct alignas(128) WgradArgs {
   WgradJob job[4];
 };
-constexpr int kWgThreads = 256, kWgStages = 3;
+constexpr int kWgThreads = 256, kWgStages = 3, kWgRun = 14;
 constexpr uint32_t kWgBlock = 64 * 128;        // 64 rows x 64 columns
 constexpr uint32_t kWgStage = 8 * kWgBlock;    // a: 256 columns, b: up to 256
 constexpr size_t kWgSmem = 1024 + kWgStages * kWgStage + 256;
@@ -304,102 +307,107 @@ static __global__ void __launch_bounds__(kWgThreads, 1) mlp_wgrad(const __grid_c
   umma::fence_after_sync();
   const uint32_t tmem = *tslot;
 
+  // Accumulators: the tensor cores cut a sum's low bits at every step of 16 rows,
+  // so one takes at most kWgRun chunks.  Chunk i goes to accumulator i % sets
+  // (256 columns of TMEM hold several of a narrow layer's); a CTA with more than
+  // sets * kWgRun chunks adds its accumulators to g several times.
+  const int stride = J.n <= 32 ? 32 : J.n <= 128 ? 128 : 256, sets = 256 / stride;
+  const int runs = (n + sets * kWgRun - 1) / (sets * kWgRun);
   int loads = 0;  // (thread 0) chunks whose loads were issued
-  if (tid == 0) {
-    for (int i = 0; i < n; i++) {
-      const int s = i % kWgStages;
-      if ((i >= kWgStages && !umma::mbar_wait(&empty[s], ((i / kWgStages) - 1) & 1)) || *bad) {
-        *bad = 1;
-        break;
-      }
-      unsigned char *st = base + s * kWgStage;
-      const int row = (int)(64 * (c0 + i));
-      umma::mbar_arrive_expect_tx(&full[s], bytes);
-      for (int k = 0; k < 4; k++) umma::tma_load_2d(st + k * kWgBlock, &J.a, 64 * k, row, &full[s]);
-      for (int k = 0; k < b_blocks; k++) umma::tma_load_2d(st + (4 + k) * kWgBlock, &J.b, 64 * k, row, &full[s]);
-      loads = i + 1;
-    }
-  } else if (warp == 1) {
-    const uint32_t idesc = umma::idesc_bf16_f32(128, J.n) | umma::kIdescMnMajorAB;
-    const uint64_t ad = umma::sdesc_mnmajor_sw128(umma::smem_u32(base), kWgBlock);
-    const uint64_t bd = ad + (4 * kWgBlock >> 4);
-    uint32_t s = 0, parity = 0;
-    bool ok = true;
-    for (int i = 0; i < n && ok; i++) {
-      if (!umma::mbar_wait_warp(&full[s], parity)) {
-        ok = false;
-        break;
-      }
-      umma::fence_after_sync();
-      const uint64_t so = s * (kWgStage >> 4);
-      if (umma::elect_one()) {
-#pragma unroll
-        for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-          for (int kk = 0; kk < 4; kk++)  // 16 rows a step
-            umma::mma_bf16(tmem + 256u * mt, ad + so + mt * (2 * kWgBlock >> 4) + kk * (2048 >> 4),
-                           bd + so + kk * (2048 >> 4), idesc, (i > 0 || kk > 0) ? 1u : 0u);
-        umma::commit(&empty[s]);
-      }
-      __syncwarp();
-      if (++s == kWgStages) {
-        s = 0;
-        parity ^= 1u;
-      }
-    }
-    if (!ok && lane == 0) *bad = 1;
-    if (umma::elect_one()) umma::commit(done);  // once every MMA issued above is complete
-    __syncwarp();
-  } else if (warp >= 4 && J.db) {
-    // column sums of a: a thread two columns (word w of block k), over the rows,
-    // 32 at a time (a running sum over a CTA's 1,500 rows loses small ones)
-    const int k = warp - 4;
-    float s0 = 0.f, s1 = 0.f;
-    bool ok = true;
-    for (int i = 0; i < n && ok; i++) {
-      const int s = i % kWgStages;
-      ok = umma::mbar_wait_warp(&full[s], (i / kWgStages) & 1);
-      if (!ok) break;
-      const unsigned char *t = base + s * kWgStage + k * kWgBlock;
-#pragma unroll
-      for (int r0 = 0; r0 < 64; r0 += 32) {
-        float p0 = 0.f, p1 = 0.f;
-#pragma unroll 16
-        for (int r = r0; r < r0 + 32; r++) {
-          const uint32_t v = *reinterpret_cast<const uint32_t *>(t + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + 4 * (lane & 3));
-          p0 += __uint_as_float(v << 16);
-          p1 += __uint_as_float(v & 0xffff0000u);
-        }
-        s0 += p0;
-        s1 += p1;
-      }
-      __syncwarp();
-      if (lane == 0) umma::mbar_arrive(&empty[s]);
-    }
-    if (!ok) {
-      if (lane == 0) *bad = 1;
-    } else if (n > 0) {
-      atomicAdd(J.db + 64 * k + 2 * lane, s0);
-      atomicAdd(J.db + 64 * k + 2 * lane + 1, s1);
-    }
-  }
-  __syncwarp();
-  const bool fin = umma::mbar_wait(done, 0);
-  const bool failed = __syncthreads_or(!fin || *bad);
-  if (failed) {
+  uint32_t ms = 0, mparity = 0;  // (warp 1) the next stage, parity of its next completion
+  float s0 = 0.f, s1 = 0.f;      // (warps 4-7) column sums
+  bool failed = false;
+  for (int run = 0; run < runs && !failed; run++) {
+    const int i0 = (int)((int64_t)n * run / runs), i1 = (int)((int64_t)n * (run + 1) / runs);
     if (tid == 0) {
-      atomicExch(err, 1);
-      // copies still in flight land before the block's shared memory goes
-      for (int i = max(0, loads - kWgStages); i < loads; i++)
-        umma::mbar_wait(&full[i % kWgStages], (i / kWgStages) & 1, 1u << 20);
+      for (; loads < min(n, i1 + kWgStages); loads++) {  // and the next run's first ones
+        const int s = loads % kWgStages;
+        if ((loads >= kWgStages && !umma::mbar_wait(&empty[s], ((loads / kWgStages) - 1) & 1)) || *bad) {
+          *bad = 1;
+          break;
+        }
+        unsigned char *st = base + s * kWgStage;
+        const int row = (int)(64 * (c0 + loads));
+        umma::mbar_arrive_expect_tx(&full[s], bytes);
+        for (int k = 0; k < 4; k++) umma::tma_load_2d(st + k * kWgBlock, &J.a, 64 * k, row, &full[s]);
+        for (int k = 0; k < b_blocks; k++) umma::tma_load_2d(st + (4 + k) * kWgBlock, &J.b, 64 * k, row, &full[s]);
+      }
+    } else if (warp == 1) {
+      const uint32_t idesc = umma::idesc_bf16_f32(128, J.n) | umma::kIdescMnMajorAB;
+      const uint64_t ad = umma::sdesc_mnmajor_sw128(umma::smem_u32(base), kWgBlock);
+      const uint64_t bd = ad + (4 * kWgBlock >> 4);
+      bool ok = true;
+      umma::fence_after_sync();
+      for (int i = i0; i < i1; i++) {
+        if (!umma::mbar_wait_warp(&full[ms], mparity)) {
+          ok = false;
+          break;
+        }
+        umma::fence_after_sync();
+        const uint64_t so = ms * (kWgStage >> 4);
+        const uint32_t acc = tmem + (uint32_t)((i - i0) % sets * stride);
+        if (umma::elect_one()) {
+#pragma unroll
+          for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++)  // 16 rows a step
+              umma::mma_bf16(acc + 256u * mt, ad + so + mt * (2 * kWgBlock >> 4) + kk * (2048 >> 4),
+                             bd + so + kk * (2048 >> 4), idesc, (i - i0 >= sets || kk > 0) ? 1u : 0u);
+          umma::commit(&empty[ms]);
+        }
+        __syncwarp();
+        if (++ms == kWgStages) {
+          ms = 0;
+          mparity ^= 1u;
+        }
+      }
+      if (!ok && lane == 0) *bad = 1;
+      if (umma::elect_one()) umma::commit(done);  // once every MMA issued above is complete
+      __syncwarp();
+    } else if (warp >= 4 && J.db) {
+      // column sums of a: a thread two columns (word w of block k), over the rows,
+      // 32 at a time (a running sum over a CTA's 1,500 rows loses small ones)
+      const int k = warp - 4;
+      for (int i = i0; i < i1; i++) {
+        const int s = i % kWgStages;
+        if (!umma::mbar_wait_warp(&full[s], (i / kWgStages) & 1)) {
+          if (lane == 0) *bad = 1;
+          break;
+        }
+        const unsigned char *t = base + s * kWgStage + k * kWgBlock;
+#pragma unroll
+        for (int r0 = 0; r0 < 64; r0 += 32) {
+          float p0 = 0.f, p1 = 0.f;
+#pragma unroll 16
+          for (int r = r0; r < r0 + 32; r++) {
+            const uint32_t v = *reinterpret_cast<const uint32_t *>(t + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + 4 * (lane & 3));
+            p0 += __uint_as_float(v << 16);
+            p1 += __uint_as_float(v & 0xffff0000u);
+          }
+          s0 += p0;
+          s1 += p1;
+        }
+        __syncwarp();
+        if (lane == 0) umma::mbar_arrive(&empty[s]);
+      }
     }
-  } else if (n > 0) {
+    __syncwarp();
+    const bool fin = umma::mbar_wait(done, run & 1);
+    failed = __syncthreads_or(!fin || *bad);
+    if (failed) break;
     umma::fence_after_sync();
     const int q = warp & 3, mt = warp >> 2, m = 128 * mt + 32 * q + lane;
     const uint32_t src = tmem + ((uint32_t)(32 * q) << 16) + 256u * (uint32_t)mt;
-    for (int k = 0; k < J.n; k += 16) {
+    for (int c = 0; c < J.n; c += 16) {
+      const int k = (c + 16 * (int)rel) % J.n;  // (the layer's CTAs start at different columns)
       float v[16];
       umma::tmem_ld16(src + k, v);
+      for (int a = 1; a < min(sets, i1 - i0); a++) {
+        float u[16];
+        umma::tmem_ld16(src + a * stride + k, u);
+#pragma unroll
+        for (int e = 0; e < 16; e++) v[e] += u[e];
+      }
       if (J.transposed) {
         atomicAdd(J.g + m, v[0]);
         atomicAdd(J.g + J.ld + m, v[1]);
@@ -409,6 +417,19 @@ static __global__ void __launch_bounds__(kWgThreads, 1) mlp_wgrad(const __grid_c
         for (int j = 0; j < 4; j++) atomicAdd(dst + j, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
       }
     }
+    umma::fence_before_sync();
+    __syncthreads();  // the next run's MMAs write the accumulators
+  }
+  if (failed) {
+    if (tid == 0) {
+      atomicExch(err, 1);
+      // copies still in flight land before the block's shared memory goes
+      for (int i = max(0, loads - kWgStages); i < loads; i++)
+        umma::mbar_wait(&full[i % kWgStages], (i / kWgStages) & 1, 1u << 20);
+    }
+  } else if (warp >= 4 && J.db && n > 0) {
+    atomicAdd(J.db + 64 * (warp - 4) + 2 * lane, s0);
+    atomicAdd(J.db + 64 * (warp - 4) + 2 * lane + 1, s1);
   }
   umma::fence_before_sync();
   __syncthreads();

@@ -64,3 +64,31 @@ def test_bias_gradient_keeps_small_terms(dpg_lib):
     g = s.get("b3", grad=True).astype(np.float64)
     assert np.abs(g / dz.sum() - 1).max() <= (31 + 64 + 64) * 2.0 ** -24
     s.close()
+
+
+def test_weight_gradient_of_one_sign(dpg_lib):
+    """dW3 = sum_b dZ3[b] H2[b] at 65,536 rows of one sign, H2 = b2 (gelu of 8 to 16
+    in bf16) and dZ3 = dY / 2 exactly.  Tolerance (rms, relative): an accumulator
+    takes at most 14 x 64 rows, 56 steps that each cut half a unit in the last place
+    on average off a partial sum that is half the total on average, 56 x 2^-23 / 4 =
+    1.7e-6, and 2 x 45 roundings of the CTAs' sums, sqrt(90) 2^-25 = 0.3e-6
+    (2.3e-6 with 92 steps)."""
+    torch = pytest.importorskip("torch")
+    from dynoplan_gb300.surrogate import SHAPES, Surrogate
+    B = 65536
+    s = Surrogate(4, max_rows=B, seed=1)
+    for k, shape in SHAPES.items():
+        s.set(k, np.zeros(shape, np.float32))
+    w4, b2 = np.zeros((16, 256), np.float32), (8 + (2 * (np.arange(256) % 64) + 1) / 16).astype(np.float32)
+    w4[1] = 1.0
+    s.set("W4", w4)
+    s.set("b2", b2)
+    dy = torch.from_numpy(np.random.default_rng(3).random(B) / B).to(torch.bfloat16).double().numpy()
+    target = np.stack([np.full(B, np.nan), -dy * B], 1).astype(np.float32)
+    feat = torch.zeros((1, 80), dtype=torch.bfloat16, device="cuda")
+    zero = torch.zeros(B, dtype=torch.int32, device="cuda")
+    s.train_step(feat, zero, zero, torch.from_numpy(target).cuda(), lr=0.0)
+    g = s.get("W3", grad=True).astype(np.float64)
+    e = g / (0.5 * dy.sum() * b2[None, :].astype(np.float64)) - 1
+    assert np.sqrt((e ** 2).mean()) <= 56 * 2.0 ** -25 + 90 ** 0.5 * 2.0 ** -25
+    s.close()
