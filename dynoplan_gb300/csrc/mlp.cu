@@ -2,6 +2,7 @@
 // surrogate MLP built on it.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include <cstring>
@@ -204,6 +205,7 @@ struct dpg_mlp {
   // activations and backward buffers (rows_pad rows)
   __nv_bfloat16 *X = nullptr, *H[3] = {}, *dZ[3] = {}, *dY = nullptr, *T1 = nullptr;
   __nv_bfloat16 *G[3] = {};  // gelu'(pre-activation) of layers 1-3 (training)
+  __nv_bfloat16 *TA = nullptr, *TB = nullptr;  // without tensor maps: transposed operands of a weight gradient
   double *loss = nullptr;  // one allocation: the loss, then the gradients g[]
   size_t sums_bytes = 0;
   int *err = nullptr;
@@ -261,7 +263,7 @@ void refresh_bf16(dpg_mlp *M, int which, cudaStream_t st) {
   if (which % 2) return;  // biases stay FP32
   const int l = which / 2, rows = kOut[l], cols = kIn[l];
   f32_to_bf16<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(M->w[which], M->W16[l], n);
-  dim3 tb(32, 8), tg((cols + 31) / 32, (rows + 31) / 32);
+  dim3 tb(32, 8), tg((rows + 31) / 32, (cols + 31) / 32);
   if (l < 3) {
     transpose_bf16<<<tg, tb, 0, st>>>(M->W16[l], M->WT16[l], rows, cols);
   } else {  // [16 x 256] -> [256 x 16] -> rows of 64 (zero padded)
@@ -363,7 +365,7 @@ int dpg_mlp_create(dpg_mlp **out, int device, int n_prims, int64_t max_rows, uin
     dpg_mlp_destroy(M);
     return DPG_ERR_OOM;
   }
-  // (without the driver's tensor maps the forward runs the layer GEMMs)
+  // (without the driver's tensor maps: layer GEMMs with operands that threads stage)
   M->maps = cudaFuncSetAttribute(mlp_forward_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem) == cudaSuccess &&
             cudaFuncSetAttribute(mlp_forward_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmem) == cudaSuccess;
   for (int v = 0; v < 2; v++) {
@@ -372,6 +374,10 @@ int dpg_mlp_create(dpg_mlp **out, int device, int n_prims, int64_t max_rows, uin
               make_kmajor_map(&M->tw[v][1], M->W16[1], kMlpHidden, kMlpHidden, kMlpHidden, bk) &&
               make_kmajor_map(&M->tw[v][2], M->W16[2], kMlpHidden, kMlpHidden, kMlpHidden, bk) &&
               make_kmajor_map(&M->tw[v][3], M->W16[3], kMlpOutPad, kMlpHidden, kMlpOutPad);
+  }
+  if (!M->maps && (dalloc(&M->TA, (size_t)R * kMlpHidden) != cudaSuccess || dalloc(&M->TB, (size_t)R * kMlpHidden) != cudaSuccess)) {
+    dpg_mlp_destroy(M);
+    return DPG_ERR_OOM;
   }
   cudaStream_t st = M->stream;
   cudaMemsetAsync(M->err, 0, sizeof(int), st);
@@ -417,7 +423,7 @@ void dpg_mlp_destroy(dpg_mlp *M) {
     cudaFree(M->G[l]);
     cudaFree(M->dZ[l]);
   }
-  void *bufs[] = {M->emb16, M->X, M->dY, M->T1, M->loss, M->err, M->in_node, M->in_prim, M->in_target, M->hp};
+  void *bufs[] = {M->TA, M->TB, M->emb16, M->X, M->dY, M->T1, M->loss, M->err, M->in_node, M->in_prim, M->in_target, M->hp};
   for (void *b : bufs) cudaFree(b);
   if (M->hp_host) cudaFreeHost(M->hp_host);
   if (M->h_err) cudaFreeHost(M->h_err);
@@ -493,10 +499,62 @@ int dpg_mlp_forward(dpg_mlp *M, const void *node_feat_dev, const uint32_t *node_
 
 }  // extern "C"
 
+// The weight-gradient kernel's arguments; false without tensor maps.
+static bool wgrad_args(dpg_mlp *M, int64_t Bp, WgradArgs &wa, int &ctas) {
+  // weight and bias gradients: the layers share the SMs by the bytes they read
+  const int64_t n_chunks = Bp / 64;
+  const int weight[4] = {6, 8, 8, 5};  // blocks of 64 columns a chunk
+  ctas = 0;
+  for (int l = 0; l < 4; l++) {
+    WgradJob &j = wa.job[l];
+    const __nv_bfloat16 *a = l < 3 ? M->dZ[l] : M->H[2], *b = l == 0 ? M->X : l < 3 ? M->H[l - 1] : M->dY;
+    if (!make_kmajor_map(&j.a, a, (uint64_t)Bp, kMlpHidden, 64) ||
+        !make_kmajor_map(&j.b, b, (uint64_t)Bp, l == 0 ? kMlpIn : l < 3 ? kMlpHidden : kDY, 64))
+      return false;
+    j.g = M->g[2 * l];
+    j.db = l < 3 ? M->g[2 * l + 1] : nullptr;
+    j.ld = l < 3 ? kIn[l] : kMlpHidden;
+    j.n = l == 0 ? kMlpNodeFeat + kMlpEmb : l < 3 ? kMlpHidden : kMlpOutPad;
+    j.transposed = l == 3;
+    j.cta0 = ctas;
+    j.ctas = (int)std::max<int64_t>(1, std::min<int64_t>(n_chunks, (int64_t)std::max(M->sm_count, 4) * weight[l] / 27));
+    ctas += j.ctas;
+  }
+  return true;
+}
+
+// The same gradients without tensor maps: operands transposed (K-major over the
+// rows), a split-K GEMM a layer.
+static cudaError_t wgrad_transposed(dpg_mlp *M, int64_t Bp, cudaStream_t st) {
+  auto transpose = [&](const __nv_bfloat16 *in, __nv_bfloat16 *out, int cols) {
+    transpose_bf16<<<dim3((unsigned)(Bp / 32), cols / 32), dim3(32, 8), 0, st>>>(in, out, Bp, cols);
+  };
+  auto split_for = [&](int rows) {
+    const int tiles = (rows + 127) / 128;
+    return (int)std::max<int64_t>(1, std::min<int64_t>(std::max(M->sm_count, 1) / tiles, Bp / 512));
+  };
+  cudaError_t e = cudaSuccess;
+  for (int l = 0; l < 3 && e == cudaSuccess; l++) {
+    transpose(M->dZ[l], M->TA, kMlpHidden);
+    transpose(l ? M->H[l - 1] : M->X, M->TB, kIn[l]);
+    e = launch_gemm(kIn[l], M->TA, M->TB, kMlpHidden, (int)Bp, split_for(kMlpHidden),
+                    EpiAtomicF32{M->g[2 * l], kIn[l], kIn[l]}, M->err, st);
+    column_sums<<<(unsigned)((Bp + 511) / 512), kMlpHidden, 0, st>>>(M->dZ[l], Bp, M->g[2 * l + 1]);
+  }
+  if (e != cudaSuccess) return e;
+  transpose(M->dY, M->TA, kDY);  // (its first 16 rows are used)
+  transpose(M->H[2], M->TB, kMlpHidden);
+  return launch_gemm(kMlpHidden, M->TA, M->TB, kMlpOutPad, (int)Bp, split_for(kMlpOutPad),
+                     EpiAtomicF32{M->g[DPG_MLP_W4], kMlpHidden, kMlpHidden}, M->err, st);
+}
+
 // Every device operation of one training step, reading the batch from the
 // fixed input buffers and the hyper-parameters from M->hp (capturable).
 static cudaError_t enqueue_train(dpg_mlp *M, const __nv_bfloat16 *nf, int64_t B, cudaStream_t st) {
   const int64_t Bp = pad128(B);
+  WgradArgs wa{};
+  int ctas = 0;
+  if (M->maps && !wgrad_args(M, Bp, wa, ctas)) return cudaErrorNotSupported;
   cudaMemsetAsync(M->err, 0, sizeof(int), st);
   cudaMemsetAsync(M->loss, 0, M->sums_bytes, st);  // the loss and every gradient
   const int64_t chunks = Bp * (kMlpIn / 8);
@@ -515,30 +573,13 @@ static cudaError_t enqueue_train(dpg_mlp *M, const __nv_bfloat16 *nf, int64_t B,
   if (e == cudaSuccess)
     e = launch_gemm(kMlpEmb, M->dZ[0], M->WT16[0] + (size_t)kMlpNodeFeat * kMlpHidden, (int)Bp, kMlpHidden, 1,
                     EpiEmbGrad{M->in_prim, M->g[DPG_MLP_EMB], B}, M->err, st);
-  if (e != cudaSuccess) return e;
-  // weight and bias gradients: the layers share the SMs by the bytes they read
-  WgradArgs wa{};
-  const int64_t n_chunks = Bp / 64;
-  const int weight[4] = {6, 8, 8, 5};  // blocks of 64 columns a chunk
-  int cta = 0;
-  for (int l = 0; l < 4; l++) {
-    WgradJob &j = wa.job[l];
-    const __nv_bfloat16 *a = l < 3 ? M->dZ[l] : M->H[2], *b = l == 0 ? M->X : l < 3 ? M->H[l - 1] : M->dY;
-    if (!make_kmajor_map(&j.a, a, (uint64_t)Bp, kMlpHidden, 64) ||
-        !make_kmajor_map(&j.b, b, (uint64_t)Bp, l == 0 ? kMlpIn : l < 3 ? kMlpHidden : kDY, 64))
-      return cudaErrorNotSupported;
-    j.g = M->g[2 * l];
-    j.db = l < 3 ? M->g[2 * l + 1] : nullptr;
-    j.ld = l < 3 ? kIn[l] : kMlpHidden;
-    j.n = l == 0 ? kMlpNodeFeat + kMlpEmb : l < 3 ? kMlpHidden : kMlpOutPad;
-    j.transposed = l == 3;
-    j.cta0 = cta;
-    j.ctas = (int)std::max<int64_t>(1, std::min<int64_t>(n_chunks, (int64_t)std::max(M->sm_count, 4) * weight[l] / 27));
-    cta += j.ctas;
+  if (e == cudaSuccess && M->maps) {
+    e = cudaFuncSetAttribute(mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem);
+    if (e == cudaSuccess) mlp_wgrad<<<ctas, kWgThreads, kWgSmem, st>>>(wa, Bp / 64, M->err);
+  } else if (e == cudaSuccess) {
+    e = wgrad_transposed(M, Bp, st);
   }
-  e = cudaFuncSetAttribute(mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem);
   if (e != cudaSuccess) return e;
-  mlp_wgrad<<<cta, kWgThreads, kWgSmem, st>>>(wa, n_chunks, M->err);
   // Adam on every parameter and the bf16 operand copies, one launch
   static_assert(kAdamSegs == DPG_MLP_NPARAM, "one Adam segment per parameter");
   AdamArgs aa{};

@@ -227,7 +227,7 @@ struct EpiEmbGrad {
 // out[C x R] = in[R x C]^T (bf16), 32x32 tiles
 static __global__ void transpose_bf16(const __nv_bfloat16 *in, __nv_bfloat16 *out, int64_t R, int64_t C) {
   __shared__ __nv_bfloat16 t[32][33];
-  const int64_t r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+  const int64_t r0 = blockIdx.x * (int64_t)32, c0 = blockIdx.y * 32;
   for (int i = threadIdx.y; i < 32; i += blockDim.y) {
     const int64_t r = r0 + i, c = c0 + threadIdx.x;
     t[i][threadIdx.x] = (r < R && c < C) ? in[r * C + c] : __float2bfloat16_rn(0.f);
@@ -237,6 +237,18 @@ static __global__ void transpose_bf16(const __nv_bfloat16 *in, __nv_bfloat16 *ou
     const int64_t c = c0 + i, r = r0 + threadIdx.x;
     if (c < C && r < R) out[c * R + r] = t[threadIdx.x][i];
   }
+}
+
+// out[c] += sum_r in[r x 256 + c]: a thread a column over 512 rows a block, 32 at a time
+static __global__ void __launch_bounds__(kMlpHidden) column_sums(const __nv_bfloat16 *in, int64_t rows, float *out) {
+  float s = 0.f;
+  const int64_t end = min(rows, (blockIdx.x + (int64_t)1) * 512);
+  for (int64_t r0 = blockIdx.x * (int64_t)512; r0 < end; r0 += 32) {
+    float p = 0.f;
+    for (int64_t r = r0; r < min(end, r0 + 32); r++) p += __bfloat162float(in[r * kMlpHidden + threadIdx.x]);
+    s += p;
+  }
+  atomicAdd(out + threadIdx.x, s);
 }
 
 // ---------------------------------------------------------------------------

@@ -92,3 +92,98 @@ def test_weight_gradient_of_one_sign(dpg_lib):
     e = g / (0.5 * dy.sum() * b2[None, :].astype(np.float64)) - 1
     assert np.sqrt((e ** 2).mean()) <= 56 * 2.0 ** -25 + 90 ** 0.5 * 2.0 ** -25
     s.close()
+
+
+_SHIM = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stdlib.h>
+#include <string.h>
+/* with SHIM_NO_MAPS the driver has no cuTensorMapEncodeTiled; the rest goes to the runtime */
+int cudaGetDriverEntryPointByVersion(const char *s, void **p, unsigned v, unsigned long long f, int *q) {
+  if (getenv("SHIM_NO_MAPS") && !strcmp(s, "cuTensorMapEncodeTiled")) { *p = 0; if (q) *q = 1; return 0; }
+  int (*real)(const char *, void **, unsigned, unsigned long long, int *) =
+      dlsym(dlopen("libcudart.so.13", RTLD_LAZY), "cudaGetDriverEntryPointByVersion");
+  return real(s, p, v, f, q);
+}
+/* no launch while SHIM_FAIL is set */
+int cudaGraphLaunch(void *g, void *st) {
+  if (getenv("SHIM_FAIL")) return 999;
+  int (*real)(void *, void *) = dlsym(dlopen("libcudart.so.13", RTLD_LAZY), "cudaGraphLaunch");
+  return real(g, st);
+}
+"""
+
+_TRAIN = r"""
+import sys
+sys.path[:0] = sys.argv[1:3]
+import numpy as np, torch
+from test_mlp import _random_params
+from dynoplan_gb300.surrogate import Surrogate
+B, P, N = int(sys.argv[3]), 40, 100
+rng = np.random.default_rng(B)
+params = _random_params(rng, P)
+feat = torch.from_numpy(rng.normal(0, 1, (N, 80)).astype(np.float32)).cuda().to(torch.bfloat16)
+dev = lambda a: torch.from_numpy(a).cuda()
+node, prim = dev(rng.integers(0, N, B).astype(np.int32)), dev(rng.integers(0, P, B).astype(np.int32))
+target = dev(np.stack([(rng.random(B) < 0.4), rng.random(B)], 1).astype(np.float32))
+s = Surrogate(P, max_rows=max(B, 128), seed=1)
+for k, v in params.items():
+    s.set(k, v)
+loss = [s.train_step(feat, node, prim, target, lr=1e-3)]
+if sys.argv[5] == "fail":
+    import os
+    from dynoplan_gb300 import _lib
+    ms = s.timing()[0]
+    s.train_step(feat, node, prim, target, lr=0.0)
+    os.environ["SHIM_FAIL"] = "1"
+    try:
+        s.train_step(feat, node, prim, target, lr=1e-3)
+        raise SystemExit("no error")
+    except _lib.DpgError as e:
+        assert e.code == _lib.DPG_ERR_CUDA
+    del os.environ["SHIM_FAIL"]
+    assert 0.2 * ms < s.timing()[0] < 5 * ms, (ms, s.timing())  # the last step that ran
+elif sys.argv[5] == "two":
+    s.train_step(feat, node, prim, target, lr=0.0)
+loss.append(s.train_step(feat, node, prim, target, lr=1e-3))
+out = {"g_" + k: s.get(k, grad=True) for k in params}
+out.update({"w_" + k: s.get(k) for k in params})
+np.savez(sys.argv[4], loss=np.array(loss), out=s.forward(feat, node, prim).cpu().numpy(), **out)
+"""
+
+
+def _train_in_children(tmp_path, B, runs):
+    """_TRAIN in a process a run (name: environment, mode), with the stand-in preloaded"""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    (tmp_path / "shim.c").write_text(_SHIM)
+    (tmp_path / "train.py").write_text(_TRAIN)
+    shim = str(tmp_path / "shim.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", shim, str(tmp_path / "shim.c"), "-ldl"], check=True)
+    got = []
+    for k, (env, mode) in enumerate(runs):
+        path = str(tmp_path / f"{k}.npz")
+        r = subprocess.run([sys.executable, str(tmp_path / "train.py"), os.path.dirname(here), here, str(B), path, mode],
+                           env={**os.environ, "LD_PRELOAD": shim, **env}, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        got.append(dict(np.load(path)))
+    return got
+
+
+@pytest.mark.parametrize("B", [1, 700, 9729])
+def test_training_without_tensor_maps(dpg_lib, tmp_path, B):
+    """Two steps and a forward in a process where the driver gives no
+    cuTensorMapEncodeTiled (a preloaded stand-in says so), against the same with
+    it: both compute the same bf16 products (tolerance as above; the weights
+    after two steps of 1e-3 within 1e-4)."""
+    a, b = _train_in_children(tmp_path, B, [({}, ""), ({"SHIM_NO_MAPS": "1"}, "")])
+    np.testing.assert_allclose(a["loss"], b["loss"], rtol=1e-3)
+    for k in a:
+        if k.startswith("g_"):
+            assert np.linalg.norm(a[k] - b[k]) <= 2e-2 * max(np.linalg.norm(a[k]), 1e-12), k
+        elif k.startswith("w_"):
+            assert np.abs(a[k] - b[k]).mean() <= 1e-4, k
+    assert np.abs(a["out"] - b["out"]).max() <= 2e-2 * (1 + np.abs(a["out"]).max())
