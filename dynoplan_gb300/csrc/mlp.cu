@@ -220,9 +220,9 @@ struct dpg_mlp {
   cudaGraphExec_t graph = nullptr;
   int64_t graph_B = -1;
   const void *graph_feat = nullptr;
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  cudaEvent_t e0 = nullptr, e1 = nullptr, d0 = nullptr, d1 = nullptr;
   double last_ms = 0, last_flops = 0;
-  bool ms_due = false;  // e0 and e1 hold the last call's time (read when asked for)
+  bool ms_due = false;  // d0 and d1 hold the last call's time (read when asked for)
   // weight maps of the forward kernels, [0]: chunks of 64 columns, [1]: of kFwdK
   CUtensorMap tw[2][4];
   bool maps = false;
@@ -304,6 +304,14 @@ double forward_flops(int64_t Bp) {
   return 2.0 * Bp * ((double)kMlpIn * kMlpHidden + 2.0 * kMlpHidden * kMlpHidden + kMlpHidden * kMlpOutPad);
 }
 
+// e0 and e1 hold the time of a call that succeeded; the next one records into
+// the other two events
+void times_due(dpg_mlp *M) {
+  std::swap(M->e0, M->d0);
+  std::swap(M->e1, M->d1);
+  M->ms_due = true;
+}
+
 int check_err(dpg_mlp *M) {
   int h = 0;
   cudaMemcpy(&h, M->err, sizeof(int), cudaMemcpyDeviceToHost);
@@ -355,7 +363,7 @@ int dpg_mlp_create(dpg_mlp **out, int device, int n_prims, int64_t max_rows, uin
   for (int l = 0; l < 3 && ok; l++)
     ok = dalloc(&M->H[l], (size_t)R * kMlpHidden) == cudaSuccess && dalloc(&M->G[l], (size_t)R * kMlpHidden) == cudaSuccess &&
          dalloc(&M->dZ[l], (size_t)R * kMlpHidden) == cudaSuccess;
-  ok = ok && cudaEventCreate(&M->e0) == cudaSuccess && cudaEventCreate(&M->e1) == cudaSuccess;
+  for (cudaEvent_t *e : {&M->e0, &M->e1, &M->d0, &M->d1}) ok = ok && cudaEventCreate(e) == cudaSuccess;
   ok = ok && dalloc(&M->in_node, R) == cudaSuccess && dalloc(&M->in_prim, R) == cudaSuccess &&
        dalloc(&M->in_target, 2 * R) == cudaSuccess && dalloc(&M->hp, 4) == cudaSuccess &&
        cudaHostAlloc(&M->hp_host, 4 * sizeof(float), cudaHostAllocDefault) == cudaSuccess;
@@ -428,8 +436,8 @@ void dpg_mlp_destroy(dpg_mlp *M) {
   if (M->hp_host) cudaFreeHost(M->hp_host);
   if (M->h_err) cudaFreeHost(M->h_err);
   if (M->graph) cudaGraphExecDestroy(M->graph);
-  if (M->e0) cudaEventDestroy(M->e0);
-  if (M->e1) cudaEventDestroy(M->e1);
+  for (cudaEvent_t e : {M->e0, M->e1, M->d0, M->d1})
+    if (e) cudaEventDestroy(e);
   if (M->stream) cudaStreamDestroy(M->stream);
   delete M;
 }
@@ -491,7 +499,7 @@ int dpg_mlp_forward(dpg_mlp *M, const void *node_feat_dev, const uint32_t *node_
   }
   cudaEventRecord(M->e1, st);
   if (cudaStreamSynchronize(st) != cudaSuccess) return DPG_ERR_CUDA;
-  M->ms_due = true;
+  times_due(M);
   M->last_flops = flops;
   if (fused) return *(volatile int *)M->h_err ? DPG_ERR_TIMEOUT : DPG_OK;
   return check_err(M);
@@ -610,11 +618,11 @@ int dpg_mlp_train_step(dpg_mlp *M, const void *node_feat_dev, const uint32_t *no
   cudaStream_t st = M->stream;
   const auto *nf = static_cast<const __nv_bfloat16 *>(node_feat_dev);
   // this step's batch and hyper-parameters into the fixed buffers
-  M->step++;
+  const int step = M->step + 1;
   M->hp_host[0] = lr;
   M->hp_host[1] = ctg_weight;
-  M->hp_host[2] = 1.f - powf(0.9f, (float)M->step);
-  M->hp_host[3] = 1.f - powf(0.999f, (float)M->step);
+  M->hp_host[2] = 1.f - powf(0.9f, (float)step);
+  M->hp_host[3] = 1.f - powf(0.999f, (float)step);
   cudaMemcpyAsync(M->in_node, node_dev, sizeof(uint32_t) * B, cudaMemcpyDeviceToDevice, st);
   cudaMemcpyAsync(M->in_prim, prim_dev, sizeof(uint32_t) * B, cudaMemcpyDeviceToDevice, st);
   cudaMemcpyAsync(M->in_target, target_dev, sizeof(float) * 2 * B, cudaMemcpyDeviceToDevice, st);
@@ -648,8 +656,9 @@ int dpg_mlp_train_step(dpg_mlp *M, const void *node_feat_dev, const uint32_t *no
   double hl = 0;
   cudaMemcpyAsync(&hl, M->loss, sizeof(double), cudaMemcpyDeviceToHost, st);
   if (cudaStreamSynchronize(st) != cudaSuccess) return DPG_ERR_CUDA;
+  M->step = step;
   if (loss) *loss = (float)(hl / (double)B);
-  M->ms_due = true;
+  times_due(M);
   // forward + the two backward GEMMs per layer
   M->last_flops = 3.0 * forward_flops(pad128(B));
   return check_err(M);
@@ -667,7 +676,7 @@ int dpg_mlp_last_timing(const dpg_mlp *M, double *ms, double *flops) {
   if (M->ms_due) {
     dpg_mlp *m = const_cast<dpg_mlp *>(M);
     float t = 0;
-    cudaEventElapsedTime(&t, m->e0, m->e1);
+    cudaEventElapsedTime(&t, m->d0, m->d1);
     m->last_ms = t;
     m->ms_due = false;
   }

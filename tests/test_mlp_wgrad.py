@@ -187,3 +187,13 @@ def test_training_without_tensor_maps(dpg_lib, tmp_path, B):
         elif k.startswith("w_"):
             assert np.abs(a[k] - b[k]).mean() <= 1e-4, k
     assert np.abs(a["out"] - b["out"]).max() <= 2e-2 * (1 + np.abs(a["out"]).max())
+
+
+def test_failed_step_does_not_count(dpg_lib, tmp_path):
+    """A step whose launch fails (a preloaded stand-in refuses it): the weights, the
+    next step's bias corrections (a fourth step's instead of a third's would change
+    its update by a tenth) and the stage times are as if it had not been called."""
+    a, b = _train_in_children(tmp_path, 700, [({}, "two"), ({}, "fail")])
+    for k in a:
+        if k.startswith("w_"):
+            assert np.abs(a[k] - b[k]).mean() <= 1e-5, k
