@@ -1400,7 +1400,8 @@ extern "C" int dpg_mlp_node_features(dpg_ctx *c, const double *x_dev, int64_t N,
     const double ext = c->hi[i] - c->lo[i];
     fs.lo[i] = c->lo[i];
     fs.ok[i] = ext > 0 ? 1 : 0;
-    fs.scale[i] = 2.0 / ext;
+    fs.ext[i] = ext;
+    fs.inv[i] = 1.0 / ext;
   }
   GoalView gv{};
   gv.has = goal ? 1 : 0;

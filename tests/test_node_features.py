@@ -64,3 +64,29 @@ def test_features(dpg_lib, kind, N, n_obs, shift):
     got, ref = out[shift:shift + N * 80].reshape(N, 80), reference(m, env, x, goal)
     np.testing.assert_array_equal(got[:, 16:], ref[:, 16:])
     np.testing.assert_allclose(got[:, :16], ref[:, :16], rtol=2.0 ** -8, atol=1e-6)
+
+
+@pytest.mark.parametrize("kind", [W.CAR1, W.QUAD3D])
+def test_positions_are_divided_by_the_extent(dpg_lib, kind):
+    """The middle of the environment is exactly 0, its upper bound exactly 1, and
+    every position 2 (x - lo) / extent - 1 as FP64 gives it (infinite ones too), for
+    extents whose reciprocal is not exact."""
+    import torch
+
+    from dynoplan_gb300 import gpu as G
+    from dynoplan_gb300.surrogate import node_features
+    m = W.robot_model(kind)
+    d = 3 if kind == W.QUAD3D else 2
+    bf16 = lambda a: torch.from_numpy(a.astype(np.float32)).to(torch.bfloat16)
+    with G.Context(m) as ctx:
+        for e in range(3, 120):
+            ext = np.array([e, e + 0.1, e / 7.0])[:d]
+            ctx.upload_env(W.Env(np.zeros(d), ext, np.zeros((0, d)), np.zeros((0, d))))
+            x = np.zeros((64, m.nx))
+            x[:, :d] = ext * np.linspace(0, 1, 64)[:, None]
+            x[0, :d], x[1, :d], x[2, :d] = 0.5 * ext, ext, 0.25 * ext
+            x[3, :d], x[4, :d] = np.inf, -1e300
+            goal = x[5].copy()
+            f = node_features(ctx, torch.from_numpy(x).cuda(), goal).cpu()
+            assert torch.equal(f[:, :d], bf16(2.0 * x[:, :d] / ext - 1.0)), e
+            assert torch.equal(f[:, 13:13 + d], bf16(2.0 * (goal[:d] - x[:, :d]) / ext)), e
