@@ -300,8 +300,9 @@ cudaError_t forward_rows(dpg_mlp *M, int64_t B, float *out, cudaStream_t st) {
                      M->err, st);
 }
 
-double forward_flops(int64_t Bp) {
-  return 2.0 * Bp * ((double)kMlpIn * kMlpHidden + 2.0 * kMlpHidden * kMlpHidden + kMlpHidden * kMlpOutPad);
+// FLOPs of Bp rows through the network, from each of them `in` columns and `out` outputs
+double forward_flops(int64_t Bp, int in = kMlpIn, int out = kMlpOutPad) {
+  return 2.0 * Bp * kMlpHidden * ((double)in + 2.0 * kMlpHidden + out);
 }
 
 // e0 and e1 hold the time of a call that succeeded; the next one records into
@@ -487,7 +488,8 @@ int dpg_mlp_forward(dpg_mlp *M, const void *node_feat_dev, const uint32_t *node_
     else
       mlp_forward_fused<<<grid, kFusedThreads, kFusedSmem, st>>>(tw[0], tw[1], tw[2], tw[3], fa);
     if (cudaGetLastError() != cudaSuccess) return DPG_ERR_CUDA;
-    flops = forward_flops(pad128(n));
+    // (mlp_forward_pair leaves out the columns that are zero)
+    flops = M->fused == 2 ? forward_flops(pad128(n), kMlpNodeFeat + kMlpEmb, 2) : forward_flops(pad128(n));
   }
   for (int64_t r0 = 0; r0 < n && !fused; r0 += M->max_rows) {
     const int64_t B = std::min(M->max_rows, n - r0), Bp = pad128(B);
@@ -659,8 +661,10 @@ int dpg_mlp_train_step(dpg_mlp *M, const void *node_feat_dev, const uint32_t *no
   M->step = step;
   if (loss) *loss = (float)(hl / (double)B);
   times_due(M);
-  // forward + the two backward GEMMs per layer
-  M->last_flops = 3.0 * forward_flops(pad128(B));
+  // the forward; dH3 (K = 64), dH2, dH1 and the embedding's columns of dX; the weight gradients
+  const int64_t Bp = pad128(B);
+  M->last_flops = forward_flops(Bp) + forward_flops(Bp, kDY, kMlpEmb) +
+                  forward_flops(Bp, M->maps ? kMlpNodeFeat + kMlpEmb : kMlpIn);
   return check_err(M);
 }
 
