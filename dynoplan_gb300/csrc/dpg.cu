@@ -557,7 +557,7 @@ static int load_tables(dpg_ctx *c, int32_t P, const int32_t *len, const double *
     build_keys<KIND><<<(P + 127) / 128, 128, 0, st>>>(rp, P, P_<int32_t>(c->len), P_<int64_t>(c->rkrow),
                                                        P_<double>(c->st64), P_<float>(c->rkey32),
                                                        P_<float>(c->rkconst32), nullptr, nullptr, true);
-    build_chunks<KIND><<<(P + 127) / 128, 128, 0, st>>>(rp, P, P_<int32_t>(c->len), P_<int64_t>(c->soff),
+    build_chunks<KIND><<<(unsigned)(((int64_t)P * kBoxLanes + 127) / 128), 128, 0, st>>>(rp, P, P_<int32_t>(c->len), P_<int64_t>(c->soff),
                                                          P_<int64_t>(c->coff), P_<Pose<double>>(c->pose64), S,
                                                          P_<float>(c->cbox32),
                                                          parts > 1 ? P_<float>(c->qbox32) : P_<float>(c->cbox32),
