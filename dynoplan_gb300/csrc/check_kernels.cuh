@@ -545,7 +545,7 @@ template <int KIND, bool ES64> struct SlotScratch {
   using Es = std::conditional_t<ES64, double, float>;
   union {
     struct {
-      // chunk of the window << 16 | part << 14 | obstacle << 5 | lane; bounds: chunk << 16 | lane
+      // chunk of the window << 16 | part << 14 | obstacle << 5 | lane; bounds: lane
       uint32_t list[kListCap];
       uint16_t slot[kSlotCap];  // obstacle << 5 | lane
       std::conditional_t<Robot<KIND>::PARTS == 1, uint8_t, uint16_t>

@@ -135,9 +135,10 @@ static int check_occupancy(dpg_ctx *c, const void *kernel, size_t smem) {
   return blocks;
 }
 
-// The exact check of the pair list on `st`: lockstep warps over (primitive,
-// 32 nodes) items, with obstacle culling when the candidate masks cover
-// every obstacle.
+// The exact check of the pair list on `st`, by persistent warps over (primitive,
+// 32 nodes) items: a lane for every test (check_pairs_slots) in FP32 with up to
+// kSlotCap obstacles, else the lockstep walk, which culls obstacles when its
+// masks cover all of them.
 // prec: DPG_FP32 (FP32 tests, FP64 decisions in the band, FP32 end states),
 // DPG_FP64 (the same tests, FP64 end states), DPG_FP64_STRICT (every test in
 // FP64).

@@ -278,13 +278,6 @@ __device__ __forceinline__ void store16(float *dst, const float *v) {
   for (int j = 0; j < 4; j++)
     reinterpret_cast<float4 *>(dst)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
 }
-__device__ __forceinline__ void load16(const float *src, float *v) {
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    const float4 t = reinterpret_cast<const float4 *>(src)[j];
-    v[4 * j] = t.x; v[4 * j + 1] = t.y; v[4 * j + 2] = t.z; v[4 * j + 3] = t.w;
-  }
-}
 
 struct EpiStoreF32 {  // C = acc (ldc = row stride, only columns < n_valid)
   static constexpr bool kPrefetch = false;
@@ -333,13 +326,9 @@ __device__ __forceinline__ float gelu(float z) {
   const float t = tanh_fast(kGeluA * z * fmaf(kGeluB * z, z, 1.0f));
   return 0.5f * z * (1.0f + t);
 }
-__device__ __forceinline__ float gelu_grad(float z) {
-  const float t = tanh_fast(kGeluA * z * fmaf(kGeluB * z, z, 1.0f));
-  const float du = kGeluA * fmaf(3.0f * kGeluB * z, z, 1.0f);
-  return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * du;
-}
 
-// gelu and gelu_grad of two values, with the roundings of the forms above
+// gelu and its derivative, (1 + t) / 2 + z / 2 (1 - t^2) u', of two values, with
+// the roundings of the form above
 __device__ __forceinline__ uint64_t gelu2_tanh(uint64_t z, uint64_t f) {
   float u0, u1;
   unpack2(mul2(mul2(pack2(kGeluA, kGeluA), z), f), u0, u1);

@@ -110,7 +110,7 @@ __global__ void lz_scatter(const uint32_t *node, int64_t n, const uint32_t *off,
 
 // A warp per node (grid-stride), nodes of at most `cap` candidates (a power of
 // two): keys (score, primitive, place) in one 64-bit word, place and primitive
-// below 2^16, sorted by a bitonic network over the next power of two.  At 82
+// below 2^16 (the call takes up to 51,200 primitives), sorted by a bitonic network over the next power of two.  At 82
 // candidates a node a block per node spent its time in barriers: 170 us for
 // 30,000 nodes.
 constexpr int kSortThreads = 256;
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(kSortThreads) lz_sort_warp(const uint32_t *off
   }
 }
 
-// More candidates or primitives than lz_sort_warp takes: one block per node
+// More candidates than lz_sort_warp takes: one block per node
 // (grid-stride), the node's candidates sorted by (score, primitive) ascending
 // with a bitonic network over the next power of two.
 __global__ void __launch_bounds__(kSortThreads) lz_sort(const uint32_t *off, uint32_t *rank, const uint32_t *prim,
@@ -386,7 +386,7 @@ extern "C" int dpg_lazy_check(dpg_ctx *c, const dpg_expand_opts *opts, int64_t N
   if (smem > 200 * 1024)
     return ctx_fail(c, DPG_ERR_CAPACITY, "lazy_check: a node has " + std::to_string(max_seg) +
                                              " candidates (at most 16384 are ranked)");
-  if (max_seg > 1 && S <= kWarpSort && P <= 65536) {
+  if (max_seg > 1 && S <= kWarpSort) {
     const size_t sm = (size_t)S * 12 * (kSortThreads / 32);
     const int64_t warps = kSortThreads / 32, blocks = (N + warps - 1) / warps;
     lz_sort_warp<<<(unsigned)std::min<int64_t>(blocks, (int64_t)c->sm_count * 32), kSortThreads, sm, st>>>(

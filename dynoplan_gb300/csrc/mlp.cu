@@ -58,7 +58,7 @@ cudaError_t launch_gemm_n(const __nv_bfloat16 *A, const __nv_bfloat16 *B, int M,
   dim3 grid((M + 127) / 128, (K + per - 1) / per);
   CUtensorMap ta, tb;
   if (tma && make_kmajor_map(&ta, A, (uint64_t)M, (uint64_t)K, 128) && make_kmajor_map(&tb, B, N, (uint64_t)K, N)) {
-    // long K per CTA (the split-K weight gradients): the deep ring, one CTA per SM
+    // long K per CTA (split K): the deep ring, one CTA per SM
     if constexpr (std::is_same<Epi, EpiAtomicF32>::value) {
       if (per >= 8 * kGemmKChunk) {
         constexpr int S = tma_stages_deep(N);
@@ -223,7 +223,7 @@ struct dpg_mlp {
   cudaEvent_t e0 = nullptr, e1 = nullptr, d0 = nullptr, d1 = nullptr;
   double last_ms = 0, last_flops = 0;
   bool ms_due = false;  // d0 and d1 hold the last call's time (read when asked for)
-  // weight maps of the forward kernels, [0]: chunks of 64 columns, [1]: of kFwdK
+  // weight maps of the forward kernels, [0]: chunks of 64 columns, [1]: of kFwdK (no W4)
   CUtensorMap tw[2][4];
   bool maps = false;
   int *h_err = nullptr, *d_err = nullptr;  // the forward's error word, mapped page-locked memory
@@ -381,9 +381,9 @@ int dpg_mlp_create(dpg_mlp **out, int device, int n_prims, int64_t max_rows, uin
     const uint32_t bk = v ? kFwdK : kGemmKChunk;  // columns of a weight chunk
     M->maps = M->maps && make_kmajor_map(&M->tw[v][0], M->W16[0], kMlpHidden, kMlpIn, kMlpHidden, bk) &&
               make_kmajor_map(&M->tw[v][1], M->W16[1], kMlpHidden, kMlpHidden, kMlpHidden, bk) &&
-              make_kmajor_map(&M->tw[v][2], M->W16[2], kMlpHidden, kMlpHidden, kMlpHidden, bk) &&
-              make_kmajor_map(&M->tw[v][3], M->W16[3], kMlpOutPad, kMlpHidden, kMlpOutPad);
+              make_kmajor_map(&M->tw[v][2], M->W16[2], kMlpHidden, kMlpHidden, kMlpHidden, bk);
   }
+  M->maps = M->maps && make_kmajor_map(&M->tw[0][3], M->W16[3], kMlpOutPad, kMlpHidden, kMlpOutPad);
   if (!M->maps && (dalloc(&M->TA, (size_t)R * kMlpHidden) != cudaSuccess || dalloc(&M->TB, (size_t)R * kMlpHidden) != cudaSuccess)) {
     dpg_mlp_destroy(M);
     return DPG_ERR_OOM;

@@ -3,10 +3,12 @@
 // descriptors, the BF16 x BF16 -> FP32 MMA, commit to an mbarrier, and
 // tensor-memory loads.  Used by the surrogate-MLP kernels (mlp_kernels.cuh).
 //
-// Operand layout used throughout: K-major with the 128-byte swizzle.  A tile
+// Operand layouts.  The usual one is K-major with the 128-byte swizzle: a tile
 // of R rows x K bf16 is stored as K/64 "k-blocks" of R x 128 bytes; inside a
 // k-block row r occupies bytes (r/8)*1024 + (r%8)*128 and its 16-byte chunk c
-// sits at chunk (c ^ (r%8)).  Tiles start on 1024-byte boundaries.
+// sits at chunk (c ^ (r%8)).  Tiles start on 1024-byte boundaries.  The forward's
+// weight chunks are K-major with the 64-byte swizzle (sdesc_kmajor_sw64), the
+// weight gradients' operands MN-major (sdesc_mnmajor_sw128).
 #pragma once
 
 #include <cstdint>

@@ -34,3 +34,8 @@ def test_lazy_sizes(N, P, limit, score_kind):
     assert checked[needed].all()
     assert st["n_checked"] == int(checked.sum()) and st["n_accepted"] == int(accepted.sum())
     assert st["n_valid"] == int((got["verdict"] == 0).sum())
+
+
+def test_lazy_many_nodes():
+    """More than 8,192 nodes: the scan over the nodes' counts takes several passes."""
+    test_lazy_sizes(20001, 20, 5, "random")
