@@ -498,7 +498,7 @@ __device__ void check_one(const CheckArgs &A, const void *obs_sm, int p, int64_t
 //
 // The lockstep walk above makes every state cost the largest candidate count
 // of any lane: lanes with fewer candidates (most have none) wait.  Here the
-// warp goes through the primitive in windows of R::WINDOW chunks of R::CHUNK
+// warp goes through the primitive in windows of WIN chunks of R::CHUNK
 // states and gives every test to a lane of its own:
 //   - slots (lane, obstacle): the union of the lanes' window boxes selects the
 //     obstacles near any lane (a lane per obstacle, one ballot per 32), each of
@@ -536,6 +536,13 @@ __device__ void check_one(const CheckArgs &A, const void *obs_sm, int p, int64_t
 // 2.2 ms: they go out through shared memory.
 
 constexpr int kSlotCap = 512;  // slots of a window held at a time; also the most obstacles of this variant
+// Slots expected of a window from which it is WINDOW_MANY chunks: lanes meet an
+// obstacle early there, and a long window's slots do not fit.  The line lies where
+// both lengths take about the same time (quad2d, 8 and 3 chunks: random motions, 40
+// obstacles of up to 1 m on 32 square metres, 355 slots expected: 145 and 131 us, 100
+// smaller ones, 715: 289 and 197; hover motions, 65 obstacles, 63: 387 and 481, 128
+// obstacles, 90: 571 and 721).
+constexpr double kManySlots = 400;
 constexpr int kListCap = 160;  // entries held at a time
 constexpr int kListMin = 4;    // entries from which a listed chunk is tested at once
 constexpr int kNever = 0x7fffffff;
@@ -666,12 +673,12 @@ __device__ __forceinline__ bool first_of_group(unsigned m, int lane) {
   return ((m >> (lane & ~(CH - 1))) & ((1u << (lane & (CH - 1))) - 1u)) == 0u;
 }
 
-template <int KIND, bool ES64>
+template <int KIND, bool ES64, int WIN>
 __device__ __forceinline__ void check_item(const CheckArgs &A, const void *obs_sm, SlotScratch<KIND, ES64> &S, int p,
                                            uint32_t pair0, int count, uint32_t node) {
   using R = Robot<KIND>;
   using Ob = std::conditional_t<R::SPHERE, Obs3<float>, Obs2<float>>;
-  constexpr int D = R::POSD, V = R::VELOFF, CH = R::CHUNK, PARTS = R::PARTS, WIN = R::WINDOW;
+  constexpr int D = R::POSD, V = R::VELOFF, CH = R::CHUNK, PARTS = R::PARTS;
   constexpr int NE = 32 / CH;  // entries a step tests at once
   static_assert(32 % CH == 0 && WIN <= 8, "a lane per (entry, state); a byte of chunk bits");
   const int lane = threadIdx.x & 31;
@@ -1186,15 +1193,15 @@ __global__ void __launch_bounds__(kCheckThreads, Robot<KIND>::CHECK_BLOCKS) chec
   });
 }
 
-// slot-parallel tests (FP32 with the band); the warps' scratch follows the
-// obstacles at A.slot_offset, A.slot_stride bytes apart
-template <int KIND, bool ES64>
+// slot-parallel tests (FP32 with the band), in windows of WIN chunks; the warps'
+// scratch follows the obstacles at A.slot_offset, A.slot_stride bytes apart
+template <int KIND, bool ES64, int WIN>
 __global__ void __launch_bounds__(kCheckThreads, Robot<KIND>::SLOT_BLOCKS) check_pairs_slots(CheckArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
   load_obstacles<float, KIND>(A.ev, smem);
   auto &scr = *reinterpret_cast<SlotScratch<KIND, ES64> *>(smem + A.slot_offset + (threadIdx.x >> 5) * A.slot_stride);
   for_items(A, [&](int p, uint32_t pair, int count, uint32_t node) {
-    check_item<KIND, ES64>(A, smem, scr, p, pair, count, node);
+    check_item<KIND, ES64, WIN>(A, smem, scr, p, pair, count, node);
     __syncwarp();  // the next item rewrites the scratch
   });
 }

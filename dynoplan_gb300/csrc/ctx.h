@@ -43,6 +43,12 @@ struct dpg_ctx {
   double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
   int n_obs = 0;
   DevBuf obs32, obs64;
+  // what the length of the check's windows is chosen by: mean half extents of a
+  // window of motion, obstacle half extents [n_obs][3], and the slots that a
+  // window of 32 nodes is expected to have (negative: to be computed)
+  double win_half[3] = {0, 0, 0};
+  std::vector<double> obs_half;
+  double window_slots = -1;
 
   // per-call arena
   DevBuf x64, nkey32, noff32, mask, cnt, tot, pbase, ord_pbase, ord_ibase;

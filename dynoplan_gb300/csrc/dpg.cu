@@ -135,6 +135,22 @@ static int check_occupancy(dpg_ctx *c, const void *kernel, size_t smem) {
   return blocks;
 }
 
+// Slots that a window of 32 nodes, uniform over the environment, is expected to
+// have: the obstacles that its mean box touches, times 32.
+static double window_slots(dpg_ctx *c) {
+  if (c->window_slots < 0) {
+    double sum = 0;
+    for (size_t o = 0; o + 3 <= c->obs_half.size(); o += 3) {
+      double p = 32;
+      for (int i = 0; i < c->dim; i++)
+        p *= std::min(1.0, 2 * (c->obs_half[o + i] + c->win_half[i]) / (c->hi[i] - c->lo[i]));
+      sum += p;
+    }
+    c->window_slots = sum;
+  }
+  return c->window_slots;
+}
+
 // The exact check of the pair list on `st`, by persistent warps over (primitive,
 // 32 nodes) items: a lane for every test (check_pairs_slots) in FP32 with up to
 // kSlotCap obstacles, else the lockstep walk, which culls obstacles when its
@@ -165,8 +181,13 @@ static void launch_check(dpg_ctx *c, const CheckArgs &ca, int prec, cudaStream_t
     const size_t scratch = es64 ? slot_scratch_bytes<KIND, true>(gap) : slot_scratch_bytes<KIND, false>(gap);
     a.slot_offset = (int)sm_obs;
     a.slot_stride = (int)scratch;
-    if (es64) go(check_pairs_slots<KIND, true>, scratch);
-    else go(check_pairs_slots<KIND, false>, scratch);
+    auto windows = [&](auto win) {
+      constexpr int WIN = decltype(win)::value;
+      if (es64) go(check_pairs_slots<KIND, true, WIN>, scratch);
+      else go(check_pairs_slots<KIND, false, WIN>, scratch);
+    };
+    if (R::WINDOW_MANY != R::WINDOW && window_slots(c) > kManySlots) windows(std::integral_constant<int, R::WINDOW_MANY>{});
+    else windows(std::integral_constant<int, R::WINDOW>{});
     return;
   }
   auto by_words = [&](auto real, auto band, auto es64) {
@@ -566,6 +587,26 @@ static int load_tables(dpg_ctx *c, int32_t P, const int32_t *len, const double *
   });
   CUDA_TRY(c, cudaGetLastError());
   CUDA_TRY(c, cudaStreamSynchronize(st));
+  c->window_slots = -1;
+  int window = 0, window_many = 0;  // states
+  with_kind(kind, [&](auto K) {
+    using R = Robot<decltype(K)::value>;
+    window = R::WINDOW * R::CHUNK;
+    window_many = R::WINDOW_MANY * R::CHUNK;
+  });
+  if (window != window_many) {  // from up to 1,024 primitives
+    const int step = (P + 1023) / 1024, n = (P + step - 1) / step;
+    const size_t row = sizeof(float) * 2 * pd;
+    std::vector<float> box((size_t)2 * pd * n);
+    CUDA_TRY(c, cudaMemcpy2D(box.data(), row, c->tbox32.p, step * row, row, n, cudaMemcpyDeviceToHost));
+    double states = 0, sum[3] = {0, 0, 0};
+    for (int k = 0; k < n; k++) {
+      const int L = len[k * step];
+      states += L;
+      for (int i = 0; i < pd; i++) sum[i] += (double)box[(size_t)2 * pd * k + pd + i] * std::min(L, window);
+    }
+    for (int i = 0; i < pd; i++) c->win_half[i] = sum[i] / states;
+  }
   if ((rc = build_key_grid(c, P)) != DPG_OK) return rc;
   c->P = P;
   c->S = S;
@@ -641,6 +682,8 @@ int dpg_upload_env(dpg_ctx *c, int32_t dim, const double *lo, const double *hi, 
   for (int i = 0; i < dim; i++)
     if (!(lo[i] <= hi[i])) return fail(c, DPG_ERR_ARG, "upload_env: bounds lo > hi");
   CUDA_TRY(c, cudaSetDevice(c->device));
+  c->window_slots = -1;
+  c->obs_half.clear();
   std::vector<float> o32;
   std::vector<double> o64;
   for (int o = 0; o < n_obs; o++) {
@@ -653,6 +696,7 @@ int dpg_upload_env(dpg_ctx *c, int32_t dim, const double *lo, const double *hi, 
     }
     for (int i = 0; i < dim; i++) { o64.push_back(cen[i]); o32.push_back((float)cen[i]); }
     for (int i = 0; i < dim; i++) { o64.push_back(half[i]); o32.push_back((float)half[i]); }
+    for (int i = 0; i < 3; i++) c->obs_half.push_back(i < dim ? half[i] : 0.0);
   }
   int rc;
   const size_t n32 = std::max<size_t>(o32.size(), 1), n64 = std::max<size_t>(o64.size(), 1);

@@ -34,6 +34,8 @@ struct RobotParams {
 // Velocity-invariant robots: canonical_state zeroes position and velocity;
 // offset = (position, velocity); transform_primitive rolls the actions out
 // again from the shifted start.
+// WINDOW: chunks whose slots the check lists together, WINDOW_MANY: where more than
+// kManySlots of them are expected
 template <int KIND> struct Robot;
 
 template <> struct Robot<DPG_ROBOT_UNICYCLE1> {
@@ -43,7 +45,7 @@ template <> struct Robot<DPG_ROBOT_UNICYCLE1> {
   static constexpr int CHUNK = 8;  // states per culling chunk
   static constexpr int CHECK_BLOCKS = 4;  // check_pairs blocks per SM (register bound)
   static constexpr int SLOT_BLOCKS = 4;  // slot-parallel check: 64 registers a thread
-  static constexpr int WINDOW = 8;  // chunks whose slots are listed together
+  static constexpr int WINDOW = 8, WINDOW_MANY = 8;
   __host__ __device__ static int key_comp(int i) { return 2; }
   __host__ __device__ static int vel_comp(int i) { return -1; }
 };
@@ -55,7 +57,7 @@ template <> struct Robot<DPG_ROBOT_CAR1> {
   static constexpr int CHUNK = 8;
   static constexpr int CHECK_BLOCKS = 4;  // measured: 4 beats 3, 5 and 6 here
   static constexpr int SLOT_BLOCKS = 4;  // slot-parallel check: 64 registers a thread
-  static constexpr int WINDOW = 4;  // chunks whose slots are listed together
+  static constexpr int WINDOW = 4, WINDOW_MANY = 4;
   __host__ __device__ static int key_comp(int i) { return 2 + i; }
   __host__ __device__ static int vel_comp(int i) { return -1; }
 };
@@ -67,11 +69,11 @@ template <> struct Robot<DPG_ROBOT_QUAD2D> {
   static constexpr int CHUNK = 16;  // dt 0.01: ten times the states of the others per second
   static constexpr int CHECK_BLOCKS = 4;
   static constexpr int SLOT_BLOCKS = 3;  // slot-parallel check: 80 registers a thread
-  // chunks whose slots are listed together: shorter among many obstacles, where
-  // lanes meet one early and a longer window's slots do not fit (check kernel, us,
-  // windows of 8 / 4 / 3 / 2: 300 nodes x 10,000 motions, 40 obstacles 145 / 129 /
-  // 131 / 141, 100 of them 289 / 201 / 197 / 215; 32 nodes, 40: 48.8 / 47.1 / 47.1 / 53.6)
-  static constexpr int WINDOW = 3;
+  // check kernel, us, windows of 8 / 6 / 3 chunks: 32 nodes x 10,000 hover motions
+  // (270,000 pairs, most of them valid), 40 obstacles 94.5 / 91.8 / 108; 1,500 nodes
+  // 3,497 / 3,551 / 3,937; 300 nodes x 10,000 random motions (8 in 100 valid), 100
+  // obstacles 289 / 263 / 197, 200 obstacles 782 / 517 / 313
+  static constexpr int WINDOW = 8, WINDOW_MANY = 3;
   __host__ __device__ static int key_comp(int i) { return i == 0 ? 2 : 5; }
   __host__ __device__ static int vel_comp(int i) { return 3 + i; }
 };
@@ -83,7 +85,7 @@ template <> struct Robot<DPG_ROBOT_QUAD3D> {
   static constexpr int CHUNK = 16;
   static constexpr int CHECK_BLOCKS = 5;  // measured: 5 beats 4 and 6 here
   static constexpr int SLOT_BLOCKS = 4;  // slot-parallel check: 64 registers a thread
-  static constexpr int WINDOW = 2;  // chunks whose slots are listed together
+  static constexpr int WINDOW = 2, WINDOW_MANY = 2;
   __host__ __device__ static int key_comp(int i) { return i < 4 ? 3 + i : 6 + i; }
   __host__ __device__ static int vel_comp(int i) { return 7 + i; }
 };
