@@ -272,8 +272,7 @@ static __global__ void __launch_bounds__(kMlpHidden) column_sums(const __nv_bflo
 // up to 256 columns, in TMEM, so each operand is read once, and adds it to g
 // (float4 atomics) at the end or after every kWgRun chunks an accumulator: longer
 // runs' error against 64 bits exceeds that of sums over 900 rows (rms of dW3 at
-// 65,536 rows of one sign 2.3e-6, 1.2e-6 with 900 rows, 0.95e-6 with these; a
-// step takes 266 us with them, 256 without).  Warps 4-7 sum the columns of a (the bias
+// 65,536 rows of one sign 2.3e-6, 1.2e-6 with 900 rows, 0.95e-6 with these).  Warps 4-7 sum the columns of a (the bias
 // gradients) from the staged tiles while the tensor cores use them.
 // Bound by reading the operands (2 x 33.5 MB a hidden layer at 65,536 rows):
 // all four layers 48 us; as transposed copies written by the layers'
@@ -434,9 +433,26 @@ static __global__ void __launch_bounds__(kWgThreads, 1) mlp_wgrad(const __grid_c
         atomicAdd(J.g + m, v[0]);
         atomicAdd(J.g + J.ld + m, v[1]);
       } else {
-        float4 *dst = reinterpret_cast<float4 *>(J.g + (int64_t)m * J.ld + k);
+        // four lanes exchange their rows' 16-byte pieces, so that an instruction adds
+        // 64 bytes of a row (a piece of each row is half of a sector: the atomics of
+        // two runs took 6 us more of a step)
 #pragma unroll
-        for (int j = 0; j < 4; j++) atomicAdd(dst + j, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
+        for (int d = 1; d < 4; d <<= 1)
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            if (j & d) continue;
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              const float a = v[4 * j + e], b = v[4 * (j + d) + e];
+              const float o = __shfl_xor_sync(0xffffffffu, lane & d ? a : b, d);
+              v[4 * j + e] = lane & d ? o : a;
+              v[4 * (j + d) + e] = lane & d ? b : o;
+            }
+          }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          atomicAdd(reinterpret_cast<float4 *>(J.g + (int64_t)((m & ~3) + j) * J.ld + k) + (lane & 3),
+                    make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
       }
     }
     umma::fence_before_sync();
