@@ -51,10 +51,11 @@ __device__ __forceinline__ void store8(__nv_bfloat16 *dst, uint4 v, bool vec) {
 // which gives the rounded quotient (P. Markstein, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).
 // Three FP64 operations; a division each took 100,000 quadrotor nodes with a goal
-// from 43.7 to 54.4 us.  An infinite product has no remainder.
+// from 43.7 to 54.4 us.  An infinite product (exponent bits all ones) has no
+// remainder.
 __device__ __forceinline__ double divide_by(double a, double b, double inv) {
   const double q = a * inv, r = fma(fma(-q, b, a), inv, q);
-  return r == r ? r : q;
+  return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : r;
 }
 
 // normalised state of one node (16 values)
@@ -64,7 +65,7 @@ __device__ __forceinline__ void node_state_features(const double *x, const Featu
 #pragma unroll
   for (int i = 0; i < 16; i++) s[i] = 0.f;
 #pragma unroll
-  for (int i = 0; i < R::POSD; i++) s[i] = fs.ok[i] ? (float)(divide_by(2.0 * (x[i] - fs.lo[i]), fs.ext[i], fs.inv[i]) - 1.0) : 0.f;
+  for (int i = 0; i < R::POSD; i++) s[i] = fs.ok[i] ? (float)fma(2.0, divide_by(x[i] - fs.lo[i], fs.ext[i], fs.inv[i]), -1.0) : 0.f;
 #pragma unroll
   for (int i = R::POSD; i < R::NX; i++) {
     const bool raw = KIND == DPG_ROBOT_QUAD3D && i < 7;
@@ -73,7 +74,7 @@ __device__ __forceinline__ void node_state_features(const double *x, const Featu
   }
   if (gv.has) {
 #pragma unroll
-    for (int i = 0; i < R::POSD; i++) s[13 + i] = fs.ok[i] ? (float)divide_by(2.0 * (gv.g[i] - x[i]), fs.ext[i], fs.inv[i]) : 0.f;
+    for (int i = 0; i < R::POSD; i++) s[13 + i] = fs.ok[i] ? (float)(2.0 * divide_by(gv.g[i] - x[i], fs.ext[i], fs.inv[i])) : 0.f;
   }
 }
 
