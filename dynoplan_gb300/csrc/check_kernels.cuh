@@ -516,8 +516,8 @@ __device__ void check_one(const CheckArgs &A, const void *obs_sm, int p, int64_t
 // results of the sequential walk (every candidate is tested at every state up
 // to the first contact).  FP32 tests with FP64 decisions in the band.
 //
-// Bound by instruction issue (75 % of the issue slots on car1, 27.6 active
-// lanes an instruction; its table reads hit L1 / L2).  Check kernel, ms, against
+// Bound by instruction issue (77 % of the issue slots on car1, 27.1 active
+// lanes an instruction, 82 % and 26.6 on the quadrotor; its table reads hit L1 / L2).  Check kernel, ms, against
 // the form that dealt (lane, chunk, obstacle) slots out and walked a slot's
 // states in one lane (17.7 active lanes), and against the first form of this
 // one (a box for all parts of a chunk, bounds and tests chunk by chunk, every
@@ -525,7 +525,7 @@ __device__ void check_one(const CheckArgs &A, const void *obs_sm, int p, int64_t
 //   car1 100,000 x 5,000          1.91   1.34   1.03
 //   quadrotor 50,000 x 5,000     10.6    6.6    5.2
 //   unicycle1 FP64 10,000 x 1,000 0.127  0.106  0.098
-//   quad2d 32 x 10,000            0.168  0.121  0.102
+//   quad2d 32 x 10,000            0.168  0.121  0.090
 // Measured beside it: a lane walking its own states in the bounds tests when
 // many lanes need them, quadrotor 6.6 -> 8.7; entries of several chunks listed
 // before they are tested (fuller steps, but lanes past their contact), car1

@@ -276,7 +276,7 @@ static __global__ void __launch_bounds__(kMlpHidden) column_sums(const __nv_bflo
 // 65,536 rows of one sign 2.3e-6, 1.2e-6 with 900 rows, 0.95e-6 with these).  Warps 4-7 sum the columns of a (the bias
 // gradients) from the staged tiles while the tensor cores use them.
 // Bound by reading the operands (2 x 33.5 MB a hidden layer at 65,536 rows):
-// all four layers 48 us; as transposed copies written by the layers'
+// all four layers 49 us; as transposed copies written by the layers'
 // epilogues (another 230 MB) and a split-K launch per layer 155 us, without the
 // writes.  Every wait is bounded, as above.
 struct alignas(128) WgradJob {
@@ -741,7 +741,7 @@ static __global__ void __launch_bounds__(kFusedThreads, 1)
 // (measured 2,600 to 3,000 with its hand-over), the MMAs 2,048 (768 for layer
 // 1, whose columns past 96 are zero and left out; measured 3,000 to 4,000 while
 // both slots' weights stream from L2, which bounds the kernel now).
-// 1,048,576 pairs: 0.38 ms, 0.45 of the measured bf16 peak (one tile in
+// 1,048,576 pairs: 0.39 ms, a call 0.405 ms, 0.42 of the measured bf16 peak (one tile in
 // flight, two accumulators alternating by layer: 0.596 ms, 0.29); 65,536 pairs
 // 36 us (53), one tile 17 us (19).  Measured beside it: eight epilogue warps a
 // slot 5 % slower; chunks of 128 rows x 64 columns (N = 128) 20 % slower.

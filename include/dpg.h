@@ -317,7 +317,7 @@ int dpg_set_abort(dpg_ctx *ctx, int32_t flag);
 void *dpg_host_alloc(size_t bytes);
 void dpg_host_free(void *p);
 
-/* Device time of the last dpg_expand, split by stage (milliseconds):
+/* Device time of the last dpg_expand that succeeded, split by stage (milliseconds):
  * t[0] ball scan + compaction, t[1] exact check (its FP64 decisions are part
  * of it: t[2] = 0),
  * t[3] host<->device copies.  Returns the number of stages written. */

@@ -74,7 +74,8 @@ int dpg_mlp_forward(dpg_mlp *mlp, const void *node_feat_dev, const uint32_t *nod
                     int64_t n, float *out_dev);
 
 /* one Adam step on a batch: target_dev[B x 2] = [collision (0/1), cost-to-go];
- * loss = mean(BCE(logit) + 0.5 ctg_weight (ctg - target)^2), returned in *loss */
+ * loss = mean(BCE(logit) + 0.5 ctg_weight (ctg - target)^2), returned in *loss.
+ * A call that fails to launch leaves the parameters and the step count as they were. */
 int dpg_mlp_train_step(dpg_mlp *mlp, const void *node_feat_dev, const uint32_t *node_dev,
                        const uint32_t *prim_dev, const float *target_dev, int64_t B, float lr, float ctg_weight,
                        float *loss);
@@ -88,7 +89,8 @@ int dpg_mlp_train_step(dpg_mlp *mlp, const void *node_feat_dev, const uint32_t *
  * and activations, FP32 accumulation, same epilogue). */
 int dpg_mlp_set_fused(dpg_mlp *mlp, int fused);
 
-/* device time of the last forward / train step (ms) and the FLOPs it ran */
+/* device time of the last forward / train step that succeeded (ms) and the
+ * FLOPs its kernels ran (rows padded to 128) */
 int dpg_mlp_last_timing(const dpg_mlp *mlp, double *ms, double *flops);
 
 #ifdef __cplusplus
