@@ -77,7 +77,11 @@ def test_positions_are_divided_by_the_extent(dpg_lib, kind):
     from dynoplan_gb300.surrogate import node_features
     m = W.robot_model(kind)
     d = 3 if kind == W.QUAD3D else 2
-    bf16 = lambda a: torch.from_numpy(a.astype(np.float32)).to(torch.bfloat16)
+
+    def bf16(a):
+        with np.errstate(over="ignore"):  # (-1e300 becomes -inf)
+            return torch.from_numpy(a.astype(np.float32)).to(torch.bfloat16)
+
     with G.Context(m) as ctx:
         for e in range(3, 120):
             ext = np.array([e, e + 0.1, e / 7.0])[:d]
